@@ -462,8 +462,9 @@ bool class_chain(const isf_batch* b, const BatchClass& c, int ci, std::vector<PP
     yzphase(PK_Y_INV, 1);
     xphase(PK_X_INV_NORM);
     auto projection = [&](const JetArgs* jets) {
-        PPhase d = new_phase(c, ci, PK_DIV, 0, up(nx, st::BX), up(ny, st::BY), up(nz, st::planes_per_cta<ST_DIV>()) * ns);
+        PPhase d = new_phase(c, ci, PK_DIV, 0, up(nx, st::BX), up(ny, st::BY), up(nz, st::kPlanes) * ns);
         d.st = bst(c, c.f, c.g.N);
+        d.st.sz = st::kPlanes;
         PPhase f = new_phase(c, ci, PK_XR_FWD, nx, rows / 32, ns, 1);
         f.x = bx(c, 1);
         PPhase pl = new_phase(c, ci, PK_PLANE, ny, nx / 2 + 1, ns, 1);
@@ -494,8 +495,9 @@ bool class_chain(const isf_batch* b, const BatchClass& c, int ci, std::vector<PP
         }
         projection(b->jets + c.first);
     }
-    PPhase v = new_phase(c, ci, PK_VEL, 0, up(nx, st::BX), up(ny, st::BY), up(nz, st::planes_per_cta<ST_VEL>()) * ns);
+    PPhase v = new_phase(c, ci, PK_VEL, 0, up(nx, st::BX), up(ny, st::BY), up(nz, st::kPlanes) * ns);
     v.st = bst(c, c.vel, kVelComp * c.g.NP);
+    v.st.sz = st::kPlanes;
     v.st.hbar = c.g.hbar;
     v.st.sharp = 1;
     out.push_back(v);

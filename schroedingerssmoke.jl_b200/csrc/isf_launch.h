@@ -83,6 +83,7 @@ struct StencilArgs {
     int nsim;
     long long bs_psi, bs_out;
     const JetArgs* jets;
+    int sz;  // z planes per CTA: chosen by launch_stencil from the grid, fixed in the persistent batch kernel
 };
 cudaError_t launch_stencil(int op, const StencilArgs& a, cudaStream_t s);
 

@@ -2,7 +2,7 @@
 // stencil kernels (k_stencil.cu) and the persistent batch kernel.
 //
 // One CTA (256 threads, two rows each) owns a 32 x 16 column block of the
-// grid and walks up to 8 consecutive z planes.  The padded 34 x 18 psi tile of
+// grid and walks a few consecutive z planes (StencilArgs::sz).  The padded 34 x 18 psi tile of
 // the current plane sits in shared memory, the tile of the next plane arrives
 // in registers while the current one is worked on (prefetch), so psi is read
 // from HBM about once and each angle of the one-form is evaluated about once
@@ -20,21 +20,15 @@ namespace isf {
 
 namespace st {
 
-// z planes per CTA (both stencils: at 256x128x128 the div stencil ran 39.8
-// us over 4 planes and 37.3 over 8; the one-form stencil 36.3 over 4 and
-// 35.9 over 8)
-#ifndef ISF_ST_SZ
-#define ISF_ST_SZ 8
-#endif
-#ifndef ISF_ST_SZ_VEL
-#define ISF_ST_SZ_VEL 8
-#endif
+// z planes a CTA walks at most (StencilArgs::sz).  On a large grid the walk
+// amortises the prologue (two tiles and their halo indices): at 256x128x128
+// the div stencil ran 39.8 us over 4 planes, 37.3 over 8 and 44.6 over 16, the
+// one-form stencil 36.3 over 4 and 35.9 over 8.
+constexpr int kPlanes = 8;
 #ifndef ISF_ST_RPT
 #define ISF_ST_RPT 2
 #endif
 constexpr int BX = 32, TY = 8, RPT = ISF_ST_RPT, BY = TY * RPT;  // 256 threads
-template <int OP>
-constexpr int planes_per_cta() { return OP == ST_DIV ? ISF_ST_SZ : ISF_ST_SZ_VEL; }
 constexpr int TW = BX + 2, TH = BY + 2, TILE = TW * TH;        // padded tile
 constexpr int LPT = (TILE + BX * TY - 1) / (BX * TY);           // tile loads per thread
 
@@ -67,7 +61,7 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
     const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
     const int tid = bk.tid, tx = tid & (BX - 1), ty = tid / BX;
     // block z = simulation * (z chunks) + z chunk
-    constexpr int SZ = planes_per_cta<OP>();
+    const int SZ = a.sz;
     const int zchunks = (nz + SZ - 1) / SZ;
     const int sim = bk.z / zchunks;
     const int x0 = bk.x * BX, y0 = bk.y * BY, z0 = (bk.z - sim * zchunks) * SZ;

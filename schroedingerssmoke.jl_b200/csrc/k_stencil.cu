@@ -24,11 +24,25 @@ __global__ void __launch_bounds__(st::BX* st::TY, 4) k_stencil_div(StencilArgs a
     stencil_body<ST_DIV, JET>(a, launch_blk(), sm);
 }
 
-cudaError_t launch_stencil(int op, const StencilArgs& a, cudaStream_t s) {
+// z planes per CTA: as many as leave about 1024 CTAs (of 592 resident ones),
+// 1 to kPlanes.  A CTA walks its planes one after another, so on a small grid
+// the walk is the whole launch: with 8 planes 64x32x32 made 16 CTAs.  Measured
+// (one-form stencil / projection / nozzle projection, us per call, 8 planes
+// -> the rule's): 64x32x32 7.7 / 23.6 / 35.7 -> 6.0 / 15.6 / 24.2 (1 plane),
+// 128x64x64 16.3 / 42.8 / 46.1 -> 6.6 / 25.7 / 34.6 (1), 160x96x80 17.9 / 56.4 /
+// 73.2 -> 11.7 / 48.9 / 64.3 (2), 200x100x112 23.0 / 79.1 / 105.5 -> 20.5 / 75.5 /
+// 103 (5), 256x128x128 unchanged (8; 1 plane there: 44.7 / 114 / 158).
+static int planes_of(const Grid& g, long long columns) {
+    const long long sz = columns * g.n[2] / 1024;
+    return (int)(sz < 1 ? 1 : (sz > st::kPlanes ? st::kPlanes : sz));
+}
+
+cudaError_t launch_stencil(int op, const StencilArgs& args, cudaStream_t s) {
+    StencilArgs a = args;
     const int nsim = a.nsim > 1 ? a.nsim : 1;
-    const int sz = op == ST_DIV ? st::planes_per_cta<ST_DIV>() : st::planes_per_cta<ST_VEL>();
-    dim3 grid((unsigned)((a.g.n[0] + st::BX - 1) / st::BX), (unsigned)((a.g.n[1] + st::BY - 1) / st::BY),
-              (unsigned)(((a.g.n[2] + sz - 1) / sz) * nsim));
+    const unsigned bx = (unsigned)((a.g.n[0] + st::BX - 1) / st::BX), by = (unsigned)((a.g.n[1] + st::BY - 1) / st::BY);
+    a.sz = planes_of(a.g, (long long)bx * by * nsim);
+    const dim3 grid(bx, by, (unsigned)(((a.g.n[2] + a.sz - 1) / a.sz) * nsim));
     const dim3 blk(st::BX * st::TY);
     const bool jet = a.use_jet != 0;
     if (op == ST_DIV)
