@@ -166,16 +166,27 @@ static __device__ __noinline__ float3 wrap_box(float3 p, float L0, float L1, flo
     return make_float3(jl_mod_box(p.x, L0), jl_mod_box(p.y, L1), jl_mod_box(p.z, L2));
 }
 
+// The twelve velocity samples of the cell (padded index c) a particle was
+// last sampled in.  A particle moves a fraction of a cell between two RK
+// stages, so most stages after the first find their samples here and gather
+// nothing; the lanes that changed cell gather for themselves.
+struct CellVel {
+    int c;
+    float x00, x10, x01, x11, y00, y10, y01, y11, z00, z10, z01, z11;
+};
+
 // staggered_velocity (parallel.jl:219-246) on the handle's padded velocity
 // grid: seven 16-byte gathers (the cells whose components the reference's
-// twelve samples need).  Interpolation weights are the reference's unnormalised
+// twelve samples need), left out when s holds the point's cell (FIRST: s is
+// empty).  Interpolation weights are the reference's unnormalised
 // w = p - (i-1) d.  An index that rounds to n (p rounded up to L by mod) is
 // clamped to the last cell and counted.  INBOX: the caller knows the point
 // lies in [0, L)^3 (the first RK stage of a live particle).  FIDX: the
 // padded grid has at most 2^24 cells, so the base cell index is formed
 // exactly in float from the floors and converted once.
-template <bool POW2, bool NORMW, class B = CtaBar, bool INBOX = false, bool FIDX = false>
-__device__ __forceinline__ float3 stag_vel(const AdvConst& k, float3 pt, unsigned& clamps, unsigned long long* chk) {
+template <bool POW2, bool NORMW, class B = CtaBar, bool INBOX = false, bool FIDX = false, bool FIRST = false>
+__device__ __forceinline__ float3 stag_vel(const AdvConst& k, float3 pt, CellVel& s, unsigned& clamps,
+                                           unsigned long long* chk) {
     if (!INBOX) {
         // mod.(point, ph_size): the identity for points inside the box.  For
         // x >= +0 and L > 0 the float order is the order of the bit patterns,
@@ -241,31 +252,34 @@ __device__ __forceinline__ float3 stag_vel(const AdvConst& k, float3 pt, unsigne
         c000 = i[0] + sy * i[1] + sz * i[2];
     }
     (void)i;
+    if (FIRST || c000 != s.c) {
+        s.c = c000;
 #ifdef ISF_CHECK
-    const float4* v = k.v;
-    const float4 a000 = ldm<B>(v + ISF_IDX(c000)), a100 = ldm<B>(v + ISF_IDX(c000 + 1));
-    const float4 a010 = ldm<B>(v + ISF_IDX(c000 + sy)), a001 = ldm<B>(v + ISF_IDX(c000 + sz));
-    const float4 a011 = ldm<B>(v + ISF_IDX(c000 + sy + sz)), a101 = ldm<B>(v + ISF_IDX(c000 + 1 + sz));
-    const float4 a110 = ldm<B>(v + ISF_IDX(c000 + 1 + sy));
+        const float4* v = k.v;
+        const float4 a000 = ldm<B>(v + ISF_IDX(c000)), a100 = ldm<B>(v + ISF_IDX(c000 + 1));
+        const float4 a010 = ldm<B>(v + ISF_IDX(c000 + sy)), a001 = ldm<B>(v + ISF_IDX(c000 + sz));
+        const float4 a011 = ldm<B>(v + ISF_IDX(c000 + sy + sz)), a101 = ldm<B>(v + ISF_IDX(c000 + 1 + sz));
+        const float4 a110 = ldm<B>(v + ISF_IDX(c000 + 1 + sy));
 #else
-    // the reference's 12 samples (parallel.jl:224-234) from 7 cells
-    const float4* b0 = k.v + c000;
-    const float4* by = b0 + sy;
-    const float4* bz = b0 + sz;
-    const float4 a000 = ldm<B>(b0), a100 = ldm<B>(b0 + 1);
-    const float4 a010 = ldm<B>(by), a001 = ldm<B>(bz);
-    const float4 a011 = ldm<B>(by + sz), a101 = ldm<B>(bz + 1);
-    const float4 a110 = ldm<B>(by + 1);
+        // the reference's 12 samples (parallel.jl:224-234) from 7 cells
+        const float4* b0 = k.v + c000;
+        const float4* by = b0 + sy;
+        const float4* bz = b0 + sz;
+        const float4 a000 = ldm<B>(b0), a100 = ldm<B>(b0 + 1);
+        const float4 a010 = ldm<B>(by), a001 = ldm<B>(bz);
+        const float4 a011 = ldm<B>(by + sz), a101 = ldm<B>(bz + 1);
+        const float4 a110 = ldm<B>(by + 1);
 #endif
-    const float x00 = a000.x, x10 = a010.x, x01 = a001.x, x11 = a011.x;
-    const float y00 = a000.y, y10 = a100.y, y01 = a001.y, y11 = a101.y;
-    const float z00 = a000.z, z10 = a100.z, z01 = a010.z, z11 = a110.z;
+        s.x00 = a000.x, s.x10 = a010.x, s.x01 = a001.x, s.x11 = a011.x;
+        s.y00 = a000.y, s.y10 = a100.y, s.y01 = a001.y, s.y11 = a101.y;
+        s.z00 = a000.z, s.z10 = a100.z, s.z01 = a010.z, s.z11 = a110.z;
+    }
     const float wx = w[0], wy = w[1], wz = w[2];
     float3 u;
     // u_x bilinear in (y, z), u_y in (x, z), u_z in (x, y) (parallel.jl:230-245)
-    u.x = (1.f - wz) * ((1.f - wy) * x00 + wy * x10) + wz * ((1.f - wy) * x01 + wy * x11);
-    u.y = (1.f - wz) * ((1.f - wx) * y00 + wx * y10) + wz * ((1.f - wx) * y01 + wx * y11);
-    u.z = (1.f - wy) * ((1.f - wx) * z00 + wx * z10) + wy * ((1.f - wx) * z01 + wx * z11);
+    u.x = (1.f - wz) * ((1.f - wy) * s.x00 + wy * s.x10) + wz * ((1.f - wy) * s.x01 + wy * s.x11);
+    u.y = (1.f - wz) * ((1.f - wx) * s.y00 + wx * s.y10) + wz * ((1.f - wx) * s.y01 + wx * s.y11);
+    u.z = (1.f - wy) * ((1.f - wx) * s.z00 + wx * s.z10) + wy * ((1.f - wx) * s.z01 + wx * s.z11);
     return u;
 }
 
@@ -281,13 +295,14 @@ __device__ __forceinline__ void advect_slot(const AdvConst& kc, float* __restric
     if (inside) {
         ++live;
         // k2 = p .+ k1 .* dt .* 0.5f0 etc. (parallel.jl:201-212)
-        const float3 k1 = stag_vel<POW2, NORMW, B, true, FIDX>(kc, p, clamps, chk);
+        CellVel cv;
+        const float3 k1 = stag_vel<POW2, NORMW, B, true, FIDX, true>(kc, p, cv, clamps, chk);
         float3 q = make_float3(p.x + k1.x * dt * 0.5f, p.y + k1.y * dt * 0.5f, p.z + k1.z * dt * 0.5f);
-        const float3 k2 = stag_vel<POW2, NORMW, B, false, FIDX>(kc, q, clamps, chk);
+        const float3 k2 = stag_vel<POW2, NORMW, B, false, FIDX>(kc, q, cv, clamps, chk);
         q = make_float3(p.x + k2.x * dt * 0.5f, p.y + k2.y * dt * 0.5f, p.z + k2.z * dt * 0.5f);
-        const float3 k3 = stag_vel<POW2, NORMW, B, false, FIDX>(kc, q, clamps, chk);
+        const float3 k3 = stag_vel<POW2, NORMW, B, false, FIDX>(kc, q, cv, clamps, chk);
         q = make_float3(p.x + k3.x * dt, p.y + k3.y * dt, p.z + k3.z * dt);
-        const float3 k4 = stag_vel<POW2, NORMW, B, false, FIDX>(kc, q, clamps, chk);
+        const float3 k4 = stag_vel<POW2, NORMW, B, false, FIDX>(kc, q, cv, clamps, chk);
         p.x = p.x + s6 * (k1.x + 2.f * k2.x + 2.f * k3.x + k4.x);
         p.y = p.y + s6 * (k1.y + 2.f * k2.y + 2.f * k3.y + k4.y);
         p.z = p.z + s6 * (k1.z + 2.f * k2.z + 2.f * k3.z + k4.z);

@@ -51,22 +51,22 @@ __global__ void k_emit_soa(float* __restrict__ x, float* __restrict__ y, float* 
 // thread t advects slot order[t]: the arithmetic of every slot is the same,
 // only the traversal changes.  FIDX: a padded grid of at most 2^24 cells
 // (the base cell index formed in float).
+// Bound by the gathers: unsorted particles fetch every sample from L2 (1M
+// particles behind a nozzle on 128x64x64: 28 32-byte sectors each, 63 us),
+// sorted ones wait on L1.  With the samples of the last cell kept (CellVel)
+// that call takes 33.4 us, and 4M ring particles on 256x128x128 take 76 us
+// after 30 steps (118 before) and 80 us after 250 (142 before).
 // ISF_ADV_MINB: resident CTAs per SM the advection is compiled for (caps its
-// registers; 0: ptxas chooses).  At 5 (48 registers, no spills) it runs 409
-// instructions per particle against 427 at the 56 ptxas picks alone.
+// registers).  At 4 (64 registers) nothing spills; at 5 (48 registers, up to
+// 32 bytes spilled) the rings ran 79.3 and 83.0 us.
 #ifndef ISF_ADV_MINB
-#define ISF_ADV_MINB 5
-#endif
-#if ISF_ADV_MINB > 0
-#define ISF_ADV_BOUNDS __launch_bounds__(256, ISF_ADV_MINB)
-#else
-#define ISF_ADV_BOUNDS __launch_bounds__(256)
+#define ISF_ADV_MINB 4
 #endif
 template <bool POW2, bool NORMW, bool FIDX, bool ORD>
-__global__ void ISF_ADV_BOUNDS k_advect(Grid g, float* __restrict__ parts, int np,
-                                                const float* __restrict__ vel,
-                                                unsigned long long* __restrict__ counters, long long bs_vel,
-                                                const int* __restrict__ order) {
+__global__ void __launch_bounds__(256, ISF_ADV_MINB) k_advect(Grid g, float* __restrict__ parts, int np,
+                                                              const float* __restrict__ vel,
+                                                              unsigned long long* __restrict__ counters,
+                                                              long long bs_vel, const int* __restrict__ order) {
     pdl_enter();
     const int sim = blockIdx.y;
     parts += sim * 3LL * np;
@@ -144,13 +144,14 @@ __global__ void __launch_bounds__(256) k_advect_active(Grid g, float* __restrict
         }
         ++moved;
         float3 p = make_float3(x[k], y[k], z[k]);
-        const float3 k1 = stag_vel<POW2, NORMW>(kc, p, clamps, chk);
+        CellVel cv;
+        const float3 k1 = stag_vel<POW2, NORMW, CtaBar, false, false, true>(kc, p, cv, clamps, chk);
         float3 q = make_float3(p.x + k1.x * dt * 0.5f, p.y + k1.y * dt * 0.5f, p.z + k1.z * dt * 0.5f);
-        const float3 k2 = stag_vel<POW2, NORMW>(kc, q, clamps, chk);
+        const float3 k2 = stag_vel<POW2, NORMW>(kc, q, cv, clamps, chk);
         q = make_float3(p.x + k2.x * dt * 0.5f, p.y + k2.y * dt * 0.5f, p.z + k2.z * dt * 0.5f);
-        const float3 k3 = stag_vel<POW2, NORMW>(kc, q, clamps, chk);
+        const float3 k3 = stag_vel<POW2, NORMW>(kc, q, cv, clamps, chk);
         q = make_float3(p.x + k3.x * dt, p.y + k3.y * dt, p.z + k3.z * dt);
-        const float3 k4 = stag_vel<POW2, NORMW>(kc, q, clamps, chk);
+        const float3 k4 = stag_vel<POW2, NORMW>(kc, q, cv, clamps, chk);
         x[k] = p.x + s6 * (k1.x + 2.f * k2.x + 2.f * k3.x + k4.x);
         y[k] = p.y + s6 * (k1.y + 2.f * k2.y + 2.f * k3.y + k4.y);
         z[k] = p.z + s6 * (k1.z + 2.f * k2.z + 2.f * k3.z + k4.z);
@@ -171,7 +172,9 @@ __global__ void __launch_bounds__(256) k_sample_vel(Grid g, const float* __restr
     const AdvConst kc = adv_const(g, vel);
     unsigned clamps = 0;
     for (long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x; j < n; j += (long long)gridDim.x * blockDim.x) {
-        const float3 u = stag_vel<POW2, NORMW>(kc, make_float3(x[j], y[j], z[j]), clamps, counters + 2);
+        CellVel cv;
+        const float3 u = stag_vel<POW2, NORMW, CtaBar, false, false, true>(kc, make_float3(x[j], y[j], z[j]), cv, clamps,
+                                                                          counters + 2);
         ux[j] = u.x;
         uy[j] = u.y;
         uz[j] = u.z;

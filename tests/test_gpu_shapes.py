@@ -36,3 +36,25 @@ def test_stencil_planes_per_cta(isfpkg, oracle_mod, L, dims):
     orc.pressure_project(psi64)
     isf.sync()
     assert rel(host(psi), psi64) < 1e-5
+
+
+# RK stages that stay in the particle's cell, change it now and then, and
+# change it at every stage, on power-of-two and general cell sizes
+@pytest.mark.parametrize("L,dims", [((4, 2, 2), (64, 32, 32)), ((3, 2, 2), (50, 40, 24))])
+@pytest.mark.parametrize("cells_per_step", [0.01, 0.7, 5.0])
+def test_advect_across_cells(isfpkg, oracle_mod, L, dims, cells_per_step):
+    isf = isfpkg.ISF(L, dims, HBAR, DT)
+    orc = oracle_mod.Oracle(L, dims, HBAR, DT)
+    rng = np.random.default_rng(41)
+    speed = cells_per_step * min(length / n for length, n in zip(L, dims)) / DT
+    vel = (speed * rng.uniform(-1, 1, dims[::-1] + (3,))).astype(np.float32)
+    parts64 = (rng.uniform(0, 1, (20011, 3)) * np.asarray(L)).astype(np.float32).astype(np.float64)
+    isf.velocity = cuda(vel)
+    orc.set_velocity(vel.astype(np.float64))
+    parts = cuda(parts64)
+    isfpkg.staggered_advect(parts, isf)
+    isf.sync()
+    po, margin = orc.staggered_advect(parts64.copy(), margin=True)
+    clear = margin >= 1e-4
+    assert clear.mean() > 0.9
+    assert (np.abs(host(parts) - po).max(axis=1)[clear] / min(L) < 1e-5).all()
