@@ -167,16 +167,9 @@ __host__ __device__ __forceinline__ long long cell(const Grid& g, int x, int y, 
     return (long long)x + (long long)g.n[0] * ((long long)y + (long long)g.n[1] * z);
 }
 
-// atan2(y, x) for the one-form angles: t = min(|x|,|y|) / max(|x|,|y|) in
-// [0, 1], atan(t) = t P(t^2) with the degree-8 polynomial fitted by
-// csrc/gen_atan_coeffs.py (Remez exchange, max error 1.1e-7 in float32), then
-// the octant / quadrant fix-ups.  |error| <= 2.5e-7 rad for finite inputs;
-// angle(0) = 0 as in Julia.
-__device__ __forceinline__ float isf_atan2(float y, float x) {
-    const float ax = fabsf(x), ay = fabsf(y);
-    const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
-    const float t = (mx > 0.f) ? __fdividef(mn, mx) : 0.f;
-    const float s = t * t;
+// atan(t) / t as a polynomial in s = t^2 on [0, 1]: degree 8, fitted by
+// csrc/gen_atan_coeffs.py (Remez exchange, max error 1.1e-7 in float32)
+__device__ __forceinline__ float atan_poly(float s) {
     float p = 2.456725575e-03f;
     p = fmaf(p, s, -1.440136135e-02f);
     p = fmaf(p, s, 3.978123143e-02f);
@@ -185,20 +178,42 @@ __device__ __forceinline__ float isf_atan2(float y, float x) {
     p = fmaf(p, s, -1.416122913e-01f);
     p = fmaf(p, s, 1.998590678e-01f);
     p = fmaf(p, s, -3.333259821e-01f);
-    p = fmaf(p, s, 9.999998808e-01f);
-    float a = t * p;
+    return fmaf(p, s, 9.999998808e-01f);
+}
+
+// atan2(y, x) for the one-form angles: t = min(|x|,|y|) / max(|x|,|y|) in
+// [0, 1], atan(t) = t P(t^2), then the octant / quadrant fix-ups.  |error| <=
+// 2.5e-7 rad for finite inputs; angle(0) = 0 as in Julia.
+__device__ __forceinline__ float isf_atan2(float y, float x) {
+    const float ax = fabsf(x), ay = fabsf(y);
+    const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
+    const float t = (mx > 0.f) ? __fdividef(mn, mx) : 0.f;
+    float a = t * atan_poly(t * t);
     if (ay > ax) a = 1.57079632679489662f - a;
     if (x < 0.f) a = 3.14159265358979324f - a;
     return copysignf(a, y);
 }
 
-// Julia `angle(conj(a1)*b1 + conj(a2)*b2)` for psi pairs a, b (parallel.jl:108-111)
-__device__ __forceinline__ float pair_angle(float4 a, float4 b) {
+// The argument z = conj(a1) b1 + conj(a2) b2 of the one-form angle between
+// psi pairs a, b (parallel.jl:108-111): (re, im)
+__device__ __forceinline__ float2 pair_z(float4 a, float4 b) {
     // conj(a1)*b1 = (a.x - i a.y)(b.x + i b.y)
-    float re = a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w;
-    float im = a.x * b.y - a.y * b.x + a.z * b.w - a.w * b.z;
-    return isf_atan2(im, re);
+    return make_float2(a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w, a.x * b.y - a.y * b.x + a.z * b.w - a.w * b.z);
 }
+
+// |angle| < pi / 4 (NaN and 0 are not): atan2 needs no min / max, no test of
+// a zero and no fix-ups there, and angle_small gives isf_atan2's bits.  The
+// stencils branch on it: most flows turn less than that over an edge nearly
+// everywhere (256x128x128 rings: div 38.1 -> 36.7 us, one-form 35.8 -> 34.6).
+__device__ __forceinline__ bool small_angle(float2 z) { return fabsf(z.y) < z.x; }
+__device__ __forceinline__ float angle_small(float2 z) {
+    const float t = __fdividef(z.y, z.x);
+    return t * atan_poly(t * t);
+}
+__device__ __forceinline__ float angle_of(float2 z) { return isf_atan2(z.y, z.x); }
+
+// Julia `angle(conj(a1)*b1 + conj(a2)*b2)` for psi pairs a, b (parallel.jl:108-111)
+__device__ __forceinline__ float pair_angle(float4 a, float4 b) { return angle_of(pair_z(a, b)); }
 
 // particles.jl:6-10, evaluated in float with every operation rounded on its
 // own (no fused multiply-add), as the reference's broadcast over Float32
