@@ -29,11 +29,27 @@
 
 namespace isf {
 
-template <int C>
-__device__ __forceinline__ int sidx(int j, int q) {
-    static_assert(C == 8 || C == 16, "tile width");
-    return j * C + (q ^ ((j ^ (j >> 3)) & (C - 1)));
+//
+// A tile of 4 pencils (the real x passes) has too few columns for a swizzle
+// to spread the stage strides; it stores pencil after pencil with one
+// element of padding every 8 (stride-8 accesses fall into distinct banks) at a
+// pitch that sets the pencils of a half warp side by side (NT lanes each).
+template <int N, int NT>
+constexpr int quad_pitch() {
+    const int rem = NT < 16 ? (NT & ~1) : 4;  // wanted pitch mod 16 (8-byte elements)
+    int p = N + N / 8;
+    while (p % 16 != rem) ++p;
+    return p;
 }
+template <int C, int N, int NT>
+__device__ __forceinline__ int sidx(int j, int q) {
+    static_assert(C == 4 || C == 8 || C == 16, "tile width");
+    if constexpr (C == 4) return q * quad_pitch<N, NT>() + j + (j >> 3);
+    else return j * C + (q ^ ((j ^ (j >> 3)) & (C - 1)));
+}
+// elements of a tile of C pencils
+template <int C, int N, int NT>
+constexpr int tile_elems() { return C == 4 ? 4 * quad_pitch<N, NT>() : N * C; }
 
 // --------------------------------------------------------------- radix DFTs
 template <int S, class T>
@@ -258,10 +274,10 @@ __device__ __forceinline__ void pipeline(T* x, int t, int q, T* sm, const float2
     if constexpr (sizeof...(Rest) == 0) {
         scatter<N, NT, R, P>(x, t, dst);
     } else {
-        scatter<N, NT, R, P>(x, t, [&](int j, const T& v) { sm[sidx<C>(j, q)] = v; });
+        scatter<N, NT, R, P>(x, t, [&](int j, const T& v) { sm[sidx<C, N, NT>(j, q)] = v; });
         bar.xsync();
         constexpr int R2 = First<Rest...>::value;
-        gather<N, NT, R2>(x, t, [&](int j) { return sm[sidx<C>(j, q)]; });
+        gather<N, NT, R2>(x, t, [&](int j) { return sm[sidx<C, N, NT>(j, q)]; });
         bar.xsync();
         pipeline<N, NT, C, S, T, Dst, B, P * R, Rest...>(x, t, q, sm, tw, dst, bar);
     }
@@ -276,10 +292,10 @@ template <int N, int NT, int C, int S, class T, class B, int P, int R, int... Re
 __device__ __forceinline__ void pipeline_keep(T* x, int t, int q, T* sm, const float2* __restrict__ tw, const B& bar) {
     butterflies<N, NT, R, P, S>(x, t, tw);
     if constexpr (sizeof...(Rest) > 0) {
-        scatter<N, NT, R, P>(x, t, [&](int j, const T& v) { sm[sidx<C>(j, q)] = v; });
+        scatter<N, NT, R, P>(x, t, [&](int j, const T& v) { sm[sidx<C, N, NT>(j, q)] = v; });
         bar.xsync();
         constexpr int R2 = First<Rest...>::value;
-        gather<N, NT, R2>(x, t, [&](int j) { return sm[sidx<C>(j, q)]; });
+        gather<N, NT, R2>(x, t, [&](int j) { return sm[sidx<C, N, NT>(j, q)]; });
         bar.xsync();
         pipeline_keep<N, NT, C, S, T, B, P * R, Rest...>(x, t, q, sm, tw, bar);
     }

@@ -139,25 +139,42 @@ __global__ void __launch_bounds__(XShape<N, OP, G>::BLK) k_xpass(XArgs a) {
 //                 restriction's code
 enum XROp { XR_FWD = 0, XR_INV_GAUGE = 1, XR_INV_REAL = 2, XR_INV_GAUGE_JET = 3 };
 
-template <int N, int G = 1, bool KM = false>
+// C row pairs per pencil group: 4 (8 rows) or 16, chosen by launch_xr_one
+// (k_fftpass.cu); the grouped tiles of the ensembles and the persistent kernel
+// have C = 16.  With C = 4 the gauge keeps the psi of its rows in shared memory
+// (GAUGE), copied there asynchronously while the half spectrum arrives, so no
+// thread waits for psi cell after cell behind its inverse transform.
+template <int N, int G = 1, bool KM = false, int C_ = 16, bool GAUGE = false>
 struct XRShape {
-    static constexpr int C = 16;
+    static constexpr int C = C_;
     static constexpr int NT = Plan<N>::NT;
     static constexpr int BLK = G * C * NT;
     // the k-major inverse stages (A, B) of N/2 + 1 k per row pair in the tile
-    static constexpr size_t TILE = (size_t)N * C * sizeof(float2);
+    static constexpr size_t TILE = (size_t)tile_elems<C, N, NT>() * sizeof(float2);
     static constexpr size_t STAGE = (size_t)(N / 2 + 1) * C * sizeof(float4);
-    static constexpr size_t SMEM = (size_t)G * (KM && STAGE > TILE ? STAGE : TILE);
+    static constexpr size_t GROUP = (KM && STAGE > TILE ? STAGE : TILE);  // bytes of one group (a multiple of 16)
+    static constexpr size_t PSI = (C == 4 && GAUGE) ? (size_t)2 * C * N * sizeof(float4) : 0;
+    static constexpr size_t SMEM = G * GROUP + PSI;
+    static_assert(PSI == 0 || G == 1, "one group where psi is staged");
 };
 
-template <int N, int OP, int G, bool KM = false, class BarT = CtaBar>
+constexpr bool xr_gauge(int op) { return op == XR_INV_GAUGE || op == XR_INV_GAUGE_JET; }
+
+// 16-byte asynchronous copy from global to shared memory
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int N, int OP, int G, bool KM = false, int C = 16, class BarT = CtaBar>
 __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned char* smraw,
                                            const BarT& bar = BarT()) {
     using T = float2;
-    constexpr int C = 16;
+    using Sh = XRShape<N, G, KM, C, xr_gauge(OP)>;
     constexpr int NT = Plan<N>::NT;
     const int grp = bk.tid / (C * NT), lt = bk.tid % (C * NT);
-    T* sm = reinterpret_cast<T*>(smraw + grp * XRShape<N, G, KM>::SMEM / G);
+    T* sm = reinterpret_cast<T*>(smraw + grp * Sh::GROUP);
     const int t = lt % NT, q = lt / NT;
     const long long rbase = 2 * ((long long)bk.x * G + grp) * C;  // first row of the group
     const long long r0 = rbase + 2 * q;
@@ -176,16 +193,16 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
         auto src = [&](int j) -> T {
             return make_float2(v0 ? ldm<BarT>(&f0[j]) : 0.f, v1 ? ldm<BarT>(&f1[j]) : 0.f);
         };
-        auto sdst = [&](int j, const T& v) { sm[sidx<C>(j, q)] = v; };
+        auto sdst = [&](int j, const T& v) { sm[sidx<C, N, NT>(j, q)] = v; };
         Plan<N>::template run<C, -1, false>(x, t, q, sm, a.g.tw[0], src, sdst, pencil_bar<NT, C>(bar));
         bar.sync();
         if constexpr (KM) {
-            // lanes over the row pairs of the group: 16 x 16 B per k
+            // lanes over the row pairs of the group: C x 16 B per k
             float4* __restrict__ F4 = reinterpret_cast<float4*>(Fs);
             for (int idx = lt; idx < (N / 2 + 1) * C; idx += C * NT) {
                 const int qq = idx % C, k = idx / C;
-                const float2 zk = sm[sidx<C>(k, qq)];
-                const float2 zn = sm[sidx<C>(k == 0 ? 0 : N - k, qq)];
+                const float2 zk = sm[sidx<C, N, NT>(k, qq)];
+                const float2 zn = sm[sidx<C, N, NT>(k == 0 ? 0 : N - k, qq)];
                 const long long r = rbase + 2 * qq;
                 const int y = (int)(r % ny), z = (int)(r / ny);
                 F4[(((long long)k * nz + z) * ny + y) >> 1] =
@@ -196,8 +213,8 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
             float2* __restrict__ B = A + wp;
 #pragma unroll 1
             for (int k = t; k <= N / 2; k += NT) {
-                const float2 zk = sm[sidx<C>(k, q)];
-                const float2 zn = sm[sidx<C>(k == 0 ? 0 : N - k, q)];
+                const float2 zk = sm[sidx<C, N, NT>(k, q)];
+                const float2 zn = sm[sidx<C, N, NT>(k == 0 ? 0 : N - k, q)];
                 if (v0) A[k] = make_float2(0.5f * (zk.x + zn.x), 0.5f * (zk.y - zn.y));
                 if (v1) B[k] = make_float2(0.5f * (zk.y + zn.y), -0.5f * (zk.x - zn.x));
             }
@@ -205,22 +222,34 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
     } else {
         const float2* __restrict__ A = Fs + r0 * wp;
         const float2* __restrict__ B = A + wp;
+        float4* __restrict__ psi = a.psi + sim * a.bs_psi;
+        // the group's psi rows, contiguous in memory, on their way to shared memory
+        constexpr bool kStaged = Sh::PSI > 0;
+        float4* ps = reinterpret_cast<float4*>(smraw + G * Sh::GROUP);
+        if constexpr (kStaged) {
+            const float4* __restrict__ src4 = psi + rbase * N;
+            const int cells = (int)(rows - rbase < 2 * C ? rows - rbase : 2 * C) * N;
+            for (int i = lt; i < cells; i += C * NT) cp_async16(&ps[i], &src4[i]);
+        }
         // k-major: (A_k, B_k) of every row pair staged in the tile first
         // (swizzled: conflict free for the lanes over row pairs that fill it
         // and for the lanes over k that read it)
         float4* stg = reinterpret_cast<float4*>(sm);
+        auto sslot = [](int k, int qq) { return k * C + (qq ^ ((C == 4 ? k >> 1 : k) & (C - 1))); };
         if constexpr (KM) {
             const float4* __restrict__ F4 = reinterpret_cast<const float4*>(Fs);
             for (int idx = lt; idx < (N / 2 + 1) * C; idx += C * NT) {
                 const int qq = idx % C, k = idx / C;
                 const long long r = rbase + 2 * qq;
                 const int y = (int)(r % ny), z = (int)(r / ny);
-                stg[k * C + (qq ^ (k & (C - 1)))] = F4[(((long long)k * nz + z) * ny + y) >> 1];
+                const float4* from = &F4[(((long long)k * nz + z) * ny + y) >> 1];
+                if constexpr (kStaged) cp_async16(&stg[sslot(k, qq)], from);
+                else stg[sslot(k, qq)] = *from;
             }
-            bar.sync();
         }
+        if constexpr (kStaged) cp_async_wait();
+        if constexpr (KM || kStaged) bar.sync();
         float* __restrict__ rout = a.rout + sim * a.bs_r;
-        float4* __restrict__ psi = a.psi + sim * a.bs_psi;
         constexpr bool kJet = OP == XR_INV_GAUGE_JET;
         JetArgs jet;
         if constexpr (kJet) jet = a.jets ? a.jets[sim] : a.jet;
@@ -228,7 +257,7 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
             const int k = j <= N / 2 ? j : N - j;
             float2 u, v;
             if constexpr (KM) {
-                const float4 s = stg[k * C + (q ^ (k & (C - 1)))];
+                const float4 s = stg[sslot(k, q)];
                 u = make_float2(s.x, s.y);
                 v = make_float2(s.z, s.w);
             } else {
@@ -244,10 +273,16 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
                 if (v0) rout[b0 + j] = v.x;
                 if (v1) rout[b1 + j] = v.y;
             } else {
-                static_assert(OP == XR_INV_GAUGE || OP == XR_INV_GAUGE_JET, "unhandled real x-pass op");
+                static_assert(xr_gauge(OP), "unhandled real x-pass op");
                 // both rows' psi loaded before either is stored (two loads in flight)
-                float4 p0 = v0 ? psi[b0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-                float4 p1 = v1 ? psi[b1 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+                float4 p0, p1;
+                if constexpr (kStaged) {
+                    p0 = ps[2 * q * N + j];
+                    p1 = ps[(2 * q + 1) * N + j];
+                } else {
+                    p0 = v0 ? psi[b0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+                    p1 = v1 ? psi[b1 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
                 if constexpr (kJet) {
                     if (v0) restrict_cell(a.g, jet, j, (int)(r0 % ny), (int)(r0 / ny), b0 + j, p0);
                     if (v1) restrict_cell(a.g, jet, j, (int)((r0 + 1) % ny), (int)((r0 + 1) / ny), b1 + j, p1);
@@ -262,17 +297,18 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
     }
 }
 
-template <int N, int OP, int G, bool KM = false>
-__global__ void __launch_bounds__(XRShape<N, G, KM>::BLK) k_xreal(XArgs a) {
+template <int N, int OP, int G, bool KM = false, int C = 16>
+__global__ void __launch_bounds__(XRShape<N, G, KM, C>::BLK) k_xreal(XArgs a) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
-    xreal_body<N, OP, G, KM>(a, launch_blk(), smraw);
+    xreal_body<N, OP, G, KM, C>(a, launch_blk(), smraw);
 }
 
-// The same pass compiled for 3 resident CTAs per SM (at most 42 registers),
+// The 16-pair pass compiled for 3 resident CTAs per SM (at most 42 registers),
 // launched for rows of at least 256 cells: the gauge pass at 256x128x128 ran
-// 35.4 -> 34.6 us.  The ensembles' short rows keep k_xreal; capped, their
-// batched step was 5 % slower.
+// 35.4 -> 34.6 us.  The ensembles' short rows keep k_xreal (capped, their
+// batched step was 5 % slower), and so does the restricted gauge, which needs
+// its registers (nozzle projection at 256x128x128: 117 us, capped 124).
 template <int N, int OP, int G, bool KM = false>
 __global__ void __launch_bounds__(XRShape<N, G, KM>::BLK, 3) k_xreal_long(XArgs a) {
     pdl_enter();

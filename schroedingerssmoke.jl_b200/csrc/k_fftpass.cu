@@ -61,18 +61,35 @@ cudaError_t launch_xpass(int op, const XArgs& a, cudaStream_t s) {
     }
 }
 
+// Row pairs per CTA of the ungrouped real x passes: 4 below 4096 rows, 16 from
+// there on.  Short grids leave the GPU idle at 16 (64x32x32: 32 CTAs; the
+// checkpointed gradient there took 1318 us with 16 and 1295 with 4).  On
+// large ones 4 writes 64-byte instead of 256-byte segments of the k-major
+// spectrum (256x128x128 forward pass 15.4 -> 16.7 us), and although the staged
+// gauge alone is faster (34.8 -> 29.8 us), its shared memory holds up the
+// other kernels when several streams share the GPU: three ring simulations
+// side by side took 291 us per step with 16 and 329 with 4, one alone 300 and
+// 298.
+constexpr long long kLongGridRows = 4096;
+
+template <int N, int OP, bool KM>
+static cudaError_t launch_xr_one(const XArgs& a, cudaStream_t s) {
+    const long long rows = (long long)a.g.n[1] * a.g.n[2] * batch_dim(a.nsim);
+    return rows >= kLongGridRows ? launch_xr_ng<N, OP, 1, KM, 16>(a, s) : launch_xr_ng<N, OP, 1, KM, 4>(a, s);
+}
+
 template <int N, int OP>
 static cudaError_t launch_xr_n(const XArgs& a, cudaStream_t s) {
     if (a.kmajor) {
         if (a.groups > 1) return cudaErrorInvalidValue;
-        return launch_xr_ng<N, OP, 1, true>(a, s);
+        return launch_xr_one<N, OP, true>(a, s);
     }
     if constexpr (grouped_size(N) && grouped_xr_op(OP)) {
         if (a.groups == 2) return launch_xr_ng<N, OP, 2>(a, s);
         if (a.groups == 4) return launch_xr_ng<N, OP, 4>(a, s);
     }
     if (a.groups > 1) return cudaErrorInvalidValue;
-    return launch_xr_ng<N, OP, 1>(a, s);
+    return launch_xr_one<N, OP, false>(a, s);
 }
 
 template <int OP>

@@ -47,15 +47,15 @@ cudaError_t launch_x_ng(const XArgs& a, cudaStream_t s) {
     return launch_pdl(k_xpass<N, OP, G, FULL>, grid, dim3(Sh::BLK), Sh::SMEM, s, a);
 }
 
-template <int N, int OP, int G, bool KM = false>
+template <int N, int OP, int G, bool KM = false, int C = 16>
 cudaError_t launch_xr_ng(const XArgs& a, cudaStream_t s) {
-    using Sh = XRShape<N, G, KM>;
+    using Sh = XRShape<N, G, KM, C, xr_gauge(OP)>;
     static std::atomic<unsigned long long> done{0};
     const long long rows = (long long)a.g.n[1] * a.g.n[2];
     if ((G > 1 || KM) && rows % (2 * Sh::C * G) != 0) return cudaErrorInvalidValue;
     constexpr auto kern = [] {
-        if constexpr (N >= 256) return k_xreal_long<N, OP, G, KM>;
-        else return k_xreal<N, OP, G, KM>;
+        if constexpr (N >= 256 && C == 16 && OP != XR_INV_GAUGE_JET) return k_xreal_long<N, OP, G, KM>;
+        else return k_xreal<N, OP, G, KM, C>;
     }();
     cudaError_t e = ensure_smem(kern, Sh::SMEM, done);
     if (e != cudaSuccess) return e;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from helpers import rel, smooth_psi
+from helpers import rel, smooth_field, smooth_psi
 
 pytestmark = pytest.mark.gpu
 
@@ -58,3 +58,27 @@ def test_advect_across_cells(isfpkg, oracle_mod, L, dims, cells_per_step):
     clear = margin >= 1e-4
     assert clear.mean() > 0.9
     assert (np.abs(host(parts) - po).max(axis=1)[clear] / min(L) < 1e-5).all()
+
+
+# real x passes with 4 row pairs per CTA (short grids, partial last tile) and
+# with 16, k-major (ny = nz in the plane sizes) and row-major, 1 to 64 lanes a row
+@pytest.mark.parametrize("L,dims", [((1, 1, 1), (8, 12, 20)), ((1, 1, 1), (12, 32, 32)), ((2, 1, 1), (50, 12, 50)),
+                                    ((4, 2, 2), (100, 48, 48)), ((2, 2, 2), (56, 64, 64)), ((4, 2, 2), (160, 50, 100)),
+                                    ((8, 1, 1), (512, 20, 50)), ((4, 4, 4), (112, 96, 96))])
+def test_real_x_passes(isfpkg, oracle_mod, L, dims):
+    isf = isfpkg.ISF(L, dims, HBAR, DT)
+    orc = oracle_mod.Oracle(L, dims, HBAR, DT)
+    cen, length, rad = [0.3 * v for v in L], 0.3 * L[0], 0.3 * L[1]
+    psi64 = smooth_psi(dims, seed=32)
+    psi = cuda(psi64)
+    isfpkg.init_jet(isf, psi, 1, (10.0, 0.0, 0.0), nozzle=(cen, length, rad), phase_mode=1)
+    orc.restrict_velocity(psi64, (10.0, 0.0, 0.0), 0.0, cen, length, rad, phase_mode=1)
+    orc.pressure_project(psi64)
+    isf.sync()
+    assert rel(host(psi), psi64) < 1e-5
+    rng = np.random.default_rng(5)
+    f = smooth_field(dims, rng, modes=6) + 0.1 * rng.normal(size=dims[::-1])
+    q = isf.poisson_solve(cuda(f))
+    isf.sync()
+    orc.set_f(f)
+    assert rel(host(q), orc.poisson_solve().real) < 1e-5
