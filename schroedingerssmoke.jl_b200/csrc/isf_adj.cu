@@ -21,8 +21,9 @@ struct isf_adj_state {
     float* q = nullptr;     // q of a projection (N)
     float* qbar = nullptr;  // N
     float* fbar = nullptr;  // N
-    float* ubar = nullptr;  // cotangent of the padded velocity planes (3 NP)
-    double* acc = nullptr;  // 8 accumulators (jet adjoint, loss)
+    float4* ubar = nullptr;  // cotangent of the padded velocity (NP)
+    double* acc = nullptr;  // 8 accumulators: [0..3] jet adjoint, [4] loss, [5] and [6] sums of qbar in turn
+    int qslot = 5;          // the accumulator the last summed qbar went into
     float4* tape = nullptr;        // 5 psi states of one step: a (flowed), b (normalised), c, d, e
     float* tq = nullptr;           // q1 | q2 of one step (2 N)
     float* tparts = nullptr;       // particles after the step's emission
@@ -69,7 +70,7 @@ int adj_ensure(isf_handle* h) {
     const Grid& g = h->g;
     if (cudaMalloc(&a->q, sizeof(float) * g.N) != cudaSuccess || cudaMalloc(&a->qbar, sizeof(float) * g.N) != cudaSuccess ||
         cudaMalloc(&a->fbar, sizeof(float) * g.N) != cudaSuccess ||
-        cudaMalloc(&a->ubar, sizeof(float) * 3 * g.NP) != cudaSuccess ||
+        cudaMalloc(&a->ubar, sizeof(float4) * g.NP) != cudaSuccess ||
         cudaMalloc(&a->acc, sizeof(double) * 8) != cudaSuccess ||
         cudaMalloc(&a->tape, sizeof(float4) * 5 * g.N) != cudaSuccess ||
         cudaMalloc(&a->tq, sizeof(float) * 2 * g.N) != cudaSuccess) {
@@ -77,7 +78,7 @@ int adj_ensure(isf_handle* h) {
         adj_free(h);
         return fail(h, ISF_ERR_NOMEM, "adjoint work buffers: device allocation failed");
     }
-    ISF_CUDA(h, cudaMemsetAsync(a->ubar, 0, sizeof(float) * 3 * g.NP, h->stream), "adjoint set-up");
+    ISF_CUDA(h, cudaMemsetAsync(a->ubar, 0, sizeof(float4) * g.NP, h->stream), "adjoint set-up");
     return ISF_OK;
 }
 
@@ -126,12 +127,15 @@ int poisson(isf_handle* h, const float* in, float* out) {
     return ISF_OK;
 }
 
-// adjoint of psi_out = psi_in exp(-i q), q = P div W(psi_in)
-int adj_projection(isf_handle* h, const float* psi_in, const float* q, float* bar) {
+// adjoint of psi_out = psi_in exp(-i q), q = P div W(psi_in); with sum, the
+// sum of qbar goes into acc[qslot] for the adjoint of a restriction before it
+int adj_projection(isf_handle* h, const float* psi_in, const float* q, float* bar, bool sum) {
     isf_adj_state* a = h->adj;
+    const int prev = a->qslot;
+    if (sum) a->qslot = 11 - prev;  // 5 and 6 in turn; the kernel clears the other one
     const float4* pin = reinterpret_cast<const float4*>(psi_in);
     float4* b = reinterpret_cast<float4*>(bar);
-    ISF_LAUNCH(h, launch_adj_gauge(h->g, pin, q, b, a->qbar, h->stream), "adj gauge");
+    ISF_LAUNCH(h, launch_adj_gauge(h->g, pin, q, b, a->qbar, sum ? a->acc + a->qslot : nullptr, a->acc + prev, h->stream), "adj gauge");
     if (int rc = poisson(h, a->qbar, a->fbar)) return rc;
     ISF_LAUNCH(h, launch_adj_oneform_div(h->g, pin, b, a->fbar, h->stream), "adj one-form (div)");
     return ISF_OK;
@@ -198,9 +202,11 @@ int step_tape(isf_handle* h, const float* psi_in, const float* parts_in, long lo
     if (int rc = run_schroedinger(h, reinterpret_cast<float*>(pa), false)) return rc;
     ISF_LAUNCH(h, launch_normalize_to(h->g, pa, pb, h->stream), "adj tape normalize");
     if (int rc = projection_q(h, reinterpret_cast<const float*>(pb), tq)) return rc;
-    ISF_LAUNCH(h, launch_gauge(h->g, pb, tq, pc, h->stream), "adj tape gauge");
     const float* parts = parts_in;
-    if (sj.jet) {
+    if (!sj.jet) {
+        ISF_LAUNCH(h, launch_gauge(h->g, pb, tq, pc, h->stream), "adj tape gauge");
+        *out_psi = pc;
+    } else {
         if (np > 0 && sj.emit_count > 0) {
             if (int rc = grow(h, a->tparts, a->tparts_cap, 3 * np, "adjoint particles")) return rc;
             ISF_CUDA(h, cudaMemcpyAsync(a->tparts, parts_in, sizeof(float) * 3 * np, cudaMemcpyDeviceToDevice, h->stream),
@@ -208,12 +214,10 @@ int step_tape(isf_handle* h, const float* psi_in, const float* parts_in, long lo
             ISF_LAUNCH(h, launch_emit(a->tparts, np, sj.emit_start % np, sj.emit_count, sj.e, h->stream), "adj tape emit");
             parts = a->tparts;
         }
-        ISF_LAUNCH(h, launch_restrict_to(h->g, pc, pd, sj.j, h->stream), "adj tape restrict");
+        ISF_LAUNCH(h, launch_gauge_restrict(h->g, pb, tq, pc, pd, sj.j, h->stream), "adj tape gauge + restrict");
         if (int rc = projection_q(h, reinterpret_cast<const float*>(pd), tq + N)) return rc;
         ISF_LAUNCH(h, launch_gauge(h->g, pd, tq + N, pe, h->stream), "adj tape gauge");
         *out_psi = pe;
-    } else {
-        *out_psi = pc;
     }
     *out_parts = parts;
     return ISF_OK;
@@ -235,12 +239,13 @@ int step_reverse(isf_handle* h, const float* parts_used, long long np, const Ste
     }
     float4* b = reinterpret_cast<float4*>(bar);
     ISF_LAUNCH(h, launch_adj_oneform_vel(h->g, psi_out, b, a->ubar, h->g.hbar, 1, h->stream), "adj one-form (velocity)");
-    ISF_CUDA(h, cudaMemsetAsync(a->ubar, 0, sizeof(float) * 3 * h->g.NP, h->stream), "adj clear velocity cotangent");
+    ISF_CUDA(h, cudaMemsetAsync(a->ubar, 0, sizeof(float4) * h->g.NP, h->stream), "adj clear velocity cotangent");
     if (sj.jet) {
-        if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + 3 * N), tq + N, bar)) return rc;
-        ISF_LAUNCH(h, launch_adj_restrict(h->g, T + 2 * N, b, sj.j, a->acc, wscale, h->stream), "adj restrict");
+        if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + 3 * N), tq + N, bar, true)) return rc;
+        ISF_LAUNCH(h, launch_adj_restrict(h->g, T + 2 * N, b, sj.j, a->acc, wscale, a->acc + a->qslot, h->stream),
+                   "adj restrict");
     }
-    if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + N), tq, bar)) return rc;
+    if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + N), tq, bar, false)) return rc;
     ISF_LAUNCH(h, launch_adj_normalize(h->g, T, b, h->stream), "adj normalize");
     return adj_schroedinger(h, bar);
 }
@@ -325,7 +330,7 @@ int isf_adj_pressure_project(isf_handle* h, const float* psi_in, float* psibar) 
     ISF_ALIGNED(h, psibar, 16, "psibar");
     if (int rc = adj_ensure(h)) return rc;
     if (int rc = projection_q(h, psi_in, h->adj->q)) return rc;
-    return adj_projection(h, psi_in, h->adj->q, psibar);
+    return adj_projection(h, psi_in, h->adj->q, psibar, false);
 }
 
 int isf_adj_restrict_velocity(isf_handle* h, const float* psi_in, float* psibar, const float kvec[3],
@@ -342,7 +347,7 @@ int isf_adj_restrict_velocity(isf_handle* h, const float* psi_in, float* psibar,
     if (int rc = clear_acc(h)) return rc;
     const JetArgs j = make_jet(kvec, jetmask, cen, len, rad, omgterm, phase_mode);
     ISF_LAUNCH(h, launch_adj_restrict(h->g, reinterpret_cast<const float4*>(psi_in), reinterpret_cast<float4*>(psibar), j,
-                                      h->adj->acc, 1.f, h->stream),
+                                      h->adj->acc, 1.f, nullptr, h->stream),
                "adj restrict");
     return read_acc(h, jetbar, 4);
 }
@@ -356,7 +361,7 @@ int isf_adj_velocity_one_form(isf_handle* h, const float* psi, float hbar, int32
     ISF_LAUNCH(h, launch_adj_oneform_vel(h->g, reinterpret_cast<const float4*>(psi), reinterpret_cast<float4*>(psibar),
                                          h->adj->ubar, hbar, sharp ? 1 : 0, h->stream),
                "adj one-form (velocity)");
-    ISF_CUDA(h, cudaMemsetAsync(h->adj->ubar, 0, sizeof(float) * 3 * h->g.NP, h->stream), "adj clear velocity cotangent");
+    ISF_CUDA(h, cudaMemsetAsync(h->adj->ubar, 0, sizeof(float4) * h->g.NP, h->stream), "adj clear velocity cotangent");
     return ISF_OK;
 }
 
@@ -374,7 +379,6 @@ int isf_adj_get_velocity_bar(isf_handle* h, float* aos) {
     ISF_ENTER(h);
     if (!aos) return fail(h, ISF_ERR_INVALID, "isf_adj_get_velocity_bar: null output");
     if (int rc = adj_ensure(h)) return rc;
-    ISF_LAUNCH(h, launch_adj_fold(h->g, h->adj->ubar, h->stream), "adj fold");
     ISF_LAUNCH(h, launch_adj_to_aos(h->g, h->adj->ubar, aos, h->stream), "adj velocity cotangent to aos");
     return ISF_OK;
 }
@@ -383,7 +387,7 @@ int isf_adj_set_velocity_bar(isf_handle* h, const float* aos) {
     ISF_ENTER(h);
     if (!aos) return fail(h, ISF_ERR_INVALID, "isf_adj_set_velocity_bar: null input");
     if (int rc = adj_ensure(h)) return rc;
-    ISF_CUDA(h, cudaMemsetAsync(h->adj->ubar, 0, sizeof(float) * 3 * h->g.NP, h->stream), "adj clear velocity cotangent");
+    ISF_CUDA(h, cudaMemsetAsync(h->adj->ubar, 0, sizeof(float4) * h->g.NP, h->stream), "adj clear velocity cotangent");
     ISF_LAUNCH(h, launch_adj_from_aos(h->g, aos, h->adj->ubar, h->stream), "adj velocity cotangent from aos");
     return ISF_OK;
 }
@@ -530,8 +534,9 @@ int isf_adj_gradient(isf_handle* h, const isf_adj_problem* p, const float* psi0,
         const float4* in = itape + (long long)it * N;
         ISF_LAUNCH(h, launch_restrict_to(h->g, in, work, j0, h->stream), "adj init restrict");
         if (int rc = projection_q(h, reinterpret_cast<const float*>(work), a->q)) return rc;
-        if (int rc = adj_projection(h, reinterpret_cast<const float*>(work), a->q, psibar0)) return rc;
-        ISF_LAUNCH(h, launch_adj_restrict(h->g, in, reinterpret_cast<float4*>(psibar0), j0, a->acc, 0.f, h->stream),
+        if (int rc = adj_projection(h, reinterpret_cast<const float*>(work), a->q, psibar0, true)) return rc;
+        ISF_LAUNCH(h, launch_adj_restrict(h->g, in, reinterpret_cast<float4*>(psibar0), j0, a->acc, 0.f,
+                                          a->acc + a->qslot, h->stream),
                    "adj init restrict");
     }
     double acc[5];

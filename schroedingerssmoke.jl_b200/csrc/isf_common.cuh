@@ -117,6 +117,20 @@ __device__ __forceinline__ auto pencil_bar(const B& b) {
     else return b;
 }
 
+// The cells of a grid as a launch of 256-thread blocks over 32 x 8 (x, y)
+// tiles, every block walking z from blockIdx.z in steps of gridDim.z: a
+// thread's coordinates cost no division (a flat index decoded with 64-bit
+// divisions made the nearest-neighbour kernels spend most of their
+// instructions on it).  At most about 16 blocks per SM.
+__device__ __forceinline__ int cell_x() { return (int)(blockIdx.x * 32 + (threadIdx.x & 31)); }
+__device__ __forceinline__ int cell_y() { return (int)(blockIdx.y * 8 + (threadIdx.x >> 5)); }
+inline dim3 cell_grid(const Grid& g) {
+    const unsigned bx = (unsigned)((g.n[0] + 31) / 32), by = (unsigned)((g.n[1] + 7) / 8);
+    unsigned bz = 148u * 16u / (bx * by);
+    bz = bz < 1 ? 1 : (bz > (unsigned)g.n[2] ? (unsigned)g.n[2] : bz);
+    return dim3(bx, by, bz);
+}
+
 // Block coordinates and thread index of one (virtual) CTA: blockIdx /
 // threadIdx for a kernel launched on its own, the work item's in the
 // persistent batch kernel.

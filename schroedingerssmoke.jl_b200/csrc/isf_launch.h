@@ -180,21 +180,25 @@ cudaError_t launch_gauge_complex(float* psi, const float* qre, const float* qim,
 cudaError_t launch_gauge(const Grid& g, const float4* in, const float* q, float4* out, cudaStream_t s);
 cudaError_t launch_normalize_to(const Grid& g, const float4* in, float4* out, cudaStream_t s);
 cudaError_t launch_restrict_to(const Grid& g, const float4* in, float4* out, const JetArgs& j, cudaStream_t s);
+// mid = in exp(-i q), out = restrict(mid)
+cudaError_t launch_gauge_restrict(const Grid& g, const float4* in, const float* q, float4* mid, float4* out,
+                                  const JetArgs& j, cudaStream_t s);
 cudaError_t launch_adj_normalize(const Grid& g, const float4* psi_in, float4* bar, cudaStream_t s);
-cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar,
-                             cudaStream_t s);
+// with sum, adds the sum of qbar into *sum and sets *clear to 0
+cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar, double* sum,
+                             double* clear, cudaStream_t s);
 cudaError_t launch_adj_oneform_div(const Grid& g, const float4* psi, float4* bar, const float* fbar, cudaStream_t s);
-// folds the padded copies of ubar, then adds the one-form transpose (scale hbar [/ d])
-cudaError_t launch_adj_oneform_vel(const Grid& g, const float4* psi, float4* bar, float* ubar, float hbar, int sharp,
-                                   cudaStream_t s);
-cudaError_t launch_adj_fold(const Grid& g, float* ubar, cudaStream_t s);
-cudaError_t launch_adj_from_aos(const Grid& g, const float* aos, float* ubar, cudaStream_t s);
-cudaError_t launch_adj_to_aos(const Grid& g, const float* ubar, float* aos, cudaStream_t s);
-// acc[0..2] += cotangent of kvec, acc[3] += cotangent of omega t times wscale
+// adds the one-form transpose of the padded velocity cotangent (scale hbar [/ d])
+cudaError_t launch_adj_oneform_vel(const Grid& g, const float4* psi, float4* bar, const float4* ubar, float hbar,
+                                   int sharp, cudaStream_t s);
+cudaError_t launch_adj_from_aos(const Grid& g, const float* aos, float4* ubar, cudaStream_t s);
+cudaError_t launch_adj_to_aos(const Grid& g, const float4* ubar, float* aos, cudaStream_t s);
+// acc[0..2] += cotangent of kvec, acc[3] += cotangent of omega t times wscale;
+// qsum: null, or the sum of qbar of the projection the restricted psi went into
 cudaError_t launch_adj_restrict(const Grid& g, const float4* psi_in, float4* bar, const JetArgs& j, double* acc,
-                                float wscale, cudaStream_t s);
+                                float wscale, const double* qsum, cudaStream_t s);
 cudaError_t launch_adj_advect(const Grid& g, const float* parts, float* lam, long long np, const float* vel,
-                              float* ubar, cudaStream_t s);
+                              float4* ubar, cudaStream_t s);
 cudaError_t launch_loss(const float* x, const float* y, float* lam, long long np, double* loss, cudaStream_t s);
 cudaError_t launch_zero_slots(float* lam, long long nslots, long long start, long long count, cudaStream_t s);
 

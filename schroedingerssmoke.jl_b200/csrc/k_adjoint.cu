@@ -27,18 +27,6 @@ inline unsigned grid_n(long long n, int block) {
     return (unsigned)(b < cap ? b : cap);
 }
 
-__device__ __forceinline__ void decode_cell(const Grid& g, long long c, int& x, int& y, int& z) {
-    x = (int)(c % g.n[0]);
-    const long long r = c / g.n[0];
-    y = (int)(r % g.n[1]);
-    z = (int)(r / g.n[1]);
-}
-
-// z = conj(a1) b1 + conj(a2) b2 for psi pairs (the one-form's argument)
-__device__ __forceinline__ float2 zpair(float4 a, float4 b) {
-    return make_float2(a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w, a.x * b.y - a.y * b.x + a.z * b.w - a.w * b.z);
-}
-
 // block-wide sum of n doubles into acc[] (one atomicAdd per value per block)
 template <int NV>
 __device__ __forceinline__ void block_sum_add(double (&v)[NV], double* acc) {
@@ -67,22 +55,33 @@ __device__ __forceinline__ void block_sum_add(double (&v)[NV], double* acc) {
 // out = in exp(-i q) with a real q per cell (the forward gauge on its own)
 __global__ void k_gauge(const float4* __restrict__ in, const float* __restrict__ q, float4* __restrict__ out,
                         long long N) {
+    pdl_enter();
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N; c += (long long)gridDim.x * blockDim.x)
         out[c] = gauge4(in[c], q[c]);
 }
 
 // out = normalize_psi(in)
 __global__ void k_normalize_to(const float4* __restrict__ in, float4* __restrict__ out, long long N) {
+    pdl_enter();
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N; c += (long long)gridDim.x * blockDim.x)
         out[c] = normalize4(in[c]);
 }
 
-// out = restrict_velocity(in) (every cell written)
-__global__ void k_restrict_to(Grid g, const float4* __restrict__ in, float4* __restrict__ out, JetArgs j) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode_cell(g, c, x, y, z);
+// out = restrict_velocity(in) (every cell written).  With q, in is gauged
+// first and mid gets what is restricted: mid = in exp(-i q), out = restrict(mid)
+template <bool GAUGE>
+__global__ void __launch_bounds__(256) k_restrict_to(Grid g, const float4* __restrict__ in, const float* __restrict__ q,
+                                                     float4* __restrict__ mid, float4* __restrict__ out, JetArgs j) {
+    pdl_enter();
+    const int x = cell_x(), y = cell_y();
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
+        const long long c = cell(g, x, y, z);
         float4 v = in[c];
+        if constexpr (GAUGE) {
+            v = gauge4(v, q[c]);
+            mid[c] = v;
+        }
         restrict_cell(g, j, x, y, z, c, v);
         out[c] = v;
     }
@@ -90,6 +89,7 @@ __global__ void k_restrict_to(Grid g, const float4* __restrict__ in, float4* __r
 
 // normalize: out = v / |v| (4 reals); bar_in = (bar_out - b (b . bar_out)) / |v|
 __global__ void k_adj_normalize(const float4* __restrict__ psi_in, float4* __restrict__ bar, long long N) {
+    pdl_enter();
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N; c += (long long)gridDim.x * blockDim.x) {
         const float4 v = psi_in[c];
         const float r = sqrtf(v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w);
@@ -106,75 +106,109 @@ __global__ void k_adj_normalize(const float4* __restrict__ psi_in, float4* __res
 }
 
 // gauge: out = in exp(-i q).  qbar = sum_k Im(conj(bar_k) out_k);
-// bar_in = bar_out exp(+i q)
-__global__ void k_adj_gauge(const float4* __restrict__ psi_in, const float* __restrict__ q, float4* __restrict__ bar,
-                            float* __restrict__ qbar, long long N) {
+// bar_in = bar_out exp(+i q).  With sum, the sum of qbar over the grid is
+// added into *sum (k_adj_restrict) and *clear, the slot of the call before,
+// becomes 0.
+__global__ void __launch_bounds__(256) k_adj_gauge(const float4* __restrict__ psi_in, const float* __restrict__ q,
+                                                   float4* __restrict__ bar, float* __restrict__ qbar, long long N,
+                                                   double* __restrict__ sum, double* __restrict__ clear) {
+    pdl_enter();
+    double total[1] = {0.0};
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N; c += (long long)gridDim.x * blockDim.x) {
         const float qc = q[c];
-        const float4 o = gauge4(psi_in[c], qc);
+        const float4 v = psi_in[c];
         const float4 g = bar[c];
-        qbar[c] = (g.x * o.y - g.y * o.x) + (g.z * o.w - g.w * o.z);
         float s, co;
         sincosf(qc, &s, &co);
+        const float4 o = make_float4(v.x * co + v.y * s, v.y * co - v.x * s, v.z * co + v.w * s, v.w * co - v.z * s);
+        const float qb = (g.x * o.y - g.y * o.x) + (g.z * o.w - g.w * o.z);
+        qbar[c] = qb;
+        total[0] += qb;
         bar[c] = make_float4(g.x * co - g.y * s, g.x * s + g.y * co, g.z * co - g.w * s, g.z * s + g.w * co);
+    }
+    if (sum) {
+        block_sum_add<1>(total, sum);
+        if (blockIdx.x == 0 && threadIdx.x == 0) *clear = 0.0;
     }
 }
 
 // Transpose of the one-form at psi, added into bar.  The one-form's cotangent
 // per edge (cell i, axis a) is
-//   mode 0: wbar_a[i] = s_a (fbar[i] - fbar[i + e_a])   (through div, s_a = 1/d_a^2)
-//   mode 1: wbar_a[i] = s_a ubar_a[i]                    (velocity planes, s_a = hbar / d_a)
+//   DIV:  wbar_a[i] = s_a (fbar[i] - fbar[i + e_a])   (through div, s_a = 1/d_a^2)
+//   else: wbar_a[i] = s_a ubar_a[i]                    (velocity, s_a = hbar [/ d_a])
 // and w_a[i] = angle(z), z = sum_k conj(psi_k[i]) psi_k[i+e_a], contributes
 //   bar_k[i]     += wbar (-i conj(z) psi_k[i+e_a]) / |z|^2
 //   bar_k[i+e_a] += wbar ( i z psi_k[i]) / |z|^2
-// gathered here per cell from the edges i and i - e_a.
+// gathered here per cell from the edges i and i - e_a.  The velocity cotangent
+// lives on the padded grid; a cell on a low face collects the periodic copies
+// of its value on the +faces as it reads.  Bound by the seven psi cells and
+// the neighbours' cotangents, most of them L1 hits of the 32 x 8 tile.
 struct AdjOneFormArgs {
     Grid g;
     const float4* psi;
     float4* bar;
-    const float* fbar;  // mode 0
-    const float* ubar;  // mode 1: padded planes (copies folded into the cells they repeat)
+    const float* fbar;   // DIV
+    const float4* ubar;  // padded velocity cotangent
     float s[3];
-    int mode;
 };
 
-__global__ void k_adj_oneform(AdjOneFormArgs A) {
+// the cotangent of cell (x, y, z)'s velocity: its own entry and those of its
+// periodic copies on the +faces
+__device__ __forceinline__ float4 ubar_at(const Grid& g, const float4* __restrict__ u, int x, int y, int z) {
+    const int p = pcell(g, x, y, z);
+    float4 v = u[p];
+    const bool cx = x == 0, cy = y == 0, cz = z == 0;
+    if (cx | cy | cz) {
+        const int ox = g.n[0], oy = g.n[1] * g.pnx, oz = g.n[2] * g.pnxy;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) {
+            const bool on = (!(k & 1) || cx) && (!(k & 2) || cy) && (!(k & 4) || cz);
+            if (on) v = cadd(v, u[p + ((k & 1) ? ox : 0) + ((k & 2) ? oy : 0) + ((k & 4) ? oz : 0)]);
+        }
+    }
+    return v;
+}
+
+template <bool DIV>
+__global__ void __launch_bounds__(256) k_adj_oneform(AdjOneFormArgs A) {
+    pdl_enter();
     const Grid& g = A.g;
     const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode_cell(g, c, x, y, z);
+    const int x = cell_x(), y = cell_y();
+    if (x >= nx || y >= ny) return;
+    const int xp = (x + 1 == nx) ? 0 : x + 1, xm = (x == 0) ? nx - 1 : x - 1;
+    const int yp = (y + 1 == ny) ? 0 : y + 1, ym = (y == 0) ? ny - 1 : y - 1;
+    for (int z = blockIdx.z; z < nz; z += gridDim.z) {
+        const int zp = (z + 1 == nz) ? 0 : z + 1, zm = (z == 0) ? nz - 1 : z - 1;
+        const int cp[3] = {(int)cell(g, xp, y, z), (int)cell(g, x, yp, z), (int)cell(g, x, y, zp)};
+        const int cm[3] = {(int)cell(g, xm, y, z), (int)cell(g, x, ym, z), (int)cell(g, x, y, zm)};
+        const int c = (int)cell(g, x, y, z);
         const float4 p0 = A.psi[c];
         float4 acc = A.bar[c];
+        float wh[3], wp[3];
+        if constexpr (DIV) {
+            const float f0 = A.fbar[c];
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                wh[a] = A.s[a] * (f0 - A.fbar[cp[a]]);
+                wp[a] = A.s[a] * (A.fbar[cm[a]] - f0);
+            }
+        } else {
+            const float4 u = ubar_at(g, A.ubar, x, y, z);
+            wh[0] = A.s[0] * u.x;
+            wh[1] = A.s[1] * u.y;
+            wh[2] = A.s[2] * u.z;
+            wp[0] = A.s[0] * ubar_at(g, A.ubar, xm, y, z).x;
+            wp[1] = A.s[1] * ubar_at(g, A.ubar, x, ym, z).y;
+            wp[2] = A.s[2] * ubar_at(g, A.ubar, x, y, zm).z;
+        }
 #pragma unroll
         for (int a = 0; a < 3; ++a) {
-            int xp = x, yp = y, zp = z, xm = x, ym = y, zm = z;
-            if (a == 0) {
-                xp = (x + 1 == nx) ? 0 : x + 1;
-                xm = (x == 0) ? nx - 1 : x - 1;
-            } else if (a == 1) {
-                yp = (y + 1 == ny) ? 0 : y + 1;
-                ym = (y == 0) ? ny - 1 : y - 1;
-            } else {
-                zp = (z + 1 == nz) ? 0 : z + 1;
-                zm = (z == 0) ? nz - 1 : z - 1;
-            }
-            const long long cp = cell(g, xp, yp, zp), cm = cell(g, xm, ym, zm);
-            float wh, wp;
-            if (A.mode == 0) {
-                const float f0 = A.fbar[c];
-                wh = A.s[a] * (f0 - A.fbar[cp]);
-                wp = A.s[a] * (A.fbar[cm] - f0);
-            } else {
-                const float* u = A.ubar + a * g.NP;
-                wh = A.s[a] * u[pcell(g, x, y, z)];
-                wp = A.s[a] * u[pcell(g, xm, ym, zm)];
-            }
-            const float4 pp = A.psi[cp], pm = A.psi[cm];
-            const float2 z1 = zpair(p0, pp);
+            const float4 pp = A.psi[cp[a]], pm = A.psi[cm[a]];
+            const float2 z1 = pair_z(p0, pp);
             const float n1 = z1.x * z1.x + z1.y * z1.y;
-            if (n1 > 0.f && wh != 0.f) {
-                const float t = wh / n1;
+            if (n1 > 0.f && wh[a] != 0.f) {
+                const float t = wh[a] / n1;
                 // -i conj(z1) pp_k
                 float mx = z1.x * pp.x + z1.y * pp.y, my = z1.x * pp.y - z1.y * pp.x;
                 acc.x += t * my;
@@ -184,10 +218,10 @@ __global__ void k_adj_oneform(AdjOneFormArgs A) {
                 acc.z += t * my;
                 acc.w -= t * mx;
             }
-            const float2 z2 = zpair(pm, p0);
+            const float2 z2 = pair_z(pm, p0);
             const float n2 = z2.x * z2.x + z2.y * z2.y;
-            if (n2 > 0.f && wp != 0.f) {
-                const float t = wp / n2;
+            if (n2 > 0.f && wp[a] != 0.f) {
+                const float t = wp[a] / n2;
                 // i z2 pm_k
                 float mx = z2.x * pm.x - z2.y * pm.y, my = z2.x * pm.y + z2.y * pm.x;
                 acc.x -= t * my;
@@ -207,17 +241,34 @@ __global__ void k_adj_oneform(AdjOneFormArgs A) {
 // -sum_k Im(conj(bar_k) out_k); acc[0..2] += phibar dphi/dk_a, acc[3] +=
 // -phibar wscale (the adjoint of omega t times wscale: t for the adjoint of
 // omega itself).
-__global__ void k_adj_restrict(Grid g, const float4* __restrict__ psi_in, float4* __restrict__ bar, JetArgs j,
-                               double* __restrict__ acc, float wscale) {
+//
+// With qsum, the restricted psi went into a projection whose qbar
+// (k_adj_gauge) sums to *qsum.  The projection turns a phase alpha per cell
+// into the single phase mean(alpha) (the one-form of alpha is exact and the
+// Poisson solve inverts its divergence but for the mean), so phibar is
+// -*qsum / N in every nozzle cell.  Left to the sum over cells it is what
+// remains of a cancellation between the gauge's and the one-form's parts, with
+// a relative error of 1e-6 to 1e-5 that changed from run to run (2^18
+// particles on 128x64x64); from the sum of qbar it is below 1e-6.
+template <bool PROJECTED>
+__global__ void __launch_bounds__(256) k_adj_restrict(Grid g, const float4* __restrict__ psi_in,
+                                                      float4* __restrict__ bar, JetArgs j, double* __restrict__ acc,
+                                                      float wscale, const double* __restrict__ qsum) {
+    pdl_enter();
     double v4[4] = {0.0, 0.0, 0.0, 0.0};
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode_cell(g, c, x, y, z);
+    bool any = false;
+    const int x = cell_x(), y = cell_y();
+    double phq = 0.0;
+    if constexpr (PROJECTED) phq = -*qsum * g.invN;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
+        if (x >= g.n[0] || y >= g.n[1]) break;
+        const long long c = cell(g, x, y, z);
         const float px = __fmul_rn((float)x, g.d[0]);
         const float py = __fmul_rn((float)y, g.d[1]);
         const float pz = __fmul_rn((float)z, g.d[2]);
         const bool jet = j.mask ? (j.mask[c] != 0) : isjet_f32(px, py, pz, j.cen, j.len, j.rad);
         if (!jet) continue;
+        any = true;
         float ph;
         if (j.phase_mode == 0)
             ph = __fadd_rn(__fadd_rn(__fadd_rn(j.kvec[0], px), __fadd_rn(j.kvec[1], py)), __fadd_rn(j.kvec[2], pz));
@@ -228,58 +279,39 @@ __global__ void k_adj_restrict(Grid g, const float4* __restrict__ psi_in, float4
         sincosf(ph, &s, &co);
         const float4 v = psi_in[c];
         const float a1 = hypotf(v.x, v.y), a2 = hypotf(v.z, v.w);
-        const float4 o = make_float4(a1 * co, a1 * s, a2 * co, a2 * s);
         const float4 gb = bar[c];
-        const float phb = -((gb.x * o.y - gb.y * o.x) + (gb.z * o.w - gb.w * o.z));
         const float r1 = gb.x * co + gb.y * s, r2 = gb.z * co + gb.w * s;
         const float i1 = a1 > 0.f ? r1 / a1 : 0.f, i2 = a2 > 0.f ? r2 / a2 : 0.f;
         bar[c] = make_float4(i1 * v.x, i1 * v.y, i2 * v.z, i2 * v.w);
+        double phb = phq;
+        if constexpr (!PROJECTED) {
+            const float4 o = make_float4(a1 * co, a1 * s, a2 * co, a2 * s);
+            phb = -((gb.x * o.y - gb.y * o.x) + (gb.z * o.w - gb.w * o.z));
+        }
         if (j.phase_mode == 0) {
             v4[0] += phb;
             v4[1] += phb;
             v4[2] += phb;
         } else {
-            v4[0] += (double)phb * px;
-            v4[1] += (double)phb * py;
-            v4[2] += (double)phb * pz;
+            v4[0] += phb * px;
+            v4[1] += phb * py;
+            v4[2] += phb * pz;
         }
-        v4[3] -= (double)phb * wscale;
+        v4[3] -= phb * wscale;
     }
-    block_sum_add<4>(v4, acc);
-}
-
-// Add the padded planes' periodic copies (x = nx, y = ny or z = nz) into the
-// cells they repeat and clear them: the cotangent of the one-form's stores.
-__global__ void k_adj_fold(Grid g, float* __restrict__ ubar) {
-    const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.NP; c += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(c % g.pnx);
-        const long long r = c / g.pnx;
-        const int y = (int)(r % (ny + 1)), z = (int)(r / (ny + 1));
-        if (x > nx || !(x == nx || y == ny || z == nz)) continue;
-        const int o = pcell(g, x == nx ? 0 : x, y == ny ? 0 : y, z == nz ? 0 : z);
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            float* u = ubar + a * g.NP;
-            const float v = u[c];
-            if (v != 0.f) atomicAdd(&u[o], v);
-            u[c] = 0.f;
-        }
-    }
+    if (__syncthreads_or(any)) block_sum_add<4>(v4, acc);  // most blocks lie outside the nozzle
 }
 
 namespace {
 
-// one staggered sample with everything its adjoint needs
+// one staggered sample: its base cell and weights
 struct Sample {
-    int c000;
-    float w[3];
-    float v[12];  // x00 x10 x01 x11 | y00 y10 y01 y11 | z00 z10 z01 z11
-    float3 u;
+    int c;
+    float wx, wy, wz;
 };
 
 template <bool POW2, bool NORMW>
-__device__ __forceinline__ void stag_sample(const AdvConst& k, float3 pt, Sample& S) {
+__device__ __forceinline__ Sample stag_sample(const AdvConst& k, float3 pt) {
     float P[3] = {pt.x, pt.y, pt.z};
     const bool inbox = (pt.x >= 0.f && pt.x < k.L[0]) && (pt.y >= 0.f && pt.y < k.L[1]) &&
                        (pt.z >= 0.f && pt.z < k.L[2]);
@@ -288,53 +320,71 @@ __device__ __forceinline__ void stag_sample(const AdvConst& k, float3 pt, Sample
         for (int a = 0; a < 3; ++a) P[a] = jl_mod_box(P[a], k.L[a]);
     }
     int i[3];
+    float w[3];
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         int ii = cell_floor<POW2>(P[a], k.dinv[a], k.d[a], k.feps[a]);
         ii = max(min(ii, k.nm[a]), 0);
         i[a] = ii;
-        S.w[a] = __fsub_rn(P[a], __fmul_rn((float)ii, k.d[a]));
-        if (NORMW) S.w[a] = __fdiv_rn(S.w[a], k.d[a]);
+        w[a] = __fsub_rn(P[a], __fmul_rn((float)ii, k.d[a]));
+        if (NORMW) w[a] = __fdiv_rn(w[a], k.d[a]);
     }
-    const int sy = k.pnx, sz = k.pnxy;
-    const int c000 = i[0] + sy * i[1] + sz * i[2];
-    S.c000 = c000;
-    const int c100 = c000 + 1, c010 = c000 + sy, c001 = c000 + sz;
-    const float4 a000 = __ldg(k.v + c000), a100 = __ldg(k.v + c100), a010 = __ldg(k.v + c010);
-    const float4 a001 = __ldg(k.v + c001), a011 = __ldg(k.v + c010 + sz), a101 = __ldg(k.v + c100 + sz);
-    const float4 a110 = __ldg(k.v + c100 + sy);
-    S.v[0] = a000.x;
-    S.v[1] = a010.x;
-    S.v[2] = a001.x;
-    S.v[3] = a011.x;
-    S.v[4] = a000.y;
-    S.v[5] = a100.y;
-    S.v[6] = a001.y;
-    S.v[7] = a101.y;
-    S.v[8] = a000.z;
-    S.v[9] = a100.z;
-    S.v[10] = a010.z;
-    S.v[11] = a110.z;
-    const float wx = S.w[0], wy = S.w[1], wz = S.w[2];
-    S.u.x = (1.f - wz) * ((1.f - wy) * S.v[0] + wy * S.v[1]) + wz * ((1.f - wy) * S.v[2] + wy * S.v[3]);
-    S.u.y = (1.f - wz) * ((1.f - wx) * S.v[4] + wx * S.v[5]) + wz * ((1.f - wx) * S.v[6] + wx * S.v[7]);
-    S.u.z = (1.f - wy) * ((1.f - wx) * S.v[8] + wx * S.v[9]) + wy * ((1.f - wx) * S.v[10] + wx * S.v[11]);
+    return Sample{i[0] + k.pnx * i[1] + k.pnxy * i[2], w[0], w[1], w[2]};
+}
+
+// v <- the twelve velocity samples of cell c, unless it holds them already
+__device__ __forceinline__ void hold_cell(const AdvConst& k, int c, CellVel& v) {
+    if (c == v.c) return;
+    v.c = c;
+    const float4* b0 = k.v + c;
+    const float4* by = b0 + k.pnx;
+    const float4* bz = b0 + k.pnxy;
+    const float4 a000 = __ldg(b0), a100 = __ldg(b0 + 1), a010 = __ldg(by), a001 = __ldg(bz);
+    const float4 a011 = __ldg(by + k.pnxy), a101 = __ldg(bz + 1), a110 = __ldg(by + 1);
+    v.x00 = a000.x, v.x10 = a010.x, v.x01 = a001.x, v.x11 = a011.x;
+    v.y00 = a000.y, v.y10 = a100.y, v.y01 = a001.y, v.y11 = a101.y;
+    v.z00 = a000.z, v.z10 = a100.z, v.z01 = a010.z, v.z11 = a110.z;
+}
+
+__device__ __forceinline__ float3 sample_u(const CellVel& v, const Sample& s) {
+    const float wx = s.wx, wy = s.wy, wz = s.wz;
+    float3 u;
+    u.x = (1.f - wz) * ((1.f - wy) * v.x00 + wy * v.x10) + wz * ((1.f - wy) * v.x01 + wy * v.x11);
+    u.y = (1.f - wz) * ((1.f - wx) * v.y00 + wx * v.y10) + wz * ((1.f - wx) * v.y01 + wx * v.y11);
+    u.z = (1.f - wy) * ((1.f - wx) * v.z00 + wx * v.z10) + wy * ((1.f - wx) * v.z01 + wx * v.z11);
+    return u;
+}
+
+// add the cotangents of cell b.c's twelve samples into the padded velocity
+// cotangent: the cells with two or three of them as one vector reduction each
+__device__ __forceinline__ void flush_cell(const AdvConst& k, const CellVel& b, float4* __restrict__ ubar) {
+    float4* u0 = ubar + b.c;
+    float4* uy = u0 + k.pnx;
+    float4* uz = u0 + k.pnxy;
+    atomicAdd(u0, make_float4(b.x00, b.y00, b.z00, 0.f));
+    atomicAdd(u0 + 1, make_float4(0.f, b.y10, b.z10, 0.f));
+    atomicAdd(uy, make_float4(b.x10, 0.f, b.z01, 0.f));
+    atomicAdd(uz, make_float4(b.x01, b.y01, 0.f, 0.f));
+    atomicAdd(&uy[k.pnxy].x, b.x11);
+    atomicAdd(&uz[1].y, b.y11);
+    atomicAdd(&uy[1].z, b.z11);
 }
 
 // adjoint of one sample: ub = cotangent of u; returns the cotangent of the
-// sample point and scatters ub times the weights into the velocity cotangent planes
+// sample point and adds ub times the weights to b, the cotangents of the
+// sample's cell (b of another cell goes to memory first)
 template <bool NORMW>
-__device__ __forceinline__ float3 stag_sample_adj(const AdvConst& k, const Sample& S, float3 ub, float* ubx, float* uby,
-                                                  float* ubz) {
-    const float wx = S.w[0], wy = S.w[1], wz = S.w[2];
-    const float* v = S.v;
+__device__ __forceinline__ float3 stag_sample_adj(const AdvConst& k, const Sample& s, float3 ub, CellVel& v, CellVel& b,
+                                                  float4* __restrict__ ubar) {
+    hold_cell(k, s.c, v);
+    const float wx = s.wx, wy = s.wy, wz = s.wz;
     // d u / d w (the weights are unnormalised: dw/dp = 1)
-    const float dux_dwy = (1.f - wz) * (v[1] - v[0]) + wz * (v[3] - v[2]);
-    const float dux_dwz = ((1.f - wy) * v[2] + wy * v[3]) - ((1.f - wy) * v[0] + wy * v[1]);
-    const float duy_dwx = (1.f - wz) * (v[5] - v[4]) + wz * (v[7] - v[6]);
-    const float duy_dwz = ((1.f - wx) * v[6] + wx * v[7]) - ((1.f - wx) * v[4] + wx * v[5]);
-    const float duz_dwx = (1.f - wy) * (v[9] - v[8]) + wy * (v[11] - v[10]);
-    const float duz_dwy = ((1.f - wx) * v[10] + wx * v[11]) - ((1.f - wx) * v[8] + wx * v[9]);
+    const float dux_dwy = (1.f - wz) * (v.x10 - v.x00) + wz * (v.x11 - v.x01);
+    const float dux_dwz = ((1.f - wy) * v.x01 + wy * v.x11) - ((1.f - wy) * v.x00 + wy * v.x10);
+    const float duy_dwx = (1.f - wz) * (v.y10 - v.y00) + wz * (v.y11 - v.y01);
+    const float duy_dwz = ((1.f - wx) * v.y01 + wx * v.y11) - ((1.f - wx) * v.y00 + wx * v.y10);
+    const float duz_dwx = (1.f - wy) * (v.z10 - v.z00) + wy * (v.z11 - v.z01);
+    const float duz_dwy = ((1.f - wx) * v.z01 + wx * v.z11) - ((1.f - wx) * v.z00 + wx * v.z10);
     float3 pb;
     pb.x = ub.y * duy_dwx + ub.z * duz_dwx;
     pb.y = ub.x * dux_dwy + ub.z * duz_dwy;
@@ -344,26 +394,25 @@ __device__ __forceinline__ float3 stag_sample_adj(const AdvConst& k, const Sampl
         pb.y *= k.dinv[1];
         pb.z *= k.dinv[2];
     }
-    const int sy = k.pnx, sz = k.pnxy;
-    const int c000 = S.c000, c100 = c000 + 1, c010 = c000 + sy, c001 = c000 + sz;
-    if (ub.x != 0.f) {
-        atomicAdd(ubx + c000, ub.x * (1.f - wz) * (1.f - wy));
-        atomicAdd(ubx + c010, ub.x * (1.f - wz) * wy);
-        atomicAdd(ubx + c001, ub.x * wz * (1.f - wy));
-        atomicAdd(ubx + c010 + sz, ub.x * wz * wy);
+    if (s.c != b.c) {
+        if (b.c >= 0) flush_cell(k, b, ubar);
+        b.c = s.c;
+        b.x00 = b.x10 = b.x01 = b.x11 = 0.f;
+        b.y00 = b.y10 = b.y01 = b.y11 = 0.f;
+        b.z00 = b.z10 = b.z01 = b.z11 = 0.f;
     }
-    if (ub.y != 0.f) {
-        atomicAdd(uby + c000, ub.y * (1.f - wz) * (1.f - wx));
-        atomicAdd(uby + c100, ub.y * (1.f - wz) * wx);
-        atomicAdd(uby + c001, ub.y * wz * (1.f - wx));
-        atomicAdd(uby + c100 + sz, ub.y * wz * wx);
-    }
-    if (ub.z != 0.f) {
-        atomicAdd(ubz + c000, ub.z * (1.f - wy) * (1.f - wx));
-        atomicAdd(ubz + c100, ub.z * (1.f - wy) * wx);
-        atomicAdd(ubz + c010, ub.z * wy * (1.f - wx));
-        atomicAdd(ubz + c100 + sy, ub.z * wy * wx);
-    }
+    b.x00 += ub.x * (1.f - wz) * (1.f - wy);
+    b.x10 += ub.x * (1.f - wz) * wy;
+    b.x01 += ub.x * wz * (1.f - wy);
+    b.x11 += ub.x * wz * wy;
+    b.y00 += ub.y * (1.f - wz) * (1.f - wx);
+    b.y10 += ub.y * (1.f - wz) * wx;
+    b.y01 += ub.y * wz * (1.f - wx);
+    b.y11 += ub.y * wz * wx;
+    b.z00 += ub.z * (1.f - wy) * (1.f - wx);
+    b.z10 += ub.z * (1.f - wy) * wx;
+    b.z01 += ub.z * wy * (1.f - wx);
+    b.z11 += ub.z * wy * wx;
     return pb;
 }
 
@@ -375,15 +424,16 @@ __device__ __forceinline__ float3 f3scale(float3 a, float s) { return make_float
 // Reverse of one RK4 advection (staggered_advect!, parallel.jl:197-216):
 // lam holds the cotangent of the positions after the step and becomes that
 // of the positions before it (parts, the positions the forward step started
-// from); the cotangent of the velocity planes is added into ubar.  A slot
-// outside the open box was set to (-1,-1,-1): its cotangent is 0.
+// from); the cotangent of the padded velocity (float4 per cell) is added into
+// ubar.  A slot outside the open box was set to (-1,-1,-1): its cotangent is 0.
+// Bound by the reductions into ubar: the four stages of a particle lie in one
+// or two cells, so their cotangents are summed per cell in registers and leave
+// as 7 reductions instead of 12 scalar ones per stage.
 template <bool POW2, bool NORMW>
 __global__ void __launch_bounds__(256) k_adj_advect(Grid g, const float* __restrict__ parts, float* __restrict__ lam,
-                                                    int np, const float* __restrict__ vel, float* __restrict__ ubar) {
+                                                    int np, const float* __restrict__ vel, float4* __restrict__ ubar) {
+    pdl_enter();
     const AdvConst kc = adv_const(g, vel);
-    float* ubx = ubar;
-    float* uby = ubar + g.NP;
-    float* ubz = ubar + 2 * g.NP;
     const float dt = g.dt, s6 = g.dt / 6.0f;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x) {
         const float3 p = make_float3(parts[3 * k], parts[3 * k + 1], parts[3 * k + 2]);
@@ -393,33 +443,39 @@ __global__ void __launch_bounds__(256) k_adj_advect(Grid g, const float* __restr
             lam[3 * k] = lam[3 * k + 1] = lam[3 * k + 2] = 0.f;
             continue;
         }
-        Sample S1, S2, S3, S4;
-        stag_sample<POW2, NORMW>(kc, p, S1);
-        const float3 k1 = S1.u;
+        CellVel v, b;
+        v.c = b.c = -1;
+        auto at = [&](const Sample& s) {
+            hold_cell(kc, s.c, v);
+            return sample_u(v, s);
+        };
+        const Sample S1 = stag_sample<POW2, NORMW>(kc, p);
+        const float3 k1 = at(S1);
         float3 q = make_float3(p.x + k1.x * dt * 0.5f, p.y + k1.y * dt * 0.5f, p.z + k1.z * dt * 0.5f);
-        stag_sample<POW2, NORMW>(kc, q, S2);
-        const float3 k2 = S2.u;
+        const Sample S2 = stag_sample<POW2, NORMW>(kc, q);
+        const float3 k2 = at(S2);
         q = make_float3(p.x + k2.x * dt * 0.5f, p.y + k2.y * dt * 0.5f, p.z + k2.z * dt * 0.5f);
-        stag_sample<POW2, NORMW>(kc, q, S3);
-        const float3 k3 = S3.u;
+        const Sample S3 = stag_sample<POW2, NORMW>(kc, q);
+        const float3 k3 = at(S3);
         q = make_float3(p.x + k3.x * dt, p.y + k3.y * dt, p.z + k3.z * dt);
-        stag_sample<POW2, NORMW>(kc, q, S4);
+        const Sample S4 = stag_sample<POW2, NORMW>(kc, q);
         // reverse of p' = p + dt/6 (k1 + 2 k2 + 2 k3 + k4)
         const float3 L = make_float3(lam[3 * k], lam[3 * k + 1], lam[3 * k + 2]);
         float3 pb = L;
         float3 kb1 = f3scale(L, s6), kb2 = f3scale(L, 2.f * s6), kb3 = f3scale(L, 2.f * s6);
         const float3 kb4 = f3scale(L, s6);
-        float3 qb = stag_sample_adj<NORMW>(kc, S4, kb4, ubx, uby, ubz);  // q4 = p + dt k3
+        float3 qb = stag_sample_adj<NORMW>(kc, S4, kb4, v, b, ubar);  // q4 = p + dt k3
         pb = f3add(pb, qb);
         kb3 = f3add(kb3, f3scale(qb, dt));
-        qb = stag_sample_adj<NORMW>(kc, S3, kb3, ubx, uby, ubz);  // q3 = p + dt/2 k2
+        qb = stag_sample_adj<NORMW>(kc, S3, kb3, v, b, ubar);  // q3 = p + dt/2 k2
         pb = f3add(pb, qb);
         kb2 = f3add(kb2, f3scale(qb, 0.5f * dt));
-        qb = stag_sample_adj<NORMW>(kc, S2, kb2, ubx, uby, ubz);  // q2 = p + dt/2 k1
+        qb = stag_sample_adj<NORMW>(kc, S2, kb2, v, b, ubar);  // q2 = p + dt/2 k1
         pb = f3add(pb, qb);
         kb1 = f3add(kb1, f3scale(qb, 0.5f * dt));
-        qb = stag_sample_adj<NORMW>(kc, S1, kb1, ubx, uby, ubz);  // k1 at p
+        qb = stag_sample_adj<NORMW>(kc, S1, kb1, v, b, ubar);  // k1 at p
         pb = f3add(pb, qb);
+        flush_cell(kc, b, ubar);
         lam[3 * k] = pb.x;
         lam[3 * k + 1] = pb.y;
         lam[3 * k + 2] = pb.z;
@@ -430,6 +486,7 @@ __global__ void __launch_bounds__(256) k_adj_advect(Grid g, const float* __restr
 // lam = dL/dx = 2 (x - y), 0 for dead slots
 __global__ void k_loss(const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ lam, int np,
                        double* __restrict__ loss) {
+    pdl_enter();
     double v[1] = {0.0};
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < np; k += gridDim.x * blockDim.x) {
         const bool alive = x[3 * k] >= 0.f;
@@ -443,33 +500,35 @@ __global__ void k_loss(const float* __restrict__ x, const float* __restrict__ y,
     block_sum_add<1>(v, loss);
 }
 
-// velocity-plane cotangent from AoS float3 per cell: the cells themselves
-// only (the periodic copies stay 0)
-__global__ void k_adj_from_aos(Grid g, const float* __restrict__ aos, float* __restrict__ ubar) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode_cell(g, c, x, y, z);
-        const int pc = pcell(g, x, y, z);
-        ubar[pc] = aos[3 * c];
-        ubar[g.NP + pc] = aos[3 * c + 1];
-        ubar[2 * g.NP + pc] = aos[3 * c + 2];
+// velocity cotangent from AoS float3 per cell: the cells themselves only (the
+// periodic copies stay 0)
+__global__ void __launch_bounds__(256) k_adj_from_aos(Grid g, const float* __restrict__ aos, float4* __restrict__ ubar) {
+    pdl_enter();
+    const int x = cell_x(), y = cell_y();
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
+        const long long c = cell(g, x, y, z);
+        ubar[pcell(g, x, y, z)] = make_float4(aos[3 * c], aos[3 * c + 1], aos[3 * c + 2], 0.f);
     }
 }
 
-// the velocity cotangent (three padded planes, folded) as AoS float3 per cell
-__global__ void k_adj_to_aos(Grid g, const float* __restrict__ ubar, float* __restrict__ aos) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode_cell(g, c, x, y, z);
-        const int pc = pcell(g, x, y, z);
-        aos[3 * c] = ubar[pc];
-        aos[3 * c + 1] = ubar[g.NP + pc];
-        aos[3 * c + 2] = ubar[2 * g.NP + pc];
+// the velocity cotangent (padded, its copies collected) as AoS float3 per cell
+__global__ void __launch_bounds__(256) k_adj_to_aos(Grid g, const float4* __restrict__ ubar, float* __restrict__ aos) {
+    pdl_enter();
+    const int x = cell_x(), y = cell_y();
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
+        const long long c = cell(g, x, y, z);
+        const float4 v = ubar_at(g, ubar, x, y, z);
+        aos[3 * c] = v.x;
+        aos[3 * c + 1] = v.y;
+        aos[3 * c + 2] = v.z;
     }
 }
 
 // cotangent 0 for the ring slots an emission overwrote
 __global__ void k_zero_slots(float* __restrict__ lam, long long nslots, long long start, long long count) {
+    pdl_enter();
     const long long j = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (j >= count) return;
     const long long s = (start + j) % nslots;
@@ -479,25 +538,25 @@ __global__ void k_zero_slots(float* __restrict__ lam, long long nslots, long lon
 // ---------------------------------------------------------------- launchers
 
 cudaError_t launch_gauge(const Grid& g, const float4* in, const float* q, float4* out, cudaStream_t s) {
-    k_gauge<<<grid_n(g.N, 256), 256, 0, s>>>(in, q, out, g.N);
-    return cudaGetLastError();
+    return launch_pdl(k_gauge, dim3(grid_n(g.N, 256)), dim3(256), 0, s, in, q, out, g.N);
 }
 cudaError_t launch_normalize_to(const Grid& g, const float4* in, float4* out, cudaStream_t s) {
-    k_normalize_to<<<grid_n(g.N, 256), 256, 0, s>>>(in, out, g.N);
-    return cudaGetLastError();
+    return launch_pdl(k_normalize_to, dim3(grid_n(g.N, 256)), dim3(256), 0, s, in, out, g.N);
 }
 cudaError_t launch_restrict_to(const Grid& g, const float4* in, float4* out, const JetArgs& j, cudaStream_t s) {
-    k_restrict_to<<<grid_n(g.N, 256), 256, 0, s>>>(g, in, out, j);
-    return cudaGetLastError();
+    return launch_pdl(k_restrict_to<false>, cell_grid(g), dim3(256), 0, s, g, in, (const float*)nullptr,
+                      (float4*)nullptr, out, j);
+}
+cudaError_t launch_gauge_restrict(const Grid& g, const float4* in, const float* q, float4* mid, float4* out,
+                                  const JetArgs& j, cudaStream_t s) {
+    return launch_pdl(k_restrict_to<true>, cell_grid(g), dim3(256), 0, s, g, in, q, mid, out, j);
 }
 cudaError_t launch_adj_normalize(const Grid& g, const float4* psi_in, float4* bar, cudaStream_t s) {
-    k_adj_normalize<<<grid_n(g.N, 256), 256, 0, s>>>(psi_in, bar, g.N);
-    return cudaGetLastError();
+    return launch_pdl(k_adj_normalize, dim3(grid_n(g.N, 256)), dim3(256), 0, s, psi_in, bar, g.N);
 }
-cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar,
-                             cudaStream_t s) {
-    k_adj_gauge<<<grid_n(g.N, 256), 256, 0, s>>>(psi_in, q, bar, qbar, g.N);
-    return cudaGetLastError();
+cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar, double* sum,
+                             double* clear, cudaStream_t s) {
+    return launch_pdl(k_adj_gauge, dim3(grid_n(g.N, 256)), dim3(256), 0, s, psi_in, q, bar, qbar, g.N, sum, clear);
 }
 cudaError_t launch_adj_oneform_div(const Grid& g, const float4* psi, float4* bar, const float* fbar, cudaStream_t s) {
     AdjOneFormArgs a;
@@ -507,15 +566,10 @@ cudaError_t launch_adj_oneform_div(const Grid& g, const float4* psi, float4* bar
     a.fbar = fbar;
     a.ubar = nullptr;
     for (int k = 0; k < 3; ++k) a.s[k] = g.inv_d2[k];
-    a.mode = 0;
-    k_adj_oneform<<<grid_n(g.N, 256), 256, 0, s>>>(a);
-    return cudaGetLastError();
+    return launch_pdl(k_adj_oneform<true>, cell_grid(g), dim3(256), 0, s, a);
 }
-cudaError_t launch_adj_oneform_vel(const Grid& g, const float4* psi, float4* bar, float* ubar, float hbar, int sharp,
-                                   cudaStream_t s) {
-    k_adj_fold<<<grid_n(g.NP, 256), 256, 0, s>>>(g, ubar);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+cudaError_t launch_adj_oneform_vel(const Grid& g, const float4* psi, float4* bar, const float4* ubar, float hbar,
+                                   int sharp, cudaStream_t s) {
     AdjOneFormArgs a;
     a.g = g;
     a.psi = psi;
@@ -523,51 +577,38 @@ cudaError_t launch_adj_oneform_vel(const Grid& g, const float4* psi, float4* bar
     a.fbar = nullptr;
     a.ubar = ubar;
     for (int k = 0; k < 3; ++k) a.s[k] = sharp ? hbar * g.dinv[k] : hbar;
-    a.mode = 1;
-    k_adj_oneform<<<grid_n(g.N, 256), 256, 0, s>>>(a);
-    return cudaGetLastError();
-}
-cudaError_t launch_adj_fold(const Grid& g, float* ubar, cudaStream_t s) {
-    k_adj_fold<<<grid_n(g.NP, 256), 256, 0, s>>>(g, ubar);
-    return cudaGetLastError();
+    return launch_pdl(k_adj_oneform<false>, cell_grid(g), dim3(256), 0, s, a);
 }
 cudaError_t launch_adj_restrict(const Grid& g, const float4* psi_in, float4* bar, const JetArgs& j, double* acc,
-                                float wscale, cudaStream_t s) {
-    k_adj_restrict<<<grid_n(g.N, 256), 256, 0, s>>>(g, psi_in, bar, j, acc, wscale);
-    return cudaGetLastError();
+                                float wscale, const double* qsum, cudaStream_t s) {
+    return launch_pdl(qsum ? k_adj_restrict<true> : k_adj_restrict<false>, cell_grid(g), dim3(256), 0, s, g, psi_in, bar,
+                      j, acc, wscale, qsum);
 }
 cudaError_t launch_adj_advect(const Grid& g, const float* parts, float* lam, long long np, const float* vel,
-                              float* ubar, cudaStream_t s) {
+                              float4* ubar, cudaStream_t s) {
     if (np <= 0) return cudaSuccess;
     if (np > kMaxParticles) return cudaErrorInvalidValue;
-    const unsigned b = grid_n(np, 256);
     const bool pow2 = g.d_pow2[0] && g.d_pow2[1] && g.d_pow2[2];
-    if (g.norm_w) {
-        if (pow2) k_adj_advect<true, true><<<b, 256, 0, s>>>(g, parts, lam, (int)np, vel, ubar);
-        else k_adj_advect<false, true><<<b, 256, 0, s>>>(g, parts, lam, (int)np, vel, ubar);
-    } else {
-        if (pow2) k_adj_advect<true, false><<<b, 256, 0, s>>>(g, parts, lam, (int)np, vel, ubar);
-        else k_adj_advect<false, false><<<b, 256, 0, s>>>(g, parts, lam, (int)np, vel, ubar);
-    }
-    return cudaGetLastError();
+    auto go = [&](auto kernel) {
+        return launch_pdl(kernel, dim3(grid_n(np, 256)), dim3(256), 0, s, g, parts, lam, (int)np, vel, ubar);
+    };
+    if (g.norm_w) return pow2 ? go(k_adj_advect<true, true>) : go(k_adj_advect<false, true>);
+    return pow2 ? go(k_adj_advect<true, false>) : go(k_adj_advect<false, false>);
 }
 cudaError_t launch_loss(const float* x, const float* y, float* lam, long long np, double* loss, cudaStream_t s) {
     if (np <= 0) return cudaSuccess;
-    k_loss<<<grid_n(np, 256), 256, 0, s>>>(x, y, lam, (int)np, loss);
-    return cudaGetLastError();
+    return launch_pdl(k_loss, dim3(grid_n(np, 256)), dim3(256), 0, s, x, y, lam, (int)np, loss);
 }
-cudaError_t launch_adj_from_aos(const Grid& g, const float* aos, float* ubar, cudaStream_t s) {
-    k_adj_from_aos<<<grid_n(g.N, 256), 256, 0, s>>>(g, aos, ubar);
-    return cudaGetLastError();
+cudaError_t launch_adj_from_aos(const Grid& g, const float* aos, float4* ubar, cudaStream_t s) {
+    return launch_pdl(k_adj_from_aos, cell_grid(g), dim3(256), 0, s, g, aos, ubar);
 }
-cudaError_t launch_adj_to_aos(const Grid& g, const float* ubar, float* aos, cudaStream_t s) {
-    k_adj_to_aos<<<grid_n(g.N, 256), 256, 0, s>>>(g, ubar, aos);
-    return cudaGetLastError();
+cudaError_t launch_adj_to_aos(const Grid& g, const float4* ubar, float* aos, cudaStream_t s) {
+    return launch_pdl(k_adj_to_aos, cell_grid(g), dim3(256), 0, s, g, ubar, aos);
 }
 cudaError_t launch_zero_slots(float* lam, long long nslots, long long start, long long count, cudaStream_t s) {
     if (count <= 0) return cudaSuccess;
-    k_zero_slots<<<(unsigned)((count + 255) / 256), 256, 0, s>>>(lam, nslots, start % nslots, count);
-    return cudaGetLastError();
+    return launch_pdl(k_zero_slots, dim3((unsigned)((count + 255) / 256)), dim3(256), 0, s, lam, nslots, start % nslots,
+                      count);
 }
 
 }  // namespace isf

@@ -82,3 +82,53 @@ def test_real_x_passes(isfpkg, oracle_mod, L, dims):
     isf.sync()
     orc.set_f(f)
     assert rel(host(q), orc.poisson_solve().real) < 1e-5
+
+
+# adjoint kernels over 32 x 8 cell tiles and z walks: partial tiles, a grid
+# thinner than a tile, and one with more planes than blocks along z; the
+# advection's cotangent with particles that stay in their cell and that leave it
+@pytest.mark.parametrize("L,dims", [((1, 1, 1), (8, 12, 20)), ((2, 2, 2), (50, 20, 56)), ((8, 2, 4), (256, 48, 100))])
+@pytest.mark.parametrize("cells_per_step", [0.05, 3.0])
+def test_adj_advect_uniform_velocity(isfpkg, L, dims, cells_per_step):
+    """A uniform velocity u is sampled as itself, so p' = p + dt u: the
+    cotangents of all samples sum to dt times that of the particles, and the
+    positions' cotangent passes through."""
+    isf = isfpkg.ISF(L, dims, HBAR, DT)
+    rng = np.random.default_rng(51)
+    P = 5003
+    d = [length / n for length, n in zip(L, dims)]
+    u = np.array([cells_per_step, -0.6 * cells_per_step, 0.3 * cells_per_step]) * min(d) / DT
+    # away from the box walls: no particle dies
+    p = (0.35 + 0.3 * rng.uniform(0, 1, (P, 3))) * np.asarray(L)
+    w = rng.normal(size=(P, 3)).astype(np.float32)
+    isf.velocity = cuda(np.broadcast_to(u.astype(np.float32), dims[::-1] + (3,)))
+    bar = cuda(w)
+    isfpkg.adj_staggered_advect(isf, cuda(p), bar)
+    ub = host(isfpkg.get_velocity_bar(isf))
+    want = DT * w.astype(np.float64).sum(axis=0)
+    scale = DT * np.abs(w).sum(axis=0)
+    assert (np.abs(ub.sum(axis=(0, 1, 2)) - want) <= 1e-5 * scale).all()
+    assert (np.abs(host(bar) - w) <= 1e-5 * np.abs(w).max()).all()
+
+
+@pytest.mark.parametrize("L,dims", [((1, 1, 1), (12, 8, 20)), ((2, 1, 2), (50, 20, 40))])
+def test_adj_project_and_one_form_on_partial_tiles(isfpkg, oracle_mod, L, dims):
+    """The projection's and the velocity one-form's transposes against central
+    differences of the FP64 oracle along a random direction."""
+    isf = isfpkg.ISF(L, dims, HBAR, DT)
+    orc = oracle_mod.Oracle(L, dims, HBAR, DT)
+    rng = np.random.default_rng(52)
+    x = smooth_psi(dims, seed=52, phase_scale=0.5).astype(np.float32).astype(np.float64)
+    u, w = rng.normal(size=x.shape), rng.normal(size=x.shape).astype(np.float32)
+    h = 1e-6
+    t = cuda(w)
+    isfpkg.adj_pressure_project(isf, cuda(x), t)
+    g = (w * (orc.pressure_project(x + h * u) - orc.pressure_project(x - h * u))).sum() / (2 * h)
+    assert abs((host(t) * u).sum() - g) <= 1e-3 * abs(g) + 1e-6 * np.linalg.norm(w) * np.linalg.norm(u)
+    wv = rng.normal(size=dims[::-1] + (3,)).astype(np.float32)
+    isfpkg.set_velocity_bar(isf, cuda(wv))
+    assert np.array_equal(host(isfpkg.get_velocity_bar(isf)), wv)
+    t = torch.zeros(x.shape, device="cuda")
+    isfpkg.adj_velocity_one_form(isf, cuda(x), t, HBAR)
+    g = (wv * (orc.velocity_one_form(x + h * u, HBAR) - orc.velocity_one_form(x - h * u, HBAR))).sum() / (2 * h)
+    assert abs((host(t) * u).sum() - g) <= 1e-3 * abs(g) + 1e-6 * np.linalg.norm(wv) * np.linalg.norm(u)
