@@ -1,6 +1,7 @@
 // C ABI of libisf (declared in include/isf.h): the ISF handle, its device
 // tables and temporaries, and the kernel sequences behind each reference
 // operator.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -422,7 +423,10 @@ int isf_create(const isf_params* p, isf_handle** out) {
         for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaEventCreateWithFlags(&h->ev_read[i], cudaEventDisableTiming);
         if (e != cudaSuccess) return cleanup(ISF_ERR_CUDA, std::string("isf_create: particle stream: ") + cudaGetErrorString(e));
     }
-    if (cudaMalloc(&h->F, sizeof(float2) * g.N) != cudaSuccess || cudaMalloc(&h->f, sizeof(float) * g.N) != cudaSuccess ||
+    // the half spectrum: a row of wp >= nx / 2 + 1 values per (y, z); rows of 8
+    // and 12 cells are padded beyond nx
+    const long long nF = std::max(g.N, (long long)h->wp * g.n[1] * g.n[2]);
+    if (cudaMalloc(&h->F, sizeof(float2) * nF) != cudaSuccess || cudaMalloc(&h->f, sizeof(float) * g.N) != cudaSuccess ||
         cudaMalloc(&h->vel_buf[0], sizeof(float) * kVelComp * g.NP) != cudaSuccess ||
         cudaMalloc(&h->vel_buf[1], sizeof(float) * kVelComp * g.NP) != cudaSuccess ||
         cudaMalloc(&h->tables, total) != cudaSuccess ||
@@ -434,7 +438,7 @@ int isf_create(const isf_params* p, isf_handle** out) {
     if (e == cudaSuccess) e = cudaMemset(h->counters, 0, 16 * sizeof(unsigned long long));
     for (int i = 0; i < 2 && e == cudaSuccess; ++i) e = cudaMemset(h->vel_buf[i], 0, sizeof(float) * kVelComp * g.NP);
     h->vel = h->vel_buf[0];
-    if (e == cudaSuccess) e = cudaMemset(h->F, 0, sizeof(float2) * g.N);
+    if (e == cudaSuccess) e = cudaMemset(h->F, 0, sizeof(float2) * nF);
     if (e != cudaSuccess) return cleanup(ISF_ERR_CUDA, std::string("isf_create: upload: ") + cudaGetErrorString(e));
     bind_tables(g, reinterpret_cast<const char*>(h->tables));
     *out = h;

@@ -15,7 +15,7 @@ struct isf_handle {
     int device = 0;
     cudaStream_t stream = nullptr;
     bool own_stream = false;
-    float2* F = nullptr;     // Poisson half spectrum (wp x ny x nz complex), N allocated
+    float2* F = nullptr;     // Poisson half spectrum: wp x ny x nz complex, at least N allocated
     int wp = 0;              // padded half-spectrum row: round_up(nx/2 + 1, 16)
     int flags = 0;           // ISF_FLAG_* of isf_create
     int kmajor = 0;          // the half spectrum is k-major and solved plane by plane (plane_supported)
