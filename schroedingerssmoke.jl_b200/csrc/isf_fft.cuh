@@ -12,13 +12,8 @@
 // (global memory, with all loads of a thread issued back to back) and the
 // last stage scatters straight to the caller's sink, so only the stage
 // boundaries in between go through shared memory: one [N][C] tile per CTA,
-// in place (a barrier after every gather and after every scatter).  The
-// tile stores element (j, q) of pencil q at j*C + (q ^ ((j ^ (j >> 3)) mod C)):
-// row-wise accesses (y/z passes: lanes over q) are conflict free for any
-// swizzle since C * sizeof(T) is 128 bytes; this one also keeps the
-// column-wise stage accesses of the x pass (lanes over j, strides 1, R and
-// the grouped p-strides) within 1.04 x the ideal wavefront count for every
-// radix plan (simulated per quarter / half warp for 16- / 8-byte elements).
+// in place (a barrier after every gather and after every scatter), in one of
+// the layouts below.
 //
 // Forward transforms use S = -1 (unnormalised), inverse S = +1 (the 1/N of
 // the reference's ifft is folded into the spectral multiply by the callers).
@@ -29,27 +24,68 @@
 
 namespace isf {
 
-//
-// A tile of 4 pencils (the real x passes) has too few columns for a swizzle
-// to spread the stage strides; it stores pencil after pencil with one
-// element of padding every 8 (stride-8 accesses fall into distinct banks) at a
-// pitch that sets the pencils of a half warp side by side (NT lanes each).
-template <int N, int NT>
-constexpr int quad_pitch() {
-    const int rem = NT < 16 ? (NT & ~1) : 4;  // wanted pitch mod 16 (8-byte elements)
-    int p = N + N / 8;
-    while (p % 16 != rem) ++p;
-    return p;
-}
-template <int C, int N, int NT>
-__device__ __forceinline__ int sidx(int j, int q) {
-    static_assert(C == 4 || C == 8 || C == 16, "tile width");
-    if constexpr (C == 4) return q * quad_pitch<N, NT>() + j + (j >> 3);
-    else return j * C + (q ^ ((j ^ (j >> 3)) & (C - 1)));
-}
-// elements of a tile of C pencils
-template <int C, int N, int NT>
-constexpr int tile_elems() { return C == 4 ? 4 * quad_pitch<N, NT>() : N * C; }
+// ------------------------------------------------------- shared tile layouts
+// Where element j of pencil q lies in the tile of C pencils:
+//   Swz<C>     j C + (q ^ ((j ^ (j >> 3)) mod C)), for lanes along either
+//              direction: rows of C elements are 128 bytes, and the column-wise
+//              accesses of the x passes (lanes over j, strides 1, R and the
+//              grouped p-strides) stay within 1.04 x the ideal wavefront count
+//              for every radix plan (simulated per quarter / half warp for 16- /
+//              8-byte elements)
+//   Row<C>     j C + q, for the y / z passes: their lanes run over q, and a row
+//              of C elements is 128 bytes, so every access is conflict free
+//              as it is, and a thread's accesses are constant offsets from one
+//              address (the swizzle costs about 4 integer instructions each)
+//   Pad<C, G>  pencil after pencil with one element of padding every 8, for
+//              lanes along j: strides of 1, 4 and 8 fall into distinct banks, and
+//              offsets are constant wherever a stage's strides are multiples
+//              of 8.  G elements make 128 bytes; the pitch sets the pencils that
+//              share a 128-byte access side by side (NT lanes each).
+// additive<D, B>: an offset D r from a base that is a multiple of B can be
+// added as step(D r).
+template <int C_>
+struct Swz {
+    static constexpr int C = C_;
+    template <int N, int NT>
+    static constexpr int elems() { return N * C; }
+    template <int N, int NT>
+    static __device__ __forceinline__ int at(int j, int q) {
+        static_assert(C == 8 || C == 16, "tile width");
+        return j * C + (q ^ ((j ^ (j >> 3)) & (C - 1)));
+    }
+    template <int D, int B>
+    static constexpr bool additive() { return false; }
+    static constexpr int step(int d) { return d * C; }
+};
+template <int C_>
+struct Row {
+    static constexpr int C = C_;
+    template <int N, int NT>
+    static constexpr int elems() { return N * C; }
+    template <int N, int NT>
+    static __device__ __forceinline__ int at(int j, int q) { return j * C + q; }
+    template <int D, int B>
+    static constexpr bool additive() { return true; }
+    static constexpr int step(int d) { return d * C; }
+};
+template <int C_, int G>
+struct Pad {
+    static constexpr int C = C_;
+    template <int N, int NT>
+    static constexpr int pitch() {
+        const int rem = NT < G ? (G == 16 ? NT & ~1 : NT) : 4;  // wanted pitch mod G (even for 8-byte elements)
+        int p = N + N / 8;
+        while (p % G != rem) ++p;
+        return p;
+    }
+    template <int N, int NT>
+    static constexpr int elems() { return C * pitch<N, NT>(); }
+    template <int N, int NT>
+    static __device__ __forceinline__ int at(int j, int q) { return q * pitch<N, NT>() + j + (j >> 3); }
+    template <int D, int B>
+    static constexpr bool additive() { return D % 8 == 0 || B % 8 == 0; }
+    static constexpr int step(int d) { return d + (d >> 3); }
+};
 
 // --------------------------------------------------------------- radix DFTs
 template <int S, class T>
@@ -186,6 +222,17 @@ __device__ __forceinline__ void dft16(T* x) {
         }
 }
 
+// A stage's radix as it appears in a plan: a plain radix, or the composite
+// pair(R1, R2) -- a radix-R1 stage followed by a radix-R2 stage whose
+// R1 R2 points stay in one thread's registers.  Stockham's index maps close
+// over such a group: stage (P, R1) followed by stage (P R1, R2) reads and
+// writes exactly the points of one stage (P, R1 R2), so gather and scatter take
+// the product as radix, and only the butterflies know the two steps.  The
+// arithmetic is that of the two stages, bit for bit; what goes is the
+// exchange through shared memory between them.
+constexpr int pair(int r1, int r2) { return 100 * r1 + r2; }
+constexpr int radix(int code) { return code < 100 ? code : (code / 100) * (code % 100); }
+
 template <int R, int S, class T>
 __device__ __forceinline__ void dft(T* x) {
     if constexpr (R == 2) dft2<S>(x[0], x[1]);
@@ -199,17 +246,18 @@ __device__ __forceinline__ void dft(T* x) {
 }
 
 // ------------------------------------------------------------ stage pieces
-template <int N, int NT, int R>
+template <int N, int NT, int RC>
 struct Stage {
+    static constexpr int R = radix(RC);
     static constexpr int NB = N / R;
     static constexpr int NBT = (NB + NT - 1) / NT;
     static constexpr int E = NBT * R;
 };
 
 // x[b*R + r] := input r of butterfly i = t + b*NT, read through src(j)
-template <int N, int NT, int R, class T, class Src>
+template <int N, int NT, int RC, class T, class Src>
 __device__ __forceinline__ void gather(T* x, int t, const Src& src) {
-    constexpr int NB = Stage<N, NT, R>::NB, NBT = Stage<N, NT, R>::NBT;
+    constexpr int R = radix(RC), NB = Stage<N, NT, RC>::NB, NBT = Stage<N, NT, RC>::NBT;
 #pragma unroll
     for (int b = 0; b < NBT; ++b) {
         const int i = t + b * NT;
@@ -220,33 +268,66 @@ __device__ __forceinline__ void gather(T* x, int t, const Src& src) {
     }
 }
 
-template <int N, int NT, int R, int P, int S, class T>
-__device__ __forceinline__ void butterflies(T* x, int t, const float2* __restrict__ tw) {
-    constexpr int NB = Stage<N, NT, R>::NB, NBT = Stage<N, NT, R>::NBT;
+// x[r STRIDE] *= w^(r k), w = exp(S 2 pi i / (P R)), then the radix-R DFT of
+// x[0], x[STRIDE], ...
+template <int N, int R, int P, int S, int STRIDE, class T>
+__device__ __forceinline__ void butterfly(T* x, int k, const float2* __restrict__ tw) {
     static_assert(N % (P * R) == 0, "bad radix plan");
     constexpr int TS = N / (P * R);  // twiddle table stride
+    if constexpr (P > 1) {
+#pragma unroll
+        for (int r = 1; r < R; ++r) {
+            float2 w = __ldg(&tw[r * k * TS]);  // r*k*TS < N
+            if (S > 0) w.y = -w.y;
+            x[r * STRIDE] = cmul(x[r * STRIDE], w);
+        }
+    }
+    if constexpr (STRIDE == 1) {
+        dft<R, S>(x);
+    } else {
+        T y[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) y[r] = x[r * STRIDE];
+        dft<R, S>(y);
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[r * STRIDE] = y[r];
+    }
+}
+
+template <int N, int NT, int RC, int P, int S, class T>
+__device__ __forceinline__ void butterflies(T* x, int t, const float2* __restrict__ tw) {
+    constexpr int R = radix(RC), NB = Stage<N, NT, RC>::NB, NBT = Stage<N, NT, RC>::NBT;
 #pragma unroll
     for (int b = 0; b < NBT; ++b) {
         const int i = t + b * NT;
         if (NB % NT == 0 || i < NB) {
-            if constexpr (P > 1) {
-                const int k = i % P;
+            const int k = i % P;
+            if constexpr (RC < 100) {
+                butterfly<N, R, P, S, 1>(x + b * R, k, tw);
+            } else {
+                // point s = r2 + R2 r1 of the group: radix R1 over r1 for every
+                // r2, then radix R2 over r2 for every r1; output r1 + R1 r2
+                constexpr int R1 = RC / 100, R2 = RC % 100;
 #pragma unroll
-                for (int r = 1; r < R; ++r) {
-                    float2 w = __ldg(&tw[r * k * TS]);  // r*k*TS < N
-                    if (S > 0) w.y = -w.y;
-                    x[b * R + r] = cmul(x[b * R + r], w);
-                }
+                for (int r2 = 0; r2 < R2; ++r2) butterfly<N, R1, P, S, R2>(x + b * R + r2, k, tw);
+#pragma unroll
+                for (int r1 = 0; r1 < R1; ++r1) butterfly<N, R2, P * R1, S, 1>(x + b * R + R2 * r1, r1 * P + k, tw);
+                T y[R];
+#pragma unroll
+                for (int r1 = 0; r1 < R1; ++r1)
+#pragma unroll
+                    for (int r2 = 0; r2 < R2; ++r2) y[r1 + R1 * r2] = x[b * R + R2 * r1 + r2];
+#pragma unroll
+                for (int r = 0; r < R; ++r) x[b * R + r] = y[r];
             }
-            dft<R, S>(x + b * R);
         }
     }
 }
 
 // dst(j, v) for every output j = (i - k) R + k + r P of this thread's butterflies
-template <int N, int NT, int R, int P, class T, class Dst>
+template <int N, int NT, int RC, int P, class T, class Dst>
 __device__ __forceinline__ void scatter(const T* x, int t, const Dst& dst) {
-    constexpr int NB = Stage<N, NT, R>::NB, NBT = Stage<N, NT, R>::NBT;
+    constexpr int R = radix(RC), NB = Stage<N, NT, RC>::NB, NBT = Stage<N, NT, RC>::NBT;
 #pragma unroll
     for (int b = 0; b < NBT; ++b) {
         const int i = t + b * NT;
@@ -264,22 +345,60 @@ struct First {
     static constexpr int value = A;
 };
 
+// one stage's outputs into the shared tile, and the next stage's inputs from it
+template <class L, int N, int NT, int RC, int P, class T>
+__device__ __forceinline__ void scatter_tile(const T* x, int t, int q, T* sm) {
+    constexpr int R = radix(RC);
+    constexpr bool kAdd = L::template additive<P, P == 1 ? R : 1>();
+    if constexpr (kAdd) {
+        constexpr int NB = Stage<N, NT, RC>::NB, NBT = Stage<N, NT, RC>::NBT;
+#pragma unroll
+        for (int b = 0; b < NBT; ++b) {
+            const int i = t + b * NT;
+            if (NB % NT == 0 || i < NB) {
+                const int k = i % P;
+                T* o = sm + L::template at<N, NT>((i - k) * R + k, q);
+#pragma unroll
+                for (int r = 0; r < R; ++r) o[L::step(r * P)] = x[b * R + r];
+            }
+        }
+    } else {
+        scatter<N, NT, RC, P>(x, t, [&](int j, const T& v) { sm[L::template at<N, NT>(j, q)] = v; });
+    }
+}
+template <class L, int N, int NT, int RC, class T>
+__device__ __forceinline__ void gather_tile(T* x, int t, int q, const T* sm) {
+    constexpr int R = radix(RC), NB = Stage<N, NT, RC>::NB, NBT = Stage<N, NT, RC>::NBT;
+    if constexpr (L::template additive<NB, 1>()) {
+#pragma unroll
+        for (int b = 0; b < NBT; ++b) {
+            const int i = t + b * NT;
+            if (NB % NT == 0 || i < NB) {
+                const T* o = sm + L::template at<N, NT>(i, q);
+#pragma unroll
+                for (int r = 0; r < R; ++r) x[b * R + r] = o[L::step(r * NB)];
+            }
+        }
+    } else {
+        gather<N, NT, RC>(x, t, [&](int j) { return sm[L::template at<N, NT>(j, q)]; });
+    }
+}
+
 // Runs stages (P, R), Rest... on x, which holds the inputs of stage (P, R);
-// intermediate results go through the shared tile sm (pencil q), the final
-// outputs to dst.  Ends without a barrier after the final scatter.
-template <int N, int NT, int C, int S, class T, class Dst, class B, int P, int R, int... Rest>
+// intermediate results go through the shared tile sm (pencil q, layout L),
+// the final outputs to dst.  Ends without a barrier after the final scatter.
+template <int N, int NT, class L, int S, class T, class Dst, class B, int P, int R, int... Rest>
 __device__ __forceinline__ void pipeline(T* x, int t, int q, T* sm, const float2* __restrict__ tw, const Dst& dst,
                                          const B& bar) {
     butterflies<N, NT, R, P, S>(x, t, tw);
     if constexpr (sizeof...(Rest) == 0) {
         scatter<N, NT, R, P>(x, t, dst);
     } else {
-        scatter<N, NT, R, P>(x, t, [&](int j, const T& v) { sm[sidx<C, N, NT>(j, q)] = v; });
+        scatter_tile<L, N, NT, R, P>(x, t, q, sm);
         bar.xsync();
-        constexpr int R2 = First<Rest...>::value;
-        gather<N, NT, R2>(x, t, [&](int j) { return sm[sidx<C, N, NT>(j, q)]; });
+        gather_tile<L, N, NT, First<Rest...>::value>(x, t, q, sm);
         bar.xsync();
-        pipeline<N, NT, C, S, T, Dst, B, P * R, Rest...>(x, t, q, sm, tw, dst, bar);
+        pipeline<N, NT, L, S, T, Dst, B, P * radix(R), Rest...>(x, t, q, sm, tw, dst, bar);
     }
 }
 
@@ -288,24 +407,23 @@ __device__ __forceinline__ void pipeline(T* x, int t, int q, T* sm, const float2
 // exactly the input layout of a first stage of radix R with N / R
 // butterflies, so an inverse transform whose radices run in the reverse
 // order can start from these registers without a pass through shared memory.
-template <int N, int NT, int C, int S, class T, class B, int P, int R, int... Rest>
+template <int N, int NT, class L, int S, class T, class B, int P, int R, int... Rest>
 __device__ __forceinline__ void pipeline_keep(T* x, int t, int q, T* sm, const float2* __restrict__ tw, const B& bar) {
     butterflies<N, NT, R, P, S>(x, t, tw);
     if constexpr (sizeof...(Rest) > 0) {
-        scatter<N, NT, R, P>(x, t, [&](int j, const T& v) { sm[sidx<C, N, NT>(j, q)] = v; });
+        scatter_tile<L, N, NT, R, P>(x, t, q, sm);
         bar.xsync();
-        constexpr int R2 = First<Rest...>::value;
-        gather<N, NT, R2>(x, t, [&](int j) { return sm[sidx<C, N, NT>(j, q)]; });
+        gather_tile<L, N, NT, First<Rest...>::value>(x, t, q, sm);
         bar.xsync();
-        pipeline_keep<N, NT, C, S, T, B, P * R, Rest...>(x, t, q, sm, tw, bar);
+        pipeline_keep<N, NT, L, S, T, B, P * radix(R), Rest...>(x, t, q, sm, tw, bar);
     }
 }
 
 // --------------------------------------------------------------- radix plans
 constexpr int isf_emax(int N, int NT, std::initializer_list<int> rs) {
     int m = 0;
-    for (int r : rs) {
-        const int nb = N / r;
+    for (int code : rs) {
+        const int r = radix(code), nb = N / r;
         const int e = ((nb + NT - 1) / NT) * r;
         m = e > m ? e : m;
     }
@@ -320,41 +438,41 @@ constexpr int isf_emax(int N, int NT, std::initializer_list<int> rs) {
 // inverse of run_spectral).
 template <int N>
 struct Plan;
-#define ISF_PLAN(NN, R0, FWD, REV) ISF_PLAN_NAMED(Plan, NN, R0, FWD, REV)
-#define ISF_PLAN_NAMED(NAME, NN, R0, FWD, REV)                                                              \
+#define ISF_PLAN(NN, R0, FWD, REV) ISF_PLAN_NAMED(Plan, NN, NN / R0, R0, FWD, REV)
+#define ISF_PLAN_NAMED(NAME, NN, LANES, R0, FWD, REV)                                                       \
     template <>                                                                                             \
     struct NAME<NN> {                                                                                       \
         static constexpr int first = R0;                                                                    \
-        static constexpr int NT = NN / R0;                                                                  \
-        static constexpr int EMAX = isf_emax(NN, NN / R0, {ISF_UNPAREN FWD});                              \
+        static constexpr int NT = LANES;                                                                    \
+        static constexpr int EMAX = isf_emax(NN, LANES, {ISF_UNPAREN FWD});                                \
         /* SYNC: barrier after the first gather (needed when src reads the tile) */                       \
-        template <int C, int S, bool SYNC, class T, class Src, class Dst, class B = CtaBar>                 \
+        template <class L, int S, bool SYNC, class T, class Src, class Dst, class B = CtaBar>               \
         static __device__ __forceinline__ void run(T* x, int t, int q, T* sm, const float2* __restrict__ tw, \
                                                    const Src& src, const Dst& dst, const B& bar = B()) {    \
-            gather<NN, NN / R0, R0>(x, t, src);                                                             \
+            gather<NN, NT, R0>(x, t, src);                                                                  \
             if constexpr (SYNC) bar.sync();                                                                 \
-            pipeline<NN, NN / R0, C, S, T, Dst, B, 1, ISF_UNPAREN FWD>(x, t, q, sm, tw, dst, bar);          \
+            pipeline<NN, NT, L, S, T, Dst, B, 1, ISF_UNPAREN FWD>(x, t, q, sm, tw, dst, bar);               \
         }                                                                                                   \
         /* forward transform, mul(j, v) on every output j in registers, inverse transform */               \
         /* (SYNC: barrier after the first gather, when src reads the tile)  */                             \
-        template <int C, bool SYNC = false, class T, class Src, class Mul, class Dst, class B = CtaBar>     \
+        template <class L, bool SYNC = false, class T, class Src, class Mul, class Dst, class B = CtaBar>   \
         static __device__ __forceinline__ void run_spectral(T* x, int t, int q, T* sm,                      \
                                                             const float2* __restrict__ tw, const Src& src,  \
                                                             const Mul& mul, const Dst& dst,                 \
                                                             const B& bar = B()) {                           \
-            constexpr int NTh = NN / R0;                                                                    \
+            constexpr int NTh = NT;                                                                         \
             gather<NN, NTh, R0>(x, t, src);                                                                 \
             if constexpr (SYNC) bar.sync();                                                                 \
-            pipeline_keep<NN, NTh, C, -1, T, B, 1, ISF_UNPAREN FWD>(x, t, q, sm, tw, bar);                  \
-            constexpr int RL = First<ISF_UNPAREN REV>::value, PL = NN / RL;                                 \
-            constexpr int NBT = Stage<NN, NTh, RL>::NBT;                                                    \
+            pipeline_keep<NN, NTh, L, -1, T, B, 1, ISF_UNPAREN FWD>(x, t, q, sm, tw, bar);                  \
+            constexpr int RC = First<ISF_UNPAREN REV>::value, RL = radix(RC), PL = NN / RL;                 \
+            constexpr int NBT = Stage<NN, NTh, RC>::NBT;                                                    \
             _Pragma("unroll") for (int b = 0; b < NBT; ++b) {                                               \
                 const int i = t + b * NTh;                                                                  \
                 if (PL % NTh == 0 || i < PL) {                                                              \
                     _Pragma("unroll") for (int r = 0; r < RL; ++r) x[b * RL + r] = mul(i + r * PL, x[b * RL + r]); \
                 }                                                                                           \
             }                                                                                               \
-            pipeline<NN, NTh, C, +1, T, Dst, B, 1, ISF_UNPAREN REV>(x, t, q, sm, tw, dst, bar);             \
+            pipeline<NN, NTh, L, +1, T, Dst, B, 1, ISF_UNPAREN REV>(x, t, q, sm, tw, dst, bar);             \
         }                                                                                                   \
     };
 
@@ -394,8 +512,36 @@ ISF_PLAN(200, 8, (8, 5, 5), (5, 5, 8))
 template <int N>
 struct PlanPlane : Plan<N> {};
 #if ISF_PLANE128_RADIX16
-ISF_PLAN_NAMED(PlanPlane, 128, 16, (16, 8), (8, 16))
+ISF_PLAN_NAMED(PlanPlane, 128, 8, 16, (16, 8), (8, 16))
 #endif
+
+// Plan<N>'s stages with two of three joined in registers (pair): a pencil
+// crosses shared memory once instead of twice, the spectral pass twice instead
+// of four times.  A thread then holds 12 to 20 float4 values, so fewer threads
+// are resident; where that costs more than the exchanges, the plan stays out.
+template <int N>
+struct PlanJoined : Plan<N> {};
+ISF_PLAN_NAMED(PlanJoined, 96, 12, 8, (8, pair(4, 3)), (pair(3, 4), 8))
+ISF_PLAN_NAMED(PlanJoined, 100, 5, pair(4, 5), (pair(4, 5), 5), (5, pair(5, 4)))
+ISF_PLAN_NAMED(PlanJoined, 112, 8, pair(4, 4), (pair(4, 4), 7), (7, pair(4, 4)))
+ISF_PLAN_NAMED(PlanJoined, 128, 8, 8, (8, pair(4, 4)), (pair(4, 4), 8))
+ISF_PLAN_NAMED(PlanJoined, 384, 24, 8, (8, pair(4, 4), 3), (3, pair(4, 4), 8))
+
+// Which launched psi passes take PlanJoined<N>, by what they measured on
+// cubes and slabs of the length (us before -> joined):
+//   x passes         112: 13.0 -> 11.2; 96 and 128 equal, 100 equal, 160 slower
+//   y / z transforms 112: 13.4 -> 12.8, 128: 23.1 -> 20.9, 384: 25.0 -> 23.0; 96
+//                    equal, 100 slower (15.1 -> 16.2)
+//   z with the mask  96: 14.8 -> 12.7, 100: 36.1 -> 29.1, 112: 25.2 -> 19.4; 128
+//                    slower (36.1 -> 39.3), as were 48, 80 and 160
+// The lengths of two stages have nothing to join, and 192, 200, 256 and 512 no
+// pair that leaves registers for the butterflies.
+enum PassRole { ROLE_X, ROLE_YZ, ROLE_SPECTRAL };
+constexpr bool joined(int n, int role) {
+    if (n == 112) return true;
+    if (n == 128 || n == 384) return role == ROLE_YZ;
+    return (n == 96 || n == 100) && role == ROLE_SPECTRAL;
+}
 #undef ISF_PLAN_NAMED
 
 }  // namespace isf

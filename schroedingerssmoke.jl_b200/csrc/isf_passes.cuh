@@ -61,10 +61,16 @@ struct XTraits {
     static constexpr int S = (OP == X_PSI_FWD || OP == X_C_FWD) ? -1 : +1;
 };
 
-template <int N, int OP, int G = 1>
+// the plan of an x or y / z pass: the psi passes of a kernel launched on its own
+// may join stages in registers; the persistent batch kernel, whose registers
+// are shared by every pass, keeps Plan<N>
+template <int N, class T, int ROLE, bool LAUNCH>
+using PlanOf = typename std::conditional<LAUNCH && sizeof(T) == 16 && joined(N, ROLE), PlanJoined<N>, Plan<N>>::type;
+
+template <int N, int OP, int G = 1, bool LAUNCH = true>
 struct XShape {
     static constexpr int C = XTraits<OP>::C;
-    static constexpr int NT = Plan<N>::NT;
+    static constexpr int NT = PlanOf<N, typename XTraits<OP>::T, ROLE_X, LAUNCH>::NT;
     static constexpr int BLK = G * C * NT;
     static constexpr size_t SMEM = (size_t)G * N * C * sizeof(typename XTraits<OP>::T);
 };
@@ -76,8 +82,9 @@ __device__ __forceinline__ void xpass_body(const XArgs a, const Blk bk, unsigned
                                            const BarT& bar = BarT()) {
     using Tr = XTraits<OP>;
     using T = typename Tr::T;
+    using Pl = PlanOf<N, T, ROLE_X, BarT::kLaunch>;
     constexpr int C = Tr::C;
-    constexpr int NT = Plan<N>::NT;
+    constexpr int NT = Pl::NT;
     const int grp = bk.tid / (C * NT), lt = bk.tid % (C * NT);
     T* sm = reinterpret_cast<T*>(smraw) + grp * (N * C);
     const int t = lt % NT, q = lt / NT;
@@ -88,7 +95,7 @@ __device__ __forceinline__ void xpass_body(const XArgs a, const Blk bk, unsigned
     const bool valid = FULL || row < (long long)a.g.n[1] * a.g.n[2];
     float4* __restrict__ psi = a.psi + bk.y * a.bs_psi;
     float2* __restrict__ F = a.F + bk.y * a.bs_F;
-    T x[Plan<N>::EMAX];
+    T x[Pl::EMAX];
 
     auto src = [&](int j) -> T {
         if (!valid) return T{};
@@ -109,7 +116,7 @@ __device__ __forceinline__ void xpass_body(const XArgs a, const Blk bk, unsigned
             F[rb + j] = v;
         }
     };
-    Plan<N>::template run<C, Tr::S, false>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
+    Pl::template run<Swz<C>, Tr::S, false>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
 }
 
 template <int N, int OP, int G, bool FULL = false>
@@ -150,7 +157,8 @@ struct XRShape {
     static constexpr int NT = Plan<N>::NT;
     static constexpr int BLK = G * C * NT;
     // the k-major inverse stages (A, B) of N/2 + 1 k per row pair in the tile
-    static constexpr size_t TILE = (size_t)tile_elems<C, N, NT>() * sizeof(float2);
+    using L = typename std::conditional<C == 4, Pad<4, 16>, Swz<16>>::type;
+    static constexpr size_t TILE = (size_t)L::template elems<N, NT>() * sizeof(float2);
     static constexpr size_t STAGE = (size_t)(N / 2 + 1) * C * sizeof(float4);
     static constexpr size_t GROUP = (KM && STAGE > TILE ? STAGE : TILE);  // bytes of one group (a multiple of 16)
     static constexpr size_t PSI = (C == 4 && GAUGE) ? (size_t)2 * C * N * sizeof(float4) : 0;
@@ -172,6 +180,7 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
                                            const BarT& bar = BarT()) {
     using T = float2;
     using Sh = XRShape<N, G, KM, C, xr_gauge(OP)>;
+    using L = typename Sh::L;
     constexpr int NT = Plan<N>::NT;
     const int grp = bk.tid / (C * NT), lt = bk.tid % (C * NT);
     T* sm = reinterpret_cast<T*>(smraw + grp * Sh::GROUP);
@@ -193,16 +202,16 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
         auto src = [&](int j) -> T {
             return make_float2(v0 ? ldm<BarT>(&f0[j]) : 0.f, v1 ? ldm<BarT>(&f1[j]) : 0.f);
         };
-        auto sdst = [&](int j, const T& v) { sm[sidx<C, N, NT>(j, q)] = v; };
-        Plan<N>::template run<C, -1, false>(x, t, q, sm, a.g.tw[0], src, sdst, pencil_bar<NT, C>(bar));
+        auto sdst = [&](int j, const T& v) { sm[L::template at<N, NT>(j, q)] = v; };
+        Plan<N>::template run<L, -1, false>(x, t, q, sm, a.g.tw[0], src, sdst, pencil_bar<NT, C>(bar));
         bar.sync();
         if constexpr (KM) {
             // lanes over the row pairs of the group: C x 16 B per k
             float4* __restrict__ F4 = reinterpret_cast<float4*>(Fs);
             for (int idx = lt; idx < (N / 2 + 1) * C; idx += C * NT) {
                 const int qq = idx % C, k = idx / C;
-                const float2 zk = sm[sidx<C, N, NT>(k, qq)];
-                const float2 zn = sm[sidx<C, N, NT>(k == 0 ? 0 : N - k, qq)];
+                const float2 zk = sm[L::template at<N, NT>(k, qq)];
+                const float2 zn = sm[L::template at<N, NT>(k == 0 ? 0 : N - k, qq)];
                 const long long r = rbase + 2 * qq;
                 const int y = (int)(r % ny), z = (int)(r / ny);
                 F4[(((long long)k * nz + z) * ny + y) >> 1] =
@@ -213,8 +222,8 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
             float2* __restrict__ B = A + wp;
 #pragma unroll 1
             for (int k = t; k <= N / 2; k += NT) {
-                const float2 zk = sm[sidx<C, N, NT>(k, q)];
-                const float2 zn = sm[sidx<C, N, NT>(k == 0 ? 0 : N - k, q)];
+                const float2 zk = sm[L::template at<N, NT>(k, q)];
+                const float2 zn = sm[L::template at<N, NT>(k == 0 ? 0 : N - k, q)];
                 if (v0) A[k] = make_float2(0.5f * (zk.x + zn.x), 0.5f * (zk.y - zn.y));
                 if (v1) B[k] = make_float2(0.5f * (zk.y + zn.y), -0.5f * (zk.x - zn.x));
             }
@@ -293,7 +302,7 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
         };
         // k-major: the staging aliases the tile, so the first gather must
         // complete before the first stage writes the tile
-        Plan<N>::template run<C, +1, KM>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
+        Plan<N>::template run<L, +1, KM>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
     }
 }
 
@@ -392,7 +401,7 @@ __device__ __forceinline__ void plane_body(const PlaneArgs a, const Blk bk, unsi
                 else
                     Fp[z * N + j] = v;
             };
-            PlanPlane<N>::template run<C, S, false>(x, t, q, tile, a.g.tw[1], src, dst, pencil_bar<NT, C>(bar));
+            PlanPlane<N>::template run<Swz<C>, S, false>(x, t, q, tile, a.g.tw[1], src, dst, pencil_bar<NT, C>(bar));
             bar.sync();
         }
     };
@@ -420,7 +429,7 @@ __device__ __forceinline__ void plane_body(const PlaneArgs a, const Blk bk, unsi
                 const float f = (zero_line && j == 0) ? 0.f : (float)(sc * __drcp_rn(dxo + __ldg(&s2z[j])));
                 return cscale(v, f);
             };
-            PlanPlane<N>::template run_spectral<C>(x, t, q, tile, a.g.tw[2], src, fmul, dst, bar);
+            PlanPlane<N>::template run_spectral<Row<C>>(x, t, q, tile, a.g.tw[2], src, fmul, dst, bar);
             bar.sync();
         }
     }
@@ -468,17 +477,27 @@ struct YZArgs {
 #define ISF_YZ_PSI_SPECTRAL_MIN_THREADS 512
 #endif
 
-template <int N, class T, int OP = 0, int G = 1>
+template <int N, class T, int OP, bool LAUNCH>
+using PlanYZ = PlanOf<N, T, (OP < YZ_MASK ? ROLE_YZ : ROLE_SPECTRAL), LAUNCH>;
+
+template <int N, class T, int OP = 0, int G = 1, bool LAUNCH = true>
 struct YZShape {
+    using Pl = PlanYZ<N, T, OP, LAUNCH>;
     static constexpr int C = 128 / (int)sizeof(T);
-    static constexpr int NT = Plan<N>::NT;
+    static constexpr int NT = Pl::NT;
     static constexpr int BLK = G * C * NT;
     static constexpr size_t SMEM = (size_t)G * N * C * sizeof(T);
-    static constexpr int MINT = (OP < 2) ? ISF_YZ_MIN_THREADS
+    // resident threads the pass is compiled for: fewer for the psi passes with
+    // 12 and more float4 values per thread (the joined stages)
+    static constexpr int E = sizeof(T) == 16 ? Pl::EMAX : 0;
+    static constexpr int MINT = E > 16 ? 384
+                                : E > 10 ? (OP < 2 ? 512 : 448)
+                                : OP < 2 ? ISF_YZ_MIN_THREADS
                                 : (sizeof(T) == 16 ? ISF_YZ_PSI_SPECTRAL_MIN_THREADS : ISF_YZ_SPECTRAL_MIN_THREADS);
     // at least 1, at most the 32 resident CTAs an SM takes (short pencils
-    // make small CTAs)
-    static constexpr int MINB = (MINT / BLK) > 32 ? 32 : ((MINT / BLK) > 1 ? (MINT / BLK) : 1);
+    // make small CTAs), counted in whole warps
+    static constexpr int WARPS = (BLK + 31) / 32 * 32;
+    static constexpr int MINB = (MINT / WARPS) > 32 ? 32 : ((MINT / WARPS) > 1 ? (MINT / WARPS) : 1);
 };
 
 __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
@@ -489,8 +508,9 @@ __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
 template <int N, class T, int OP, int G, bool FULL = false, class BarT = CtaBar>
 __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsigned char* smraw,
                                             const BarT& bar = BarT()) {
+    using Pl = PlanYZ<N, T, OP, BarT::kLaunch>;
     constexpr int C = YZShape<N, T>::C;
-    constexpr int NT = Plan<N>::NT;
+    constexpr int NT = Pl::NT;
     const int grp = bk.tid / (C * NT), lt = bk.tid % (C * NT);
     T* sm = reinterpret_cast<T*>(smraw) + grp * (N * C);
     const int q = lt % C, t = lt / C;
@@ -507,7 +527,7 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
     }
     T* __restrict__ data = reinterpret_cast<T*>(a.data) + bk.z * a.bstride;
     const float2* tw = a.g.tw[a.axis];
-    T x[Plan<N>::EMAX];
+    T x[Pl::EMAX];
 
     // columns past the row's end (a row length that is not a multiple of
     // C) read zeros and store nothing
@@ -518,9 +538,9 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
     };
 
     if constexpr (OP == YZ_FWD) {
-        Plan<N>::template run<C, -1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
+        Pl::template run<Row<C>, -1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
     } else if constexpr (OP == YZ_INV) {
-        Plan<N>::template run<C, +1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
+        Pl::template run<Row<C>, +1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
     } else {
         // spectral multiply between the forward and the inverse transform of
         // this pencil; k along the pass axis is the pencil position j
@@ -534,13 +554,12 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
             cxo.x *= a.g.invN;
             cxo.y *= a.g.invN;
             const double2* __restrict__ mt = a.g.mtab[a.axis];
-            const double msign = a.conj_mask ? -1.0 : 1.0;
+            const float msign = a.conj_mask ? -1.f : 1.f;
             auto mmul = [&](int j, const T& v) -> T {
-                double2 m = zmul(cxo, __ldg(&mt[j]));
-                m.y *= msign;
-                return cmul(v, make_float2((float)m.x, (float)m.y));
+                const double2 m = zmul(cxo, __ldg(&mt[j]));
+                return cmul(v, make_float2((float)m.x, msign * (float)m.y));
             };
-            Plan<N>::template run_spectral<C>(x, t, q, sm, tw, gsrc, mmul, gdst, bar);
+            Pl::template run_spectral<Row<C>>(x, t, q, sm, tw, gsrc, mmul, gdst, bar);
         } else {
             static_assert(OP == YZ_FAC, "unhandled y/z op");
             // fac(k)/N, fac = -0.25 / sum_a (sin(pi k_a / n_a) / d_a)^2, fac(0) = 0
@@ -554,7 +573,7 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
                 const float f = (pad || (zero_line && j == 0)) ? 0.f : (float)(sc * __drcp_rn(dxo + __ldg(&s2[j])));
                 return cscale(v, f);
             };
-            Plan<N>::template run_spectral<C>(x, t, q, sm, tw, gsrc, fmul, gdst, bar);
+            Pl::template run_spectral<Row<C>>(x, t, q, sm, tw, gsrc, fmul, gdst, bar);
         }
     }
 }

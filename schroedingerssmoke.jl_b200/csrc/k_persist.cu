@@ -322,9 +322,9 @@ int host_plane(int n, const F& f) {
 int persist_vblk(int kind, int len) {
     switch (kind) {
         case PK_X_FWD: case PK_X_INV_NORM:
-            return host_xlen(len, [](auto n) { return XShape<decltype(n)::value, X_PSI_FWD, 1>::BLK; });
+            return host_xlen(len, [](auto n) { return XShape<decltype(n)::value, X_PSI_FWD, 1, false>::BLK; });
         case PK_Y_FWD: case PK_Z_MASK: case PK_Y_INV:
-            return host_plane(len, [](auto n) { return YZShape<decltype(n)::value, float4, YZ_FWD, 1>::BLK; });
+            return host_plane(len, [](auto n) { return YZShape<decltype(n)::value, float4, YZ_FWD, 1, false>::BLK; });
         case PK_XR_FWD: case PK_XR_INV_GAUGE:
             return host_xlen(len, [](auto n) { return XRShape<decltype(n)::value, 1, true>::BLK; });
         case PK_PLANE:
@@ -337,9 +337,9 @@ int persist_vblk(int kind, int len) {
 int persist_smem(int kind, int len) {
     switch (kind) {
         case PK_X_FWD: case PK_X_INV_NORM:
-            return host_xlen(len, [](auto n) { return (int)XShape<decltype(n)::value, X_PSI_FWD, 1>::SMEM; });
+            return host_xlen(len, [](auto n) { return (int)XShape<decltype(n)::value, X_PSI_FWD, 1, false>::SMEM; });
         case PK_Y_FWD: case PK_Z_MASK: case PK_Y_INV:
-            return host_plane(len, [](auto n) { return (int)YZShape<decltype(n)::value, float4, YZ_FWD, 1>::SMEM; });
+            return host_plane(len, [](auto n) { return (int)YZShape<decltype(n)::value, float4, YZ_FWD, 1, false>::SMEM; });
         case PK_XR_FWD: case PK_XR_INV_GAUGE:
             return host_xlen(len, [](auto n) { return (int)XRShape<decltype(n)::value, 1, true>::SMEM; });
         case PK_PLANE:

@@ -158,7 +158,7 @@ __global__ void __launch_bounds__(ZT<N>::BLK, ZT<N>::MINB)
         };
         auto dst = [&](int j, const float4& v) { data[base + j * stride + q] = v; };
         // the buffer is the stage-exchange tile too: a barrier after the first gather
-        Plan<N>::template run_spectral<C, true>(x, t, q, sm, tw, src, mmul, dst);
+        Plan<N>::template run_spectral<Row<C>, true>(x, t, q, sm, tw, src, mmul, dst);
         // the buffer's generic accesses are done before the copy engine refills it
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         __syncthreads();

@@ -132,3 +132,19 @@ def test_adj_project_and_one_form_on_partial_tiles(isfpkg, oracle_mod, L, dims):
     isfpkg.adj_velocity_one_form(isf, cuda(x), t, HBAR)
     g = (wv * (orc.velocity_one_form(x + h * u, HBAR) - orc.velocity_one_form(x - h * u, HBAR))).sum() / (2 * h)
     assert abs((host(t) * u).sum() - g) <= 1e-3 * abs(g) + 1e-6 * np.linalg.norm(wv) * np.linalg.norm(u)
+
+
+# every pencil length whose psi passes join two stages in registers, in each
+# direction, on whole and partial tiles
+@pytest.mark.parametrize("dims", [(112, 8, 8), (100, 8, 112), (50, 112, 8), (8, 128, 100), (20, 384, 96), (12, 20, 384),
+                                  (16, 96, 128)])
+def test_schroedinger_flow_lengths(isfpkg, oracle_mod, dims):
+    L = (1, 1, 1)
+    isf = isfpkg.ISF(L, dims, HBAR, DT)
+    orc = oracle_mod.Oracle(L, dims, HBAR, DT)
+    psi64 = np.random.default_rng(61).normal(size=dims[::-1] + (4,)).astype(np.float32).astype(np.float64)
+    psi = cuda(psi64)
+    isfpkg.schroedinger_flow(isf, psi)
+    isf.sync()
+    orc.schroedinger_flow(psi64)
+    assert rel(host(psi), psi64) < 1e-5
