@@ -24,16 +24,17 @@ __global__ void __launch_bounds__(st::BX* st::TY, 4) k_stencil_div(StencilArgs a
     stencil_body<ST_DIV, JET>(a, launch_blk(), sm);
 }
 
-// z planes per CTA: as many as leave about 1024 CTAs (of 592 resident ones),
+// z planes per CTA: as many as leave about one wave of the 592 resident CTAs,
 // 1 to kPlanes.  A CTA walks its planes one after another, so on a small grid
-// the walk is the whole launch: with 8 planes 64x32x32 made 16 CTAs.  Measured
-// (one-form stencil / projection / nozzle projection, us per call, 8 planes
-// -> the rule's): 64x32x32 7.7 / 23.6 / 35.7 -> 6.0 / 15.6 / 24.2 (1 plane),
-// 128x64x64 16.3 / 42.8 / 46.1 -> 6.6 / 25.7 / 34.6 (1), 160x96x80 17.9 / 56.4 /
-// 73.2 -> 11.7 / 48.9 / 64.3 (2), 200x100x112 23.0 / 79.1 / 105.5 -> 20.5 / 75.5 /
-// 103 (5), 256x128x128 unchanged (8; 1 plane there: 44.7 / 114 / 158).
+// the walk is the whole launch (with 8 planes 64x32x32 made 16 CTAs); every
+// CTA also loads a plane more than it writes and evaluates an extra z edge, so
+// fewer planes cost more in all, which shows when other streams keep the GPU
+// busy.  Jet step, us alone / three simulations side by side: 128x64x64 95.6 /
+// 59.5 at 1 plane, 100 / 53.7 at 2 (the rule's), 124 / 62.4 at 8; 96x96x96 171 /
+// 106, 162 / 93 at 3 (the rule's), 191 / 106; 256x128x128 419 / 430 at 1, 347 /
+// 346 at 8 (the rule's).  One-form stencil on 64x32x32 7.7 at 8, 6.0 at 1.
 static int planes_of(const Grid& g, long long columns) {
-    const long long sz = columns * g.n[2] / 1024;
+    const long long sz = (columns * g.n[2] + 296) / 592;
     return (int)(sz < 1 ? 1 : (sz > st::kPlanes ? st::kPlanes : sz));
 }
 

@@ -20,9 +20,10 @@ def host(t):
     return t.detach().double().cpu().numpy()
 
 
-# planes per stencil CTA: 1 (few columns), 3 with a remainder of 2, 4, 5 with a
-# remainder of 2, and 8, on whole and partial tiles
-@pytest.mark.parametrize("L,dims", [((2, 1, 1), (40, 12, 50)), ((8, 1, 1), (512, 64, 50)), ((6, 2, 1), (384, 100, 56)),
+# planes per stencil CTA: 1 (few columns), 3 and 6 with a remainder of 2, 5, and 8, on
+# whole and partial tiles
+@pytest.mark.parametrize("L,dims", [((2, 1, 1), (40, 12, 50)), ((5, 3, 2), (160, 96, 56)), ((8, 1, 1), (512, 64, 56)),
+                                    ((8, 1, 1), (512, 64, 50)), ((6, 2, 1), (384, 100, 56)),
                                     ((6, 3, 3), (200, 100, 112)), ((8, 4, 1), (512, 128, 64))])
 def test_stencil_planes_per_cta(isfpkg, oracle_mod, L, dims):
     isf = isfpkg.ISF(L, dims, HBAR, DT)
