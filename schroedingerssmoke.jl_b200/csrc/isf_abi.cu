@@ -460,6 +460,7 @@ int isf_destroy(isf_handle* h) {
         cudaFree(h->keep_counts);
         free_order(h);
         adj_free(h);
+        seq_free(h);
         destroy_side(h);
         if (h->own_stream) cudaStreamDestroy(h->stream);
         for (cudaEvent_t e : h->ev_pool) cudaEventDestroy(e);
@@ -534,7 +535,9 @@ int isf_schroedinger_flow(isf_handle* h, float* psi) {
     ISF_ENTER(h);
     if (!psi) return fail(h, ISF_ERR_INVALID, "isf_schroedinger_flow: null psi");
     ISF_ALIGNED(h, psi, 16, "psi");
-    return run_schroedinger(h, psi, false);
+    Sequence seq(h);
+    if (int rc = run_schroedinger(h, psi, false)) return rc;
+    return seq.submit(h->stream, "schroedinger_flow");
 }
 
 int isf_normalize_psi(isf_handle* h, float* psi) {
@@ -549,7 +552,9 @@ int isf_pressure_project(isf_handle* h, float* psi) {
     ISF_ENTER(h);
     if (!psi) return fail(h, ISF_ERR_INVALID, "isf_pressure_project: null psi");
     ISF_ALIGNED(h, psi, 16, "psi");
-    return run_projection(h, psi, nullptr);
+    Sequence seq(h);
+    if (int rc = run_projection(h, psi, nullptr)) return rc;
+    return seq.submit(h->stream, "pressure_project");
 }
 
 int isf_velocity_one_form(isf_handle* h, const float* psi, float hbar) {
@@ -610,8 +615,11 @@ int isf_init_jet(isf_handle* h, float* psi, int32_t iters, const float kvec[3], 
     // restrict_velocity!(isf, psi, kvec, isjet, 0) + pressure_project!, the
     // restriction fused into the projection's stencil and gauge pass as in isf_step
     JetArgs j = make_jet(kvec, mask, cen ? cen : zero, len, rad, 0.f, phase_mode);
-    for (int it = 0; it < iters; ++it)
+    for (int it = 0; it < iters; ++it) {
+        Sequence seq(h);
         if (int rc = run_projection(h, psi, &j)) return rc;
+        if (int rc = seq.submit(h->stream, "init_jet")) return rc;
+    }
     return ISF_OK;
 }
 
@@ -688,6 +696,9 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
                         (h->order_n != np || h->order_parts != parts || h->order_age >= h->order_every);
     if (resort)
         if (int rc = ensure_order(h, np)) return rc;
+    // the psi passes and the one-form as one sequence; what the one-form waits
+    // for (the advection two steps back, run_one_form) is waited for before it
+    Sequence fields(h);
     int rc = run_schroedinger(h, psi, true);  // schroedinger_flow! + normalize_psi
     if (rc) return rc;
     rc = run_projection(h, psi, nullptr);     // pressure_project!
@@ -701,6 +712,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
     // velocity_one_form!(isf, psi, isf.hbar) + staggered sharp
     rc = run_one_form(h, psi, h->g.hbar, 1, "step one_form");
     if (rc) return rc;
+    if ((rc = fields.submit(h->stream, "step"))) return rc;
     // add_particles! (before the projections in the reference; the particles
     // are independent of psi) and staggered_advect!.  With a particle stream
     // they run there, after this step's velocity, while the caller queues the
@@ -712,6 +724,9 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
         ISF_CUDA(h, cudaEventRecord(h->ev_vel, h->stream), "step velocity event");
         ISF_CUDA(h, cudaStreamWaitEvent(h->side, h->ev_vel, 0), "step velocity event");
     }
+    // emission and advection as another; a sort between them launches on its own
+    const bool sort_now = h->order_every > 0 && np > 0 && resort;
+    Sequence particles(h);
     if (emit) {
         EmitArgs e;
         for (int k = 0; k < 3; ++k) e.cen[k] = a->nozzle_cen[k];
@@ -724,13 +739,16 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
     }
     const int* order = nullptr;
     if (h->order_every > 0 && np > 0) {
-        if (resort)
+        if (sort_now) {
+            if ((rc = particles.submit(ps, "step"))) return rc;
             if (int rc_o = run_order(h, parts, np, ps, "step")) return rc_o;
+        }
         ++h->order_age;
         order = h->ord.order;
     }
     if (np > 0)
         ISF_LAUNCH_ON(h, ps, launch_advect(h->g, parts, np, h->vel, h->counters, ps, 1, 0, order), "step advect");
+    if ((rc = particles.submit(ps, "step"))) return rc;
     if (h->side && (emit || np > 0)) {
         ISF_CUDA(h, cudaEventRecord(h->ev_read[h->vcur], h->side), "step particle event");
         ISF_CUDA(h, cudaEventRecord(h->ev_side, h->side), "step particle event");
@@ -763,10 +781,11 @@ int isf_poisson_solve(isf_handle* h, const float* f, float* q) {
     XArgs xa = xargs(h);
     xa.rin = f;
     xa.rout = q;
+    Sequence seq(h);
     ISF_LAUNCH(h, launch_xreal(XR_FWD, xa, h->stream), "poisson x fwd");
     if (int rc = run_poisson_spectral(h, "poisson")) return rc;
     ISF_LAUNCH(h, launch_xreal(XR_INV_REAL, xa, h->stream), "poisson x inv");
-    return ISF_OK;
+    return seq.submit(h->stream, "poisson_solve");
 }
 
 int isf_fft3(isf_handle* h, float* data, int32_t sign) {

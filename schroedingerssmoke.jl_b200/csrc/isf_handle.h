@@ -8,6 +8,19 @@
 #include "isf_launch.h"
 #include "isf_passes.cuh"
 
+// A sequence of kernels a handle has launched before (isf_seq.cu): the kernels,
+// and once it has come back often enough an executable graph of them.  The
+// graph holds no argument from one call to the next: every node's shape and
+// arguments are set anew for each launch.
+struct isf_seq {
+    std::vector<const void*> funcs;
+    cudaGraphExec_t exec = nullptr;
+    std::vector<cudaGraphNode_t> nodes;
+    cudaGraph_t graph = nullptr;
+    int seen = 0;             // calls so far (saturating)
+    bool failed = false;      // the graph could not be built: plain launches
+};
+
 struct isf_adj_state;  // adjoint work buffers, allocated on first use (isf_adj.cu)
 
 struct isf_handle {
@@ -49,6 +62,8 @@ struct isf_handle {
     std::vector<double> site_ms;
     std::vector<long long> site_count;
     isf_adj_state* adj = nullptr;
+    isf::LaunchList rec;               // the launches being recorded
+    std::vector<isf_seq> seqs;         // sequences seen
     // cell order of the particle slots (isf_set_particle_order / isf_sort_particles)
     int order_every = 0;                 // isf_step re-sorts every order_every steps (0: storage order)
     int order_age = 0;                   // isf_step advections since the last sort
@@ -109,6 +124,24 @@ int run_order(isf_handle* h, const float* parts, long long np, cudaStream_t st, 
 
 // releases the adjoint work buffers (isf_adj.cu)
 void adj_free(isf_handle* h);
+
+// While a Sequence is alive the kernels launched through launch_pdl on this
+// thread are recorded; submit() issues them on st as one graph launch, or one
+// after another (isf_seq.cu).  The code in between queues nothing else on st that
+// has to come after one of them.  Not while profiling, which times every launch.
+class Sequence {
+  public:
+    explicit Sequence(isf_handle* h);
+    ~Sequence();
+    int submit(cudaStream_t st, const char* where);
+
+  private:
+    isf_handle* h_;
+    LaunchList* outer_;
+    bool on_;
+};
+// releases the graphs of the handle's sequences
+void seq_free(isf_handle* h);
 
 }  // namespace isf_int
 

@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -11,12 +12,46 @@
 
 namespace isf {
 
+// The launches of one library call, recorded instead of issued (isf_seq.cu):
+// kernel, shape and a copy of the arguments each.
+struct LaunchList {
+    struct Rec {
+        const void* func;
+        dim3 grid, block;
+        size_t smem;
+        size_t arg0;  // first entry of offs
+        size_t nargs;
+    };
+    std::vector<Rec> recs;
+    std::vector<size_t> offs;      // argument offsets into bytes
+    std::vector<unsigned char> bytes;
+    void clear() {
+        recs.clear();
+        offs.clear();
+        bytes.clear();
+    }
+    template <class T>
+    void arg(const T& v) {
+        const size_t at = (bytes.size() + 15) & ~(size_t)15;
+        bytes.resize(at + sizeof(T));
+        std::memcpy(bytes.data() + at, &v, sizeof(T));
+        offs.push_back(at);
+    }
+};
+// the list this thread records into, or null: launches are issued
+extern thread_local LaunchList* t_record;
+
 // Launch with programmatic stream serialization: the kernel (which must call
 // pdl_enter before touching global memory) may be scheduled while the
 // previous kernel on the stream drains.
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args... args) {
+    if (LaunchList* l = t_record) {
+        l->recs.push_back({reinterpret_cast<const void*>(kernel), grid, block, smem, l->offs.size(), sizeof...(KArgs)});
+        (l->arg(static_cast<KArgs>(args)), ...);
+        return cudaSuccess;
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;

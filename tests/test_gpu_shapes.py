@@ -149,3 +149,49 @@ def test_schroedinger_flow_lengths(isfpkg, oracle_mod, dims):
     isf.sync()
     orc.schroedinger_flow(psi64)
     assert rel(host(psi), psi64) < 1e-5
+
+
+@pytest.mark.parametrize("L,dims", [((2, 1, 1), (32, 16, 16)), ((2, 2, 2), (40, 20, 24))])
+@pytest.mark.parametrize("caller_stream", [False, True])
+def test_sequences_as_graphs(isfpkg, cfgs, L, dims, caller_stream):
+    """A sequence of kernels that comes back is launched as a graph, with every
+    argument set per call: steps that change psi buffer, particle count, jet and
+    emission from call to call give the bits of a handle that launches kernel by
+    kernel (profiling), and so do steps under stream capture."""
+    st = torch.cuda.Stream() if caller_stream else None
+    a = isfpkg.ISF(L, dims, HBAR, DT, stream=st)
+    b = isfpkg.ISF(L, dims, HBAR, DT)
+    b.profile_start()
+    kvec, omega = cfgs.jet_omega()
+    psis = [[cuda(smooth_psi(dims, seed=70 + k)) for k in range(2)] for _ in range(2)]
+    rng = np.random.default_rng(71)
+    parts = [[cuda(p) for p in (rng.uniform(0, 1, (n, 3)) * np.asarray(L))] for n in (300, 5000)]
+    parts = [[torch.stack(p).contiguous() for p in parts] for _ in range(2)]
+    torch.cuda.synchronize()
+
+    def run(h, s, k):
+        jet = None
+        if k % 3:
+            jet = dict(kvec=kvec, omega_t=0.1 * k, cen=(0.3 * L[0], 0.5 * L[1], 0.5 * L[2]), len=0.1 + 0.01 * k, rad=0.3,
+                       emit_start=10 * k, emit_count=10 + k, seed=5, counter=k, emit_mode=1, phase_mode=1)
+        isfpkg.step(h, psis[s][k % 2], parts[s][(k // 2) % 2], jet)
+        isfpkg.schroedinger_flow(h, psis[s][(k + 1) % 2])
+        isfpkg.pressure_project(h, psis[s][(k + 1) % 2])
+
+    for k in range(24):
+        run(a, 0, k)
+        run(b, 1, k)
+    a.sync()
+    b.sync()
+    if caller_stream:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=st):
+            run(a, 0, 24)
+        g.replay()
+        run(b, 1, 24)
+        torch.cuda.synchronize()
+    for k in range(2):
+        assert torch.equal(psis[0][k], psis[1][k])
+        assert torch.equal(parts[0][k], parts[1][k])
+    assert a.counters()["live"] == b.counters()["live"]
+    b.profile_stop()
