@@ -250,6 +250,17 @@ struct JetArgs {
     const uint8_t* mask;     // optional precomputed isjet array (N bytes) or null
 };
 
+// |psi_c| exp(i ph) for both components: out of line, since the kernels that
+// restrict on the fly test every cell of several unrolled ones and few lie in
+// the nozzle.  Inlined, the copies of sincosf and hypotf were most of those
+// kernels' code, which small launches fetch cold.
+static __device__ __noinline__ float4 restrict_value(float4 v, float ph) {
+    float s, co;
+    sincosf(ph, &s, &co);
+    const float a1 = hypotf(v.x, v.y), a2 = hypotf(v.z, v.w);
+    return make_float4(a1 * co, a1 * s, a2 * co, a2 * s);
+}
+
 // restrict_kernel (particles.jl:12-20) for cell (x,y,z); returns true if
 // the cell is a nozzle cell and v was replaced.
 __device__ __forceinline__ bool restrict_cell(const Grid& g, const JetArgs& j, int x, int y, int z, long long c,
@@ -264,11 +275,7 @@ __device__ __forceinline__ bool restrict_cell(const Grid& g, const JetArgs& j, i
         ph = __fadd_rn(__fadd_rn(__fadd_rn(j.kvec[0], px), __fadd_rn(j.kvec[1], py)), __fadd_rn(j.kvec[2], pz));
     else
         ph = j.kvec[0] * px + j.kvec[1] * py + j.kvec[2] * pz;
-    ph = ph - j.omgterm;
-    float s, co;
-    sincosf(ph, &s, &co);
-    const float a1 = hypotf(v.x, v.y), a2 = hypotf(v.z, v.w);
-    v = make_float4(a1 * co, a1 * s, a2 * co, a2 * s);
+    v = restrict_value(v, ph - j.omgterm);
     return true;
 }
 

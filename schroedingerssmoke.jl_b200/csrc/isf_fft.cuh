@@ -453,6 +453,17 @@ struct Plan;
             if constexpr (SYNC) bar.sync();                                                                 \
             pipeline<NN, NT, L, S, T, Dst, B, 1, ISF_UNPAREN FWD>(x, t, q, sm, tw, dst, bar);               \
         }                                                                                                   \
+        /* run without the final scatter: butterfly i = t + b NT (i < N / RL) of the last radix RL keeps    \
+           output i + r N / RL at x[b RL + r] */                                                            \
+        template <class L, int S, bool SYNC, class T, class Src, class B = CtaBar>                          \
+        static __device__ __forceinline__ void run_keep(T* x, int t, int q, T* sm,                          \
+                                                        const float2* __restrict__ tw, const Src& src,      \
+                                                        const B& bar = B()) {                               \
+            gather<NN, NT, R0>(x, t, src);                                                                  \
+            if constexpr (SYNC) bar.sync();                                                                 \
+            pipeline_keep<NN, NT, L, S, T, B, 1, ISF_UNPAREN FWD>(x, t, q, sm, tw, bar);                    \
+        }                                                                                                   \
+        static constexpr int last = radix(First<ISF_UNPAREN REV>::value);                                   \
         /* forward transform, mul(j, v) on every output j in registers, inverse transform */               \
         /* (SYNC: barrier after the first gather, when src reads the tile)  */                             \
         template <class L, bool SYNC = false, class T, class Src, class Mul, class Dst, class B = CtaBar>   \

@@ -191,6 +191,10 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
     const int ny = a.g.n[1], nz = a.g.n[2];
     const int sim = bk.y;
     float2* __restrict__ Fs = a.F + sim * a.bs_F;
+    // k-major spectrum: this thread moves row pair kq for k = k0, k0 + NT, ...;
+    // row r = y + ny z lies at element k ny nz + r, a pair is one float4
+    const int kq = lt % C, k0 = lt / C;
+    const long long plane2 = ((long long)ny * nz) >> 1;
     T x[Plan<N>::EMAX];
     // row pairs past the last row (a row count that is not a multiple of
     // 2 C) read zeros and store nothing; the k-major layout has none
@@ -207,14 +211,11 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
         bar.sync();
         if constexpr (KM) {
             // lanes over the row pairs of the group: C x 16 B per k
-            float4* __restrict__ F4 = reinterpret_cast<float4*>(Fs);
-            for (int idx = lt; idx < (N / 2 + 1) * C; idx += C * NT) {
-                const int qq = idx % C, k = idx / C;
-                const float2 zk = sm[L::template at<N, NT>(k, qq)];
-                const float2 zn = sm[L::template at<N, NT>(k == 0 ? 0 : N - k, qq)];
-                const long long r = rbase + 2 * qq;
-                const int y = (int)(r % ny), z = (int)(r / ny);
-                F4[(((long long)k * nz + z) * ny + y) >> 1] =
+            float4* __restrict__ F4 = reinterpret_cast<float4*>(Fs) + ((rbase + 2 * kq) >> 1);
+            for (int k = k0; k <= N / 2; k += NT) {
+                const float2 zk = sm[L::template at<N, NT>(k, kq)];
+                const float2 zn = sm[L::template at<N, NT>(k == 0 ? 0 : N - k, kq)];
+                F4[k * plane2] =
                     make_float4(0.5f * (zk.x + zn.x), 0.5f * (zk.y - zn.y), 0.5f * (zk.y + zn.y), -0.5f * (zk.x - zn.x));
             }
         } else {
@@ -246,14 +247,10 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
         float4* stg = reinterpret_cast<float4*>(sm);
         auto sslot = [](int k, int qq) { return k * C + (qq ^ ((C == 4 ? k >> 1 : k) & (C - 1))); };
         if constexpr (KM) {
-            const float4* __restrict__ F4 = reinterpret_cast<const float4*>(Fs);
-            for (int idx = lt; idx < (N / 2 + 1) * C; idx += C * NT) {
-                const int qq = idx % C, k = idx / C;
-                const long long r = rbase + 2 * qq;
-                const int y = (int)(r % ny), z = (int)(r / ny);
-                const float4* from = &F4[(((long long)k * nz + z) * ny + y) >> 1];
-                if constexpr (kStaged) cp_async16(&stg[sslot(k, qq)], from);
-                else stg[sslot(k, qq)] = *from;
+            const float4* __restrict__ F4 = reinterpret_cast<const float4*>(Fs) + ((rbase + 2 * kq) >> 1);
+            for (int k = k0; k <= N / 2; k += NT) {
+                if constexpr (kStaged) cp_async16(&stg[sslot(k, kq)], &F4[k * plane2]);
+                else stg[sslot(k, kq)] = F4[k * plane2];
             }
         }
         if constexpr (kStaged) cp_async_wait();
@@ -277,32 +274,77 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
             return make_float2(u.x + v.y, v.x - u.y);
         };
         const long long b0 = r0 * N, b1 = b0 + N;
-        auto dst = [&](int j, const T& v) {
-            if constexpr (OP == XR_INV_REAL) {
-                if (v0) rout[b0 + j] = v.x;
-                if (v1) rout[b1 + j] = v.y;
-            } else {
-                static_assert(xr_gauge(OP), "unhandled real x-pass op");
-                // both rows' psi loaded before either is stored (two loads in flight)
-                float4 p0, p1;
-                if constexpr (kStaged) {
-                    p0 = ps[2 * q * N + j];
-                    p1 = ps[(2 * q + 1) * N + j];
-                } else {
-                    p0 = v0 ? psi[b0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-                    p1 = v1 ? psi[b1 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-                if constexpr (kJet) {
-                    if (v0) restrict_cell(a.g, jet, j, (int)(r0 % ny), (int)(r0 / ny), b0 + j, p0);
-                    if (v1) restrict_cell(a.g, jet, j, (int)((r0 + 1) % ny), (int)((r0 + 1) / ny), b1 + j, p1);
-                }
-                if (v0) psi[b0 + j] = gauge4(p0, v.x);
-                if (v1) psi[b1 + j] = gauge4(p1, v.y);
-            }
-        };
         // k-major: the staging aliases the tile, so the first gather must
         // complete before the first stage writes the tile
-        Plan<N>::template run<L, +1, KM>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
+        if constexpr (OP == XR_INV_REAL) {
+            auto dst = [&](int j, const T& v) {
+                if (v0) rout[b0 + j] = v.x;
+                if (v1) rout[b1 + j] = v.y;
+            };
+            Plan<N>::template run<L, +1, KM>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
+        } else {
+            static_assert(xr_gauge(OP), "unhandled real x-pass op");
+            if constexpr (kStaged) {
+                // (q of row 0, q of row 1) of each pair into the tile, then a
+                // loop over the group's cells: two copies of the gauge's code
+                // instead of one per output, and whole rows written in order
+                auto dst = [&](int j, const T& v) { sm[L::template at<N, NT>(j, q)] = v; };
+                Plan<N>::template run<L, +1, KM>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
+                bar.sync();
+                const int cells = (int)(rows - rbase < 2 * C ? rows - rbase : 2 * C) * N;
+                float4* __restrict__ out = psi + rbase * N;
+#pragma unroll 2
+                for (int i = lt; i < cells; i += C * NT) {
+                    const int row = i / N, j = i - row * N;
+                    const T qq = sm[L::template at<N, NT>(j, row >> 1)];
+                    float4 v = ps[i];
+                    if constexpr (kJet) {
+                        const unsigned r = (unsigned)rbase + row;
+                        restrict_cell(a.g, jet, j, (int)(r % (unsigned)ny), (int)(r / (unsigned)ny), rbase * N + i, v);
+                    }
+                    out[i] = gauge4(v, (row & 1) ? qq.y : qq.x);
+                }
+                return;
+            }
+            Plan<N>::template run_keep<L, +1, KM>(x, t, q, sm, a.g.tw[0], src, pencil_bar<NT, C>(bar));
+            int y0 = 0, z0 = 0, y1 = 0, z1 = 0;
+            if constexpr (kJet) {
+                const unsigned r = (unsigned)r0;
+                y0 = (int)(r % (unsigned)ny), z0 = (int)(r / (unsigned)ny);
+                y1 = y0 + 1 == ny ? 0 : y0 + 1, z1 = y1 == 0 ? z0 + 1 : z0;
+            }
+            // GB outputs of both rows at a time: their psi is loaded before any
+            // of them is stored (2 GB loads in flight)
+            constexpr int RL = Plan<N>::last, P = N / RL, NBT = Stage<N, NT, RL>::NBT;
+            constexpr int GB = N >= 256 ? 1 : (RL % 4 == 0 ? 4 : (RL % 2 == 0 ? 2 : 1));
+#pragma unroll
+            for (int b = 0; b < NBT; ++b) {
+                const int i = t + b * NT;
+                if (P % NT == 0 || i < P) {
+#pragma unroll
+                    for (int r = 0; r < RL; r += GB) {
+                        float4 p0[GB], p1[GB];
+#pragma unroll
+                        for (int u = 0; u < GB; ++u) {
+                            const int j = i + (r + u) * P;
+                            p0[u] = v0 ? psi[b0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+                            p1[u] = v1 ? psi[b1 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+                        }
+#pragma unroll
+                        for (int u = 0; u < GB; ++u) {
+                            const int j = i + (r + u) * P;
+                            const T v = x[b * RL + r + u];
+                            if constexpr (kJet) {
+                                if (v0) restrict_cell(a.g, jet, j, y0, z0, b0 + j, p0[u]);
+                                if (v1) restrict_cell(a.g, jet, j, y1, z1, b1 + j, p1[u]);
+                            }
+                            if (v0) psi[b0 + j] = gauge4(p0[u], v.x);
+                            if (v1) psi[b1 + j] = gauge4(p1[u], v.y);
+                        }
+                    }
+                }
+            }
+        }
     }
 }
 
@@ -313,13 +355,13 @@ __global__ void __launch_bounds__(XRShape<N, G, KM, C>::BLK) k_xreal(XArgs a) {
     xreal_body<N, OP, G, KM, C>(a, launch_blk(), smraw);
 }
 
-// The 16-pair pass compiled for 3 resident CTAs per SM (at most 42 registers),
-// launched for rows of at least 256 cells: the gauge pass at 256x128x128 ran
-// 35.4 -> 34.6 us.  The ensembles' short rows keep k_xreal (capped, their
-// batched step was 5 % slower), and so does the restricted gauge, which needs
-// its registers (nozzle projection at 256x128x128: 117 us, capped 124).
+// The 16-pair pass on rows of at least 256 cells, compiled for 3 resident CTAs
+// per SM (at most 42 registers; the gauge pass at 256x128x128 ran 35.4 -> 34.6
+// us), the restricted gauge for 2 (64 registers: nozzle projection there
+// 112 us, uncapped, at 72 registers and 1 CTA, 124).  The ensembles' short rows keep
+// k_xreal; capped, their batched step was 5 % slower.
 template <int N, int OP, int G, bool KM = false>
-__global__ void __launch_bounds__(XRShape<N, G, KM>::BLK, 3) k_xreal_long(XArgs a) {
+__global__ void __launch_bounds__(XRShape<N, G, KM>::BLK, OP == XR_INV_GAUGE_JET ? 2 : 3) k_xreal_long(XArgs a) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     xreal_body<N, OP, G, KM>(a, launch_blk(), smraw);

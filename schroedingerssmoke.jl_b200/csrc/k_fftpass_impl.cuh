@@ -54,7 +54,7 @@ cudaError_t launch_xr_ng(const XArgs& a, cudaStream_t s) {
     const long long rows = (long long)a.g.n[1] * a.g.n[2];
     if ((G > 1 || KM) && rows % (2 * Sh::C * G) != 0) return cudaErrorInvalidValue;
     constexpr auto kern = [] {
-        if constexpr (N >= 256 && C == 16 && OP != XR_INV_GAUGE_JET) return k_xreal_long<N, OP, G, KM>;
+        if constexpr (N >= 256 && C == 16) return k_xreal_long<N, OP, G, KM>;
         else return k_xreal<N, OP, G, KM, C>;
     }();
     cudaError_t e = ensure_smem(kern, Sh::SMEM, done);

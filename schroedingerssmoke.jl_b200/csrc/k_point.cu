@@ -14,36 +14,39 @@ static inline unsigned grid_for(long long n, int block) {
 
 // normalize_psi broadcast (parallel.jl:162-165, examples/benchmark.jl:50)
 __global__ void k_normalize(float4* __restrict__ psi, long long N) {
+    pdl_enter();
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N; c += (long long)gridDim.x * blockDim.x)
         psi[c] = normalize4(psi[c]);
 }
 
 // restrict_velocity! (particles.jl:25-27 -> restrict_kernel :12-20)
-__global__ void k_restrict(Grid g, float4* __restrict__ psi, JetArgs j) {
-    const long long N = g.N;
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N; c += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(c % g.n[0]);
-        const long long r = c / g.n[0];
-        const int y = (int)(r % g.n[1]), z = (int)(r / g.n[1]);
+__global__ void __launch_bounds__(256) k_restrict(Grid g, float4* __restrict__ psi, JetArgs j) {
+    pdl_enter();
+    const int x = cell_x(), y = cell_y();
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
+        const long long c = cell(g, x, y, z);
         float4 v = psi[c];
         if (restrict_cell(g, j, x, y, z, c, v)) psi[c] = v;
     }
 }
 
 // isjet.(isf.positions, ...) (particles.jl:6-10, examples/benchmark.jl:26)
-__global__ void k_isjet(Grid g, uint8_t* __restrict__ out, float c0, float c1, float c2, float len, float rad) {
+__global__ void __launch_bounds__(256) k_isjet(Grid g, uint8_t* __restrict__ out, float c0, float c1, float c2, float len,
+                                               float rad) {
+    pdl_enter();
     const float cen[3] = {c0, c1, c2};
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        const int x = (int)(c % g.n[0]);
-        const long long r = c / g.n[0];
-        const int y = (int)(r % g.n[1]), z = (int)(r / g.n[1]);
+    const int x = cell_x(), y = cell_y();
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const float px = __fmul_rn((float)x, g.d[0]), py = __fmul_rn((float)y, g.d[1]), pz = __fmul_rn((float)z, g.d[2]);
-        out[c] = isjet_f32(px, py, pz, cen, len, rad) ? 1 : 0;
+        out[cell(g, x, y, z)] = isjet_f32(px, py, pz, cen, len, rad) ? 1 : 0;
     }
 }
 
 // staggered sharp on the handle's padded velocity grid (examples/benchmark.jl:61-63)
 __global__ void k_sharp(Grid g, float4* __restrict__ vel) {
+    pdl_enter();
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.NP; c += (long long)gridDim.x * blockDim.x) {
         float4 v = vel[c];
         v.x = __fmul_rn(v.x, g.dinv[0]);
@@ -53,44 +56,51 @@ __global__ void k_sharp(Grid g, float4* __restrict__ vel) {
     }
 }
 
-__device__ __forceinline__ void decode(const Grid& g, long long c, int& x, int& y, int& z) {
-    x = (int)(c % g.n[0]);
-    const long long r = c / g.n[0];
-    y = (int)(r % g.n[1]);
-    z = (int)(r / g.n[1]);
-}
-
 // div! (parallel.jl:131-152) from the padded velocity grid
-__global__ void k_div(Grid g, const float4* __restrict__ vel, float* __restrict__ f) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode(g, c, x, y, z);
-        const int xm = (x == 0) ? g.n[0] - 1 : x - 1;
-        const int ym = (y == 0) ? g.n[1] - 1 : y - 1;
+__global__ void __launch_bounds__(256) k_div(Grid g, const float4* __restrict__ vel, float* __restrict__ f) {
+    pdl_enter();
+    const int x = cell_x(), y = cell_y();
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    const int xm = (x == 0) ? g.n[0] - 1 : x - 1, ym = (y == 0) ? g.n[1] - 1 : y - 1;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const int zm = (z == 0) ? g.n[2] - 1 : z - 1;
         const float4 v = vel[pcell(g, x, y, z)];
         const float t0 = (v.x - vel[pcell(g, xm, y, z)].x) * g.inv_d2[0];
         const float t1 = (v.y - vel[pcell(g, x, ym, z)].y) * g.inv_d2[1];
         const float t2 = (v.z - vel[pcell(g, x, y, zm)].z) * g.inv_d2[2];
-        f[c] = (t0 + t1) + t2;
+        f[cell(g, x, y, z)] = (t0 + t1) + t2;
     }
 }
 
-__global__ void k_vel_to_aos(Grid g, const float4* __restrict__ vel, float* __restrict__ aos) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode(g, c, x, y, z);
-        const float4 v = vel[pcell(g, x, y, z)];
-        aos[3 * c + 0] = v.x;
-        aos[3 * c + 1] = v.y;
-        aos[3 * c + 2] = v.z;
+// The velocity as AoS float3, one warp per 32 cells of a row: the cells' 384
+// bytes leave as three whole 128-byte stores per warp, each lane fetching the
+// components of its words from the lanes that loaded them (12-byte strided
+// stores touch every sector three times).
+__global__ void __launch_bounds__(256) k_vel_to_aos(Grid g, const float4* __restrict__ vel, float* __restrict__ aos) {
+    pdl_enter();
+    const int lane = threadIdx.x & 31, x0 = (int)blockIdx.x * 32, y = cell_y();
+    if (y >= g.n[1]) return;  // whole warps
+    const int nw = 3 * min(32, g.n[0] - x0);  // words of this warp's cells
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (x0 + lane < g.n[0]) v = vel[pcell(g, x0 + lane, y, z)];
+        float* o = aos + 3 * cell(g, x0, y, z);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const int w = lane + 32 * k, from = w / 3, comp = w - 3 * from;
+            const float vx = __shfl_sync(0xffffffffu, v.x, from), vy = __shfl_sync(0xffffffffu, v.y, from),
+                        vz = __shfl_sync(0xffffffffu, v.z, from);
+            if (w < nw) o[w] = comp == 0 ? vx : (comp == 1 ? vy : vz);
+        }
     }
 }
 
-__global__ void k_vel_from_aos(Grid g, const float* __restrict__ aos, float4* __restrict__ vel) {
-    for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < g.N; c += (long long)gridDim.x * blockDim.x) {
-        int x, y, z;
-        decode(g, c, x, y, z);
+__global__ void __launch_bounds__(256) k_vel_from_aos(Grid g, const float* __restrict__ aos, float4* __restrict__ vel) {
+    pdl_enter();
+    const int x = cell_x(), y = cell_y();
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
+        const long long c = cell(g, x, y, z);
         pstore(g, vel, x, y, z, make_float3(aos[3 * c + 0], aos[3 * c + 1], aos[3 * c + 2]));
     }
 }
@@ -122,32 +132,25 @@ cudaError_t launch_scale_c(const Grid& g, float2* a, float s, cudaStream_t st) {
     return cudaGetLastError();
 }
 cudaError_t launch_normalize(const Grid& g, float4* psi, cudaStream_t s) {
-    k_normalize<<<grid_for(g.N, 256), 256, 0, s>>>(psi, g.N);
-    return cudaGetLastError();
+    return launch_pdl(k_normalize, dim3(grid_for(g.N, 256)), dim3(256), 0, s, psi, g.N);
 }
 cudaError_t launch_restrict(const Grid& g, float4* psi, const JetArgs& j, cudaStream_t s) {
-    k_restrict<<<grid_for(g.N, 256), 256, 0, s>>>(g, psi, j);
-    return cudaGetLastError();
+    return launch_pdl(k_restrict, cell_grid(g), dim3(256), 0, s, g, psi, j);
 }
 cudaError_t launch_isjet(const Grid& g, uint8_t* out, const float* cen, float len, float rad, cudaStream_t s) {
-    k_isjet<<<grid_for(g.N, 256), 256, 0, s>>>(g, out, cen[0], cen[1], cen[2], len, rad);
-    return cudaGetLastError();
+    return launch_pdl(k_isjet, cell_grid(g), dim3(256), 0, s, g, out, cen[0], cen[1], cen[2], len, rad);
 }
 cudaError_t launch_sharp(const Grid& g, float* vel, cudaStream_t s) {
-    k_sharp<<<grid_for(g.NP, 256), 256, 0, s>>>(g, reinterpret_cast<float4*>(vel));
-    return cudaGetLastError();
+    return launch_pdl(k_sharp, dim3(grid_for(g.NP, 256)), dim3(256), 0, s, g, reinterpret_cast<float4*>(vel));
 }
 cudaError_t launch_div(const Grid& g, const float* vel, float* f, cudaStream_t s) {
-    k_div<<<grid_for(g.N, 256), 256, 0, s>>>(g, reinterpret_cast<const float4*>(vel), f);
-    return cudaGetLastError();
+    return launch_pdl(k_div, cell_grid(g), dim3(256), 0, s, g, reinterpret_cast<const float4*>(vel), f);
 }
 cudaError_t launch_vel_to_aos(const Grid& g, const float* vel, float* aos, cudaStream_t s) {
-    k_vel_to_aos<<<grid_for(g.N, 256), 256, 0, s>>>(g, reinterpret_cast<const float4*>(vel), aos);
-    return cudaGetLastError();
+    return launch_pdl(k_vel_to_aos, cell_grid(g), dim3(256), 0, s, g, reinterpret_cast<const float4*>(vel), aos);
 }
 cudaError_t launch_vel_from_aos(const Grid& g, const float* aos, float* vel, cudaStream_t s) {
-    k_vel_from_aos<<<grid_for(g.N, 256), 256, 0, s>>>(g, aos, reinterpret_cast<float4*>(vel));
-    return cudaGetLastError();
+    return launch_pdl(k_vel_from_aos, cell_grid(g), dim3(256), 0, s, g, aos, reinterpret_cast<float4*>(vel));
 }
 
 }  // namespace isf
