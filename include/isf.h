@@ -434,6 +434,21 @@ ISF_API int isf_launch_count(const isf_handle* h, uint64_t* out);
 /* psi (float4 per cell) from / to psi1, psi2 (complex128 per cell) */
 ISF_API int isf_psi_from_f64(isf_handle* h, const double* psi1, const double* psi2, float* psi);
 ISF_API int isf_psi_to_f64(isf_handle* h, const float* psi, double* psi1, double* psi2);
+/* The conversions in, the operator and the conversions out as one call:
+ * SchroedingerFlow, Normalize, PressureProject (src/MatlabPort.jl:87-93, 147-160),
+ * VelocityOneForm and StaggeredSharp (:99-126).  psi is a float4-per-cell work
+ * array of the caller (overwritten); the results equal those of the three calls
+ * each stands for, the handle's velocity included. */
+ISF_API int isf_f64_schroedinger_flow(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1,
+                                      double* out2);
+ISF_API int isf_f64_normalize(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1,
+                              double* out2);
+ISF_API int isf_f64_pressure_project(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1,
+                                     double* out2);
+ISF_API int isf_f64_velocity_one_form(isf_handle* h, const double* psi1, const double* psi2, float* psi, float hbar,
+                                      double* vx, double* vy, double* vz);
+ISF_API int isf_f64_staggered_sharp(isf_handle* h, const double* vx, const double* vy, const double* vz, double* ox,
+                                    double* oy, double* oz);
 /* the handle's velocity from / to vx, vy, vz (float64 per cell) */
 ISF_API int isf_velocity_from_f64(isf_handle* h, const double* vx, const double* vy, const double* vz);
 ISF_API int isf_velocity_to_f64(isf_handle* h, double* vx, double* vy, double* vz);

@@ -32,7 +32,8 @@ EXPORTS = (
     "isf_adj_schroedinger_flow", "isf_adj_normalize_psi", "isf_adj_pressure_project", "isf_adj_restrict_velocity",
     "isf_adj_velocity_one_form", "isf_adj_staggered_advect", "isf_adj_get_velocity_bar", "isf_adj_set_velocity_bar",
     "isf_adj_step", "isf_adj_loss", "isf_adj_gradient",
-    "isf_psi_from_f64", "isf_psi_to_f64", "isf_velocity_from_f64", "isf_velocity_to_f64", "isf_real_from_f64",
+    "isf_f64_schroedinger_flow", "isf_f64_normalize", "isf_f64_pressure_project", "isf_f64_velocity_one_form",
+    "isf_f64_staggered_sharp", "isf_psi_from_f64", "isf_psi_to_f64", "isf_velocity_from_f64", "isf_velocity_to_f64", "isf_real_from_f64",
     "isf_real_to_f64", "isf_complex_to_f64", "isf_gauge_transform", "isf_add_particles_soa",
     "isf_staggered_velocity", "isf_advect_active", "isf_keep_inside", "isf_gather_particles",
     "isf_set_particle_order", "isf_sort_particles", "isf_get_particle_order", "isf_batch_set_persistent",
@@ -193,6 +194,11 @@ def load(path: str | None = None):
         "isf_adj_step": [vp, vp, vp, i64, C.POINTER(IsfStepArgs), vp, vp, dp],
         "isf_adj_loss": [vp, C.POINTER(IsfAdjProblem), vp, vp, i64, vp, dp],
         "isf_adj_gradient": [vp, C.POINTER(IsfAdjProblem), vp, vp, i64, vp, dp, vp, vp, dp],
+        "isf_f64_schroedinger_flow": [vp] * 6,
+        "isf_f64_normalize": [vp] * 6,
+        "isf_f64_pressure_project": [vp] * 6,
+        "isf_f64_velocity_one_form": [vp, vp, vp, vp, C.c_float, vp, vp, vp],
+        "isf_f64_staggered_sharp": [vp] * 7,
         "isf_psi_from_f64": [vp, vp, vp, vp],
         "isf_psi_to_f64": [vp, vp, vp, vp],
         "isf_velocity_from_f64": [vp, vp, vp, vp],

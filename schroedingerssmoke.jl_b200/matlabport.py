@@ -92,6 +92,15 @@ class _Grid:
         nx, ny, nz = self.res
         return torch.empty((nz, ny, nx), dtype=dtype, device=self.device).permute(2, 1, 0)
 
+    def psi_call(self, fn, psi1, psi2):
+        """fn on (psi1, psi2): conversions and operator in one library call"""
+        a, h1 = self.field(psi1, torch.complex128)
+        b, h2 = self.field(psi2, torch.complex128)
+        oa, ob = self.new(torch.complex128), self.new(torch.complex128)
+        self.chk(fn(self.h, _vp(a), _vp(b), _vp(self.psi), _vp(oa), _vp(ob)))
+        host = h1 or h2
+        return _out(oa, host), _out(ob, host)
+
     def psi_in(self, psi1, psi2):
         a, h1 = self.field(psi1, torch.complex128)
         b, h2 = self.field(psi2, torch.complex128)
@@ -214,25 +223,27 @@ class ISF:
 def SchroedingerFlow(obj: ISF, psi1, psi2):
     """MatlabPort.jl:87-93: solves the Schroedinger equation for dt."""
     g = obj._g
-    host = g.psi_in(psi1, psi2)
-    g.chk(g.L.isf_schroedinger_flow(g.h, _vp(g.psi)))
-    return g.psi_out(host)
+    return g.psi_call(g.L.isf_f64_schroedinger_flow, psi1, psi2)
 
 
 def StaggeredSharp(obj: ISF, vx, vy, vz):
     """MatlabPort.jl:99-104: the staggered vector field v^sharp = v / d."""
     g = obj._g
-    host = g.vel_in(vx, vy, vz)
-    g.chk(g.L.isf_staggered_sharp(g.h))
-    return g.vel_out(host)
+    (a, h1), (b, h2), (c, h3) = g.field(vx), g.field(vy), g.field(vz)
+    o = [g.new() for _ in range(3)]
+    g.chk(g.L.isf_f64_staggered_sharp(g.h, _vp(a), _vp(b), _vp(c), *(_vp(t) for t in o)))
+    host = h1 or h2 or h3
+    return tuple(_out(t, host) for t in o)
 
 
 def VelocityOneForm(obj: ISF, psi1, psi2, hbar=1.0):
     """MatlabPort.jl:106-126: v_a = hbar angle(conj psi1 psi1[+e_a] + conj psi2 psi2[+e_a])."""
     g = obj._g
-    host = g.psi_in(psi1, psi2)
-    g.chk(g.L.isf_velocity_one_form(g.h, _vp(g.psi), float(hbar)))
-    return g.vel_out(host)
+    (a, h1), (b, h2) = g.field(psi1, torch.complex128), g.field(psi2, torch.complex128)
+    o = [g.new() for _ in range(3)]
+    g.chk(g.L.isf_f64_velocity_one_form(g.h, _vp(a), _vp(b), _vp(g.psi), float(hbar), *(_vp(t) for t in o)))
+    host = h1 or h2
+    return tuple(_out(t, host) for t in o)
 
 
 def PoissonSolve(obj: ISF, f):
@@ -267,17 +278,13 @@ def GaugeTransform(psi1, psi2, q):
 def PressureProject(obj: ISF, psi1, psi2):
     """MatlabPort.jl:147-153: one-form (hbar 1), Div, PoissonSolve, gauge."""
     g = obj._g
-    host = g.psi_in(psi1, psi2)
-    g.chk(g.L.isf_pressure_project(g.h, _vp(g.psi)))
-    return g.psi_out(host)
+    return g.psi_call(g.L.isf_f64_pressure_project, psi1, psi2)
 
 
 def Normalize(psi1, psi2):
     """MatlabPort.jl:155-160: psi / sqrt(|psi1|^2 + |psi2|^2)."""
     g = _context(tuple(psi1.shape), _device_of(psi1, psi2))
-    host = g.psi_in(psi1, psi2)
-    g.chk(g.L.isf_normalize_psi(g.h, _vp(g.psi)))
-    return g.psi_out(host)
+    return g.psi_call(g.L.isf_f64_normalize, psi1, psi2)
 
 
 def Div(obj: ISF, vx, vy, vz):
