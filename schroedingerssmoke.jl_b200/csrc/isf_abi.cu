@@ -277,23 +277,19 @@ int run_one_form(isf_handle* h, const float* psi, float hbar, int sharp, const c
     return ISF_OK;
 }
 
-// pressure_project! with the optional nozzle restriction fused in front:
+// pressure_project!, after the nozzle restriction (in place) with a jet:
 // f = div(one-form) -> Poisson solve -> gauge
 int run_projection(isf_handle* h, float* psi, const JetArgs* jet) {
+    if (jet)
+        ISF_LAUNCH(h, launch_restrict(h->g, reinterpret_cast<float4*>(psi), *jet, h->stream), "projection restrict");
     StencilArgs sa = stargs(h, psi, h->f);
     XArgs xa = xargs(h);
     xa.psi = reinterpret_cast<float4*>(psi);
     xa.rin = h->f;
-    if (jet) {
-        sa.jet = *jet;
-        sa.use_jet = 1;
-        xa.jet = *jet;
-        xa.use_jet = 1;
-    }
     ISF_LAUNCH(h, launch_stencil(ST_DIV, sa, h->stream), "projection div");
     ISF_LAUNCH(h, launch_xreal(XR_FWD, xa, h->stream), "projection x fwd");
     if (int rc = run_poisson_spectral(h, "projection")) return rc;
-    ISF_LAUNCH(h, launch_xreal(jet ? XR_INV_GAUGE_JET : XR_INV_GAUGE, xa, h->stream), "projection x inv + gauge");
+    ISF_LAUNCH(h, launch_xreal(XR_INV_GAUGE, xa, h->stream), "projection x inv + gauge");
     return ISF_OK;
 }
 
@@ -612,8 +608,7 @@ int isf_init_jet(isf_handle* h, float* psi, int32_t iters, const float kvec[3], 
     if (phase_mode != ISF_PHASE_REFERENCE_SUM && phase_mode != ISF_PHASE_DOT)
         return fail(h, ISF_ERR_INVALID, "isf_init_jet: bad phase_mode");
     const float zero[3] = {0.f, 0.f, 0.f};
-    // restrict_velocity!(isf, psi, kvec, isjet, 0) + pressure_project!, the
-    // restriction fused into the projection's stencil and gauge pass as in isf_step
+    // restrict_velocity!(isf, psi, kvec, isjet, 0) + pressure_project!
     JetArgs j = make_jet(kvec, mask, cen ? cen : zero, len, rad, 0.f, phase_mode);
     for (int it = 0; it < iters; ++it) {
         Sequence seq(h);

@@ -228,12 +228,7 @@ cudaError_t class_projection(const BatchClass& c, const JetArgs* jets, cudaStrea
     cudaError_t e;
     StencilArgs sa = bst(c, c.f, c.g.N);
     XArgs xa = bx(c, c.tiles[ISF_TILE_X_REAL]);
-    if (jets) {
-        sa.use_jet = 1;
-        sa.jets = jets;
-        xa.use_jet = 1;
-        xa.jets = jets;
-    }
+    if (jets && (e = launch_restrict_batch(c.g, c.psi, jets, c.nsim, c.g.N, s)) != cudaSuccess) return e;
     if ((e = launch_stencil(ST_DIV, sa, s)) != cudaSuccess) return e;
     if ((e = launch_xreal(XR_FWD, xa, s)) != cudaSuccess) return e;
     if (c.kmajor) {
@@ -243,7 +238,7 @@ cudaError_t class_projection(const BatchClass& c, const JetArgs* jets, cudaStrea
         if ((e = launch_yzpass_c(YZ_FAC, byz(c, true, 2, c.tiles[ISF_TILE_Z_HALF]), s)) != cudaSuccess) return e;
         if ((e = launch_yzpass_c(YZ_INV, byz(c, true, 1, c.tiles[ISF_TILE_Y_HALF]), s)) != cudaSuccess) return e;
     }
-    return launch_xreal(jets ? XR_INV_GAUGE_JET : XR_INV_GAUGE, xa, s);
+    return launch_xreal(XR_INV_GAUGE, xa, s);
 }
 
 // the simloop body of isf_step for every simulation of the class
@@ -474,10 +469,10 @@ bool class_chain(const isf_batch* b, const BatchClass& c, int ci, std::vector<PP
         PPhase gi = new_phase(c, ci, PK_XR_INV_GAUGE, nx, rows / 32, ns, 1);
         gi.x = bx(c, 1);
         if (jets) {
-            d.st.use_jet = 1;
-            d.st.jets = jets;
-            gi.x.use_jet = 1;
-            gi.x.jets = jets;
+            // one virtual CTA per (32 x 8) column tile
+            PPhase r = new_phase(c, ci, PK_RESTRICT, 0, up(nx, 32), up(ny, 8), ns);
+            r.psi = c.psi;
+            out.push_back(r);
         }
         out.push_back(d);
         out.push_back(f);
@@ -544,7 +539,8 @@ int build_plan(isf_batch* b, int reps, int blocks_per_sm_cap) {
     // chain, and a few also wait for a pass of the previous step, so that
     // step n's advection runs beside step n+1's psi passes:
     //   prologue(n+1) after the last pass of step n that reads the jet and
-    //     emission arguments it rewrites (the jet projection's gauge pass);
+    //     emission arguments it rewrites (the restriction, which follows the
+    //     emission);
     //   x fwd(n+1), which transforms psi in place, after the one-form of step
     //     n, the last reader of psi;
     //   emission and one-form of step n+1, which write the particles and the
@@ -560,14 +556,13 @@ int build_plan(isf_batch* b, int reps, int blocks_per_sm_cap) {
                 }
             return found;
         };
-        const bool jet = b->cls[ci].key.jet;
         const int vel = slot(PK_VEL, true), adv = slot(PK_ADVECT, true);
-        const int jet_gauge = jet ? slot(PK_XR_INV_GAUGE, true) : -1;
+        const int jet_last = std::max(slot(PK_RESTRICT, true), slot(PK_EMIT, true));
         for (size_t j = 0; j < ch.size(); ++j) {
             PPhase& p = ph[slot_of[ci][j]];
             p.dep = j > 0 ? slot_of[ci][j - 1] : -1;
             switch (p.kind) {
-                case PK_PROLOGUE: p.dep_prev = jet_gauge; break;
+                case PK_PROLOGUE: p.dep_prev = jet_last; break;
                 case PK_X_FWD: p.dep_prev = vel; break;
                 case PK_EMIT: case PK_VEL: p.dep_prev = adv; break;
                 default: p.dep_prev = -1; break;

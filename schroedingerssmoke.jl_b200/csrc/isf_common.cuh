@@ -250,33 +250,47 @@ struct JetArgs {
     const uint8_t* mask;     // optional precomputed isjet array (N bytes) or null
 };
 
-// |psi_c| exp(i ph) for both components: out of line, since the kernels that
-// restrict on the fly test every cell of several unrolled ones and few lie in
-// the nozzle.  Inlined, the copies of sincosf and hypotf were most of those
-// kernels' code, which small launches fetch cold.
-static __device__ __noinline__ float4 restrict_value(float4 v, float ph) {
+// is (x, y, z), cell c, a nozzle cell?
+__device__ __forceinline__ bool jet_cell(const Grid& g, const JetArgs& j, int x, int y, int z, long long c) {
+    if (j.mask) return j.mask[c] != 0;
+    return isjet_f32(__fmul_rn((float)x, g.d[0]), __fmul_rn((float)y, g.d[1]), __fmul_rn((float)z, g.d[2]), j.cen, j.len,
+                     j.rad);
+}
+
+// restrict_kernel (particles.jl:12-20) at the nozzle cell (x, y, z): |psi_c| exp(i phase)
+__device__ __forceinline__ float4 restrict_value(const Grid& g, const JetArgs& j, int x, int y, int z, float4 v) {
+    const float px = __fmul_rn((float)x, g.d[0]);
+    const float py = __fmul_rn((float)y, g.d[1]);
+    const float pz = __fmul_rn((float)z, g.d[2]);
+    float ph;
+    if (j.phase_mode == 0)
+        ph = __fadd_rn(__fadd_rn(__fadd_rn(j.kvec[0], px), __fadd_rn(j.kvec[1], py)), __fadd_rn(j.kvec[2], pz));
+    else
+        ph = j.kvec[0] * px + j.kvec[1] * py + j.kvec[2] * pz;
+    ph = ph - j.omgterm;
     float s, co;
     sincosf(ph, &s, &co);
     const float a1 = hypotf(v.x, v.y), a2 = hypotf(v.z, v.w);
     return make_float4(a1 * co, a1 * s, a2 * co, a2 * s);
 }
 
-// restrict_kernel (particles.jl:12-20) for cell (x,y,z); returns true if
-// the cell is a nozzle cell and v was replaced.
-__device__ __forceinline__ bool restrict_cell(const Grid& g, const JetArgs& j, int x, int y, int z, long long c,
-                                              float4& v) {
-    const float px = __fmul_rn((float)x, g.d[0]);
-    const float py = __fmul_rn((float)y, g.d[1]);
-    const float pz = __fmul_rn((float)z, g.d[2]);
-    bool jet = j.mask ? (j.mask[c] != 0) : isjet_f32(px, py, pz, j.cen, j.len, j.rad);
-    if (!jet) return false;
-    float ph;
-    if (j.phase_mode == 0)
-        ph = __fadd_rn(__fadd_rn(__fadd_rn(j.kvec[0], px), __fadd_rn(j.kvec[1], py)), __fadd_rn(j.kvec[2], pz));
-    else
-        ph = j.kvec[0] * px + j.kvec[1] * py + j.kvec[2] * pz;
-    v = restrict_value(v, ph - j.omgterm);
-    return true;
+// restrict_velocity! (particles.jl:25-27) on column (x, y), planes z0, z0 +
+// dz, ...  A column outside the nozzle's length, or further from its axis in
+// y alone than the radius (the sum of the rounded squares is no less than
+// either), has no nozzle cell and is left at once.
+__device__ __forceinline__ void restrict_columns(const Grid& g, float4* __restrict__ psi, const JetArgs& j, int x, int y,
+                                                 int z0, int dz) {
+    if (x >= g.n[0] || y >= g.n[1]) return;
+    if (!j.mask) {
+        const float ey = __fsub_rn(__fmul_rn((float)y, g.d[1]), j.cen[1]);
+        if (!(fabsf(__fsub_rn(__fmul_rn((float)x, g.d[0]), j.cen[0])) <= __fdiv_rn(j.len, 2.0f)) ||
+            __fmul_rn(ey, ey) > __fmul_rn(j.rad, j.rad))
+            return;
+    }
+    for (int z = z0; z < g.n[2]; z += dz) {
+        const long long c = cell(g, x, y, z);
+        if (jet_cell(g, j, x, y, z, c)) psi[c] = restrict_value(g, j, x, y, z, psi[c]);
+    }
 }
 
 // normalize_psi (parallel.jl:162-165): psi * (1 / |psi|) with the

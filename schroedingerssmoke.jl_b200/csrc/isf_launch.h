@@ -108,16 +108,12 @@ struct StencilArgs {
     Grid g;
     const float4* psi;
     float* out;  // ST_DIV: f[N]; ST_VEL: padded velocity grid, float4 (vx, vy, vz, 0) per cell (kVelComp NP floats)
-    JetArgs jet;
-    int use_jet;
     float hbar;
     int sharp;
     // a batch of nsim simulations of this grid (0 or 1: a single one):
-    // simulation s reads psi + s * bs_psi, writes out + s * bs_out and, with
-    // jets != null, restricts with jets[s] instead of jet
+    // simulation s reads psi + s * bs_psi and writes out + s * bs_out
     int nsim;
     long long bs_psi, bs_out;
-    const JetArgs* jets;
     int sz;  // z planes per CTA: chosen by launch_stencil from the grid, fixed in the persistent batch kernel
 };
 cudaError_t launch_stencil(int op, const StencilArgs& a, cudaStream_t s);
@@ -125,6 +121,9 @@ cudaError_t launch_stencil(int op, const StencilArgs& a, cudaStream_t s);
 // pointwise kernels (k_point.cu)
 cudaError_t launch_normalize(const Grid& g, float4* psi, cudaStream_t s);
 cudaError_t launch_restrict(const Grid& g, float4* psi, const JetArgs& j, cudaStream_t s);
+// nsim simulations, psi bs_psi cells apart, simulation s with jets[s] (device array)
+cudaError_t launch_restrict_batch(const Grid& g, float4* psi, const JetArgs* jets, int nsim, long long bs_psi,
+                                  cudaStream_t s);
 cudaError_t launch_isjet(const Grid& g, uint8_t* out, const float* cen, float len, float rad, cudaStream_t s);
 cudaError_t launch_sharp(const Grid& g, float* vel, cudaStream_t s);
 cudaError_t launch_div(const Grid& g, const float* vel, float* f, cudaStream_t s);

@@ -5,7 +5,7 @@
 //   Schroedinger step  x fwd | y fwd | z fwd * mask/N, z inv | y inv | x inv + normalize
 //   Poisson solve      real-to-complex x fwd of the divergence f | y fwd on the half
 //                      spectrum | z fwd * fac/N, z inv | y inv | complex-to-real x inv
-//                      + gauge of psi (+ the nozzle restriction)
+//                      + gauge of psi
 // so the reference's split/merge broadcasts (parallel.jl:179-180, 185), the
 // complex(f) copy (:169), the mask / fac multiplies (:171, :182-183) and the
 // gauge broadcast (:159) never touch HBM on their own.
@@ -40,15 +40,12 @@ struct XArgs {
     float2* F;
     const float* rin;
     float* rout;
-    JetArgs jet;
-    int use_jet;
     int wp;  // row stride (complex elements) of the half spectrum of real data
     // a batch of nsim simulations of this grid (blockIdx.y = simulation;
     // 0 or 1: a single one): element strides between simulations of psi, F
-    // and the real rows, and per-simulation jets (null: jet)
+    // and the real rows
     int nsim;
     long long bs_psi, bs_F, bs_r;
-    const JetArgs* jets;
     int groups;  // pencil groups per CTA (0 or 1: one)
     int kmajor;  // real x passes: the half spectrum is k-major (see k_xreal)
 };
@@ -131,7 +128,7 @@ __global__ void __launch_bounds__(XShape<N, OP, G>::BLK) k_xpass(XArgs a) {
 //   XR_FWD        f rows -> half spectra A[k], B[k], k = 0..N/2, with
 //                 A = (Z_k + conj Z_{N-k}) / 2 and B = (Z_k - conj Z_{N-k}) / 2i
 //   XR_INV_GAUGE  Z_j = A_j + i B_j (Hermitian extension for j > N/2) ->
-//                 inverse -> q rows (Re, Im) -> psi = gauge(psi (restricted), q)
+//                 inverse -> q rows (Re, Im) -> psi = gauge(psi, q)
 //   XR_INV_REAL   the same inverse, q rows to a real output array
 // Half-spectrum layouts:
 //   row-major (KM = false)  row r's spectrum at F + r * wp (wp >= N/2 + 1,
@@ -141,10 +138,7 @@ __global__ void __launch_bounds__(XShape<N, OP, G>::BLK) k_xpass(XArgs a) {
 //                           (k_poisson_plane); A and B of a row pair are
 //                           neighbours, moved as one 16-byte vector, with the
 //                           lanes running over row pairs.
-//   XR_INV_GAUGE_JET  the gauge with psi restricted in the nozzle first (use_jet):
-//                 a separate op so that the plain gauge carries none of the
-//                 restriction's code
-enum XROp { XR_FWD = 0, XR_INV_GAUGE = 1, XR_INV_REAL = 2, XR_INV_GAUGE_JET = 3 };
+enum XROp { XR_FWD = 0, XR_INV_GAUGE = 1, XR_INV_REAL = 2 };
 
 // C row pairs per pencil group: 4 (8 rows) or 16, chosen by launch_xr_one
 // (k_fftpass.cu); the grouped tiles of the ensembles and the persistent kernel
@@ -166,7 +160,7 @@ struct XRShape {
     static_assert(PSI == 0 || G == 1, "one group where psi is staged");
 };
 
-constexpr bool xr_gauge(int op) { return op == XR_INV_GAUGE || op == XR_INV_GAUGE_JET; }
+constexpr bool xr_gauge(int op) { return op == XR_INV_GAUGE; }
 
 // 16-byte asynchronous copy from global to shared memory
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -256,9 +250,6 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
         if constexpr (kStaged) cp_async_wait();
         if constexpr (KM || kStaged) bar.sync();
         float* __restrict__ rout = a.rout + sim * a.bs_r;
-        constexpr bool kJet = OP == XR_INV_GAUGE_JET;
-        JetArgs jet;
-        if constexpr (kJet) jet = a.jets ? a.jets[sim] : a.jet;
         auto src = [&](int j) -> T {
             const int k = j <= N / 2 ? j : N - j;
             float2 u, v;
@@ -297,22 +288,11 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
                 for (int i = lt; i < cells; i += C * NT) {
                     const int row = i / N, j = i - row * N;
                     const T qq = sm[L::template at<N, NT>(j, row >> 1)];
-                    float4 v = ps[i];
-                    if constexpr (kJet) {
-                        const unsigned r = (unsigned)rbase + row;
-                        restrict_cell(a.g, jet, j, (int)(r % (unsigned)ny), (int)(r / (unsigned)ny), rbase * N + i, v);
-                    }
-                    out[i] = gauge4(v, (row & 1) ? qq.y : qq.x);
+                    out[i] = gauge4(ps[i], (row & 1) ? qq.y : qq.x);
                 }
                 return;
             }
             Plan<N>::template run_keep<L, +1, KM>(x, t, q, sm, a.g.tw[0], src, pencil_bar<NT, C>(bar));
-            int y0 = 0, z0 = 0, y1 = 0, z1 = 0;
-            if constexpr (kJet) {
-                const unsigned r = (unsigned)r0;
-                y0 = (int)(r % (unsigned)ny), z0 = (int)(r / (unsigned)ny);
-                y1 = y0 + 1 == ny ? 0 : y0 + 1, z1 = y1 == 0 ? z0 + 1 : z0;
-            }
             // GB outputs of both rows at a time: their psi is loaded before any
             // of them is stored (2 GB loads in flight)
             constexpr int RL = Plan<N>::last, P = N / RL, NBT = Stage<N, NT, RL>::NBT;
@@ -334,10 +314,6 @@ __device__ __forceinline__ void xreal_body(const XArgs a, const Blk bk, unsigned
                         for (int u = 0; u < GB; ++u) {
                             const int j = i + (r + u) * P;
                             const T v = x[b * RL + r + u];
-                            if constexpr (kJet) {
-                                if (v0) restrict_cell(a.g, jet, j, y0, z0, b0 + j, p0[u]);
-                                if (v1) restrict_cell(a.g, jet, j, y1, z1, b1 + j, p1[u]);
-                            }
                             if (v0) psi[b0 + j] = gauge4(p0[u], v.x);
                             if (v1) psi[b1 + j] = gauge4(p1[u], v.y);
                         }
@@ -355,13 +331,12 @@ __global__ void __launch_bounds__(XRShape<N, G, KM, C>::BLK) k_xreal(XArgs a) {
     xreal_body<N, OP, G, KM, C>(a, launch_blk(), smraw);
 }
 
-// The 16-pair pass on rows of at least 256 cells, compiled for 3 resident CTAs
-// per SM (at most 42 registers; the gauge pass at 256x128x128 ran 35.4 -> 34.6
-// us), the restricted gauge for 2 (64 registers: nozzle projection there
-// 112 us, uncapped, at 72 registers and 1 CTA, 124).  The ensembles' short rows keep
-// k_xreal; capped, their batched step was 5 % slower.
+// The 16-pair pass compiled for 3 resident CTAs per SM (at most 42 registers),
+// launched for rows of at least 256 cells: the gauge pass at 256x128x128 ran
+// 35.4 -> 34.6 us.  The ensembles' short rows keep k_xreal; capped, their
+// batched step was 5 % slower.
 template <int N, int OP, int G, bool KM = false>
-__global__ void __launch_bounds__(XRShape<N, G, KM>::BLK, OP == XR_INV_GAUGE_JET ? 2 : 3) k_xreal_long(XArgs a) {
+__global__ void __launch_bounds__(XRShape<N, G, KM>::BLK, 3) k_xreal_long(XArgs a) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     xreal_body<N, OP, G, KM>(a, launch_blk(), smraw);

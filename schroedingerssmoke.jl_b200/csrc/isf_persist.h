@@ -34,10 +34,11 @@ enum PKind : int {
     PK_Z_MASK,          // schroedinger z fwd * mask / N, z inv
     PK_Y_INV,           // schroedinger y inv
     PK_X_INV_NORM,      // schroedinger x inv + normalize
-    PK_DIV,             // projection div stencil (restricted with the step's jets when use_jet)
+    PK_RESTRICT,        // restrict_velocity! with the step's jets
+    PK_DIV,             // projection div stencil
     PK_XR_FWD,          // projection x fwd (real, k-major half spectrum)
     PK_PLANE,           // projection (y, z) planes
-    PK_XR_INV_GAUGE,    // projection x inv + gauge (restricted when use_jet)
+    PK_XR_INV_GAUGE,    // projection x inv + gauge
     PK_EMIT,            // add_particles! into the step's ring slots
     PK_VEL,             // one-form stencil (hbar, sharp)
     PK_ADVECT,          // staggered_advect!
@@ -61,7 +62,8 @@ struct PPhase {
     YZArgs yz;
     StencilArgs st;
     PlaneArgs pl;
-    Grid g;                      // PROLOGUE / EMIT / ADVECT
+    Grid g;                      // PROLOGUE / RESTRICT / EMIT / ADVECT
+    float4* psi;                 // RESTRICT: nsim x N
     int first, nsim;             // the class's simulations (class-major index of the first)
     float* parts;                // EMIT / ADVECT: nsim x 3 nslots
     long long nslots, count;     // slots per simulation, emitted per step
@@ -89,7 +91,7 @@ struct PPlan {
 
 constexpr int kPersistThreads = 256;
 // slots (passes of all classes in one step) the kernel's shared slot table holds
-constexpr int kPersistMaxSlots = 255;
+constexpr int kPersistMaxSlots = 271;
 // slots an advection thread steps per work item
 constexpr int kAdvectSlots = 4;
 // x pencil lengths and (y, z) plane sizes the persistent kernel is built for

@@ -9,8 +9,6 @@
 // per cell.
 //
 //   ST_DIV  f = div(velocity_one_form(psi, 1))       parallel.jl:100-122, 131-152
-//           with psi optionally restricted in the nozzle on the fly
-//           (restrict_kernel, particles.jl:12-20)
 //   ST_VEL  padded velocity grid (vx, vy, vz, 0) = one_form(psi, hbar) [* 1/d]
 //           (parallel.jl:115-122, staggered sharp examples/benchmark.jl:61-63)
 #pragma once
@@ -48,12 +46,9 @@ struct StencilSmem<ST_VEL> {
     float4 tile[2][st::TH][st::TW];
 };
 
-// JET: psi is restricted in the nozzle on the fly (a.use_jet set).  A
-// compile-time switch: left to a run-time test, the restriction's code shaped
-// the plane loop of every launch (about 24 instructions per cell more, with
-// use_jet 0).  SHARP (one-form stencil): the one-form is divided by the cell
-// sizes (a.sharp set), also a compile-time switch.
-template <int OP, bool JET, bool SHARP = false, class B = CtaBar>
+// SHARP (one-form stencil): the one-form is divided by the cell sizes (a.sharp
+// set), a compile-time switch.
+template <int OP, bool SHARP = false, class B = CtaBar>
 __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, StencilSmem<OP>& S,
                                              const B& bar = B()) {
     using namespace st;
@@ -79,7 +74,7 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
     // padded column c <-> x0 + c - 1 and row r <-> y0 + r - 1 (periodic), so
     // column W+1 / row H+1 is the + halo even for a partial tile; columns and
     // rows past the halo repeat it and stay inside the grid.
-    int toff[LPT], tx_[LPT], ty_[LPT], tsl[LPT];
+    int toff[LPT], tsl[LPT];
 #pragma unroll
     for (int k = 0; k < LPT; ++k) {
         const int e = tid + k * BX * TY;
@@ -88,8 +83,6 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
         int xx = x0 + cc - 1, yy = y0 + rr - 1;
         xx = xx < 0 ? xx + nx : (xx >= nx ? xx - nx : xx);
         yy = yy < 0 ? yy + ny : (yy >= ny ? yy - ny : yy);
-        tx_[k] = xx;
-        ty_[k] = yy;
         toff[k] = xx + nx * yy;
         tsl[k] = (e < TILE) ? e : -1;
     }
@@ -97,8 +90,6 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
     // kernel-parameter fields used in the plane loop, held in registers
     const float4* __restrict__ psi = a.psi + sim * a.bs_psi;
     float* __restrict__ out = a.out + sim * a.bs_out;
-    JetArgs jet;
-    if constexpr (JET) jet = a.jets ? a.jets[sim] : a.jet;
     const float id0 = g.inv_d2[0], id1 = g.inv_d2[1], id2 = g.inv_d2[2];
     const float hb = a.hbar;
     const float di0 = g.dinv[0], di1 = g.dinv[1], di2 = g.dinv[2];
@@ -106,10 +97,7 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
     float4* __restrict__ out4 = reinterpret_cast<float4*>(out);
     const int ox = nx, oy = ny * pnx, oz = nz * pnxy;  // +face copy offsets
     auto tile_e = [&](int k, int z) -> float4 {
-        const int cidx = toff[k] + nxy * z;
-        float4 v = ldm<B>(&psi[cidx]);
-        if constexpr (JET) restrict_cell(g, jet, tx_[k], ty_[k], z, cidx, v);
-        return v;
+        return ldm<B>(&psi[toff[k] + nxy * z]);
     };
     float4* tflat0 = &tile[0][0][0];
     float4* tflat1 = &tile[1][0][0];
@@ -138,7 +126,6 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
                 const int y = y0 + ty + TY * m;
                 const int cm = x + nx * y + nxy * zm;
                 pm[m] = ldm<B>(&psi[cm]);
-                if constexpr (JET) restrict_cell(g, jet, x, y, zm, cm, pm[m]);
             }
         }
         bar.sync();

@@ -82,8 +82,7 @@ __global__ void __launch_bounds__(256) k_restrict_to(Grid g, const float4* __res
             v = gauge4(v, q[c]);
             mid[c] = v;
         }
-        restrict_cell(g, j, x, y, z, c, v);
-        out[c] = v;
+        out[c] = jet_cell(g, j, x, y, z, c) ? restrict_value(g, j, x, y, z, v) : v;
     }
 }
 

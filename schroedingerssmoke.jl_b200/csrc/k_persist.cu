@@ -126,13 +126,11 @@ __device__ __forceinline__ void run_tile(const PPlan& P, const PPhase& ph, int t
             with_xlen(ph.len, [&](auto n) { xreal_body<decltype(n)::value, XR_FWD, 1, true>(ph.x, bk, sm, bar); });
             break;
         case PK_XR_INV_GAUGE:
-            with_xlen(ph.len,
-                      [&](auto n) {
-                          if (ph.x.use_jet)
-                              xreal_body<decltype(n)::value, XR_INV_GAUGE_JET, 1, true>(ph.x, bk, sm, bar);
-                          else
-                              xreal_body<decltype(n)::value, XR_INV_GAUGE, 1, true>(ph.x, bk, sm, bar);
-                      });
+            with_xlen(ph.len, [&](auto n) { xreal_body<decltype(n)::value, XR_INV_GAUGE, 1, true>(ph.x, bk, sm, bar); });
+            break;
+        case PK_RESTRICT:
+            restrict_columns(ph.g, ph.psi + (long long)bk.z * ph.g.N, P.jets[ph.first + bk.z], bk.x * 32 + (vt & 31),
+                             bk.y * 8 + (vt >> 5), 0, 1);
             break;
         case PK_PLANE:
             with_plane(ph.len, [&](auto n) {
@@ -141,16 +139,13 @@ __device__ __forceinline__ void run_tile(const PPlan& P, const PPhase& ph, int t
             });
             break;
         case PK_DIV:
-            if (ph.st.use_jet)
-                stencil_body<ST_DIV, true>(ph.st, bk, *reinterpret_cast<StencilSmem<ST_DIV>*>(sm), bar);
-            else
-                stencil_body<ST_DIV, false>(ph.st, bk, *reinterpret_cast<StencilSmem<ST_DIV>*>(sm), bar);
+            stencil_body<ST_DIV>(ph.st, bk, *reinterpret_cast<StencilSmem<ST_DIV>*>(sm), bar);
             break;
-        case PK_VEL:  // the one-form is never restricted (isf_batch.cu builds it with use_jet 0)
+        case PK_VEL:
             if (ph.st.sharp)
-                stencil_body<ST_VEL, false, true>(ph.st, bk, *reinterpret_cast<StencilSmem<ST_VEL>*>(sm), bar);
+                stencil_body<ST_VEL, true>(ph.st, bk, *reinterpret_cast<StencilSmem<ST_VEL>*>(sm), bar);
             else
-                stencil_body<ST_VEL, false>(ph.st, bk, *reinterpret_cast<StencilSmem<ST_VEL>*>(sm), bar);
+                stencil_body<ST_VEL>(ph.st, bk, *reinterpret_cast<StencilSmem<ST_VEL>*>(sm), bar);
             break;
         case PK_EMIT: {
             const long long j = (long long)bk.x * ph.vblk + vt;

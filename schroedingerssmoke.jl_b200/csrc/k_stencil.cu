@@ -8,20 +8,19 @@ namespace isf {
 // Both stencils are compiled for 4 resident CTAs per SM (at most 64
 // registers).  The one-form stencil: 60 registers and 185 instructions per
 // cell left to ptxas (35.9 us at 256x128x128), 64 and 181 capped (34.6 us).
-template <int OP, bool JET, bool SHARP = false>
+template <int OP, bool SHARP = false>
 __global__ void __launch_bounds__(st::BX* st::TY, 4) k_stencil(StencilArgs a) {
     pdl_enter();
     __shared__ StencilSmem<OP> sm;
-    stencil_body<OP, JET, SHARP>(a, launch_blk(), sm);
+    stencil_body<OP, SHARP>(a, launch_blk(), sm);
 }
 
 // The div stencil: 48 registers and 235 instructions per cell left to
 // ptxas (40.9 us at 256x128x128), 64 and 200 capped (37.9 us).
-template <bool JET>
 __global__ void __launch_bounds__(st::BX* st::TY, 4) k_stencil_div(StencilArgs a) {
     pdl_enter();
     __shared__ StencilSmem<ST_DIV> sm;
-    stencil_body<ST_DIV, JET>(a, launch_blk(), sm);
+    stencil_body<ST_DIV>(a, launch_blk(), sm);
 }
 
 // z planes per CTA: as many as leave about one wave of the 592 resident CTAs,
@@ -45,17 +44,10 @@ cudaError_t launch_stencil(int op, const StencilArgs& args, cudaStream_t s) {
     a.sz = planes_of(a.g, (long long)bx * by * nsim);
     const dim3 grid(bx, by, (unsigned)(((a.g.n[2] + a.sz - 1) / a.sz) * nsim));
     const dim3 blk(st::BX * st::TY);
-    const bool jet = a.use_jet != 0;
-    if (op == ST_DIV)
-        return jet ? launch_pdl(k_stencil_div<true>, grid, blk, 0, s, a)
-                   : launch_pdl(k_stencil_div<false>, grid, blk, 0, s, a);
-    if (op == ST_VEL) {
-        if (a.sharp)
-            return jet ? launch_pdl(k_stencil<ST_VEL, true, true>, grid, blk, 0, s, a)
-                       : launch_pdl(k_stencil<ST_VEL, false, true>, grid, blk, 0, s, a);
-        return jet ? launch_pdl(k_stencil<ST_VEL, true>, grid, blk, 0, s, a)
-                   : launch_pdl(k_stencil<ST_VEL, false>, grid, blk, 0, s, a);
-    }
+    if (op == ST_DIV) return launch_pdl(k_stencil_div, grid, blk, 0, s, a);
+    if (op == ST_VEL)
+        return a.sharp ? launch_pdl(k_stencil<ST_VEL, true>, grid, blk, 0, s, a)
+                       : launch_pdl(k_stencil<ST_VEL>, grid, blk, 0, s, a);
     return cudaErrorInvalidValue;
 }
 
