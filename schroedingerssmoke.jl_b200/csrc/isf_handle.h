@@ -136,6 +136,8 @@ class Sequence {
     int submit(cudaStream_t st, const char* where);
 
   private:
+    int launch(cudaStream_t st, const char* where);
+
     isf_handle* h_;
     LaunchList* outer_;
     bool on_;

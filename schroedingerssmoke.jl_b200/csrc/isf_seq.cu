@@ -1,14 +1,15 @@
 // Kernel sequences of the library's calls as graphs.
 //
 // On small grids a call is bound by its launches: about 1.9 us of host time
-// each, against kernels of 1.5 to 3 us.  Jet steps of 16 kernels on 64x32x32, three
-// simulations side by side, took 43 us each one by one and take 27 as graphs.  A sequence that a handle launches again and again
-// (the same kernels in the same order) becomes an executable graph whose nodes
-// are chained by programmatic edges, as the plain launches are.  Every call sets
-// every node's shape and arguments (0.2 us each) and launches the graph (0.9
-// us): 13 kernels take 3.7 us of host time instead of 25 us, and 16.3 us back to
-// back on one stream instead of 24.6 us.  Nothing is keyed by an address: another
-// psi or particle buffer costs the same as the last one.
+// each, against kernels of 1.5 to 3 us.  Jet steps of 16 kernels on 64x32x32,
+// three simulations side by side, took 39 us each one by one and took 27.6 as
+// graphs.  A sequence that a handle launches again and again (the same kernels
+// in the same order) becomes an executable graph whose nodes are chained by
+// programmatic edges, as the plain launches are.  Every call sets every node's
+// shape and arguments (0.2 us each) and launches the graph (0.9 us): 13 kernels
+// take 3.7 us of host time instead of 25 us, and 16.3 us back to back on one
+// stream instead of 24.6 us.  Nothing is keyed by an address: another psi or
+// particle buffer costs the same as the last one.
 //
 // A graph is built (about 100 us) on the fourth call of its sequence, so
 // programs that make few calls never pay for it.
@@ -153,6 +154,14 @@ int Sequence::submit(cudaStream_t st, const char* where) {
     if (!on_) return ISF_OK;  // issued already, or part of an outer sequence
     t_record = outer_;
     on_ = false;
+    try {
+        return launch(st, where);
+    } catch (const std::bad_alloc&) {
+        return fail(h_, ISF_ERR_NOMEM, std::string(where) + ": host allocation failed");
+    }
+}
+
+int Sequence::launch(cudaStream_t st, const char* where) {
     LaunchList& l = h_->rec;
     if (l.recs.empty()) return ISF_OK;
     const size_t n = l.recs.size();
