@@ -22,8 +22,7 @@ struct isf_adj_state {
     float* qbar = nullptr;  // N
     float* fbar = nullptr;  // N
     float4* ubar = nullptr;  // cotangent of the padded velocity (NP)
-    double* acc = nullptr;  // 8 accumulators: [0..3] jet adjoint, [4] loss, [5] and [6] sums of qbar in turn
-    int qslot = 5;          // the accumulator the last summed qbar went into
+    double* acc = nullptr;  // 8 accumulators: [0..3] jet adjoint, [4] loss
     float4* tape = nullptr;        // 5 psi states of one step: a (flowed), b (normalised), c, d, e
     float* tq = nullptr;           // q1 | q2 of one step (2 N)
     float* tparts = nullptr;       // particles after the step's emission
@@ -127,15 +126,12 @@ int poisson(isf_handle* h, const float* in, float* out) {
     return ISF_OK;
 }
 
-// adjoint of psi_out = psi_in exp(-i q), q = P div W(psi_in); with sum, the
-// sum of qbar goes into acc[qslot] for the adjoint of a restriction before it
-int adj_projection(isf_handle* h, const float* psi_in, const float* q, float* bar, bool sum) {
+// adjoint of psi_out = psi_in exp(-i q), q = P div W(psi_in)
+int adj_projection(isf_handle* h, const float* psi_in, const float* q, float* bar) {
     isf_adj_state* a = h->adj;
-    const int prev = a->qslot;
-    if (sum) a->qslot = 11 - prev;  // 5 and 6 in turn; the kernel clears the other one
     const float4* pin = reinterpret_cast<const float4*>(psi_in);
     float4* b = reinterpret_cast<float4*>(bar);
-    ISF_LAUNCH(h, launch_adj_gauge(h->g, pin, q, b, a->qbar, sum ? a->acc + a->qslot : nullptr, a->acc + prev, h->stream), "adj gauge");
+    ISF_LAUNCH(h, launch_adj_gauge(h->g, pin, q, b, a->qbar, h->stream), "adj gauge");
     if (int rc = poisson(h, a->qbar, a->fbar)) return rc;
     ISF_LAUNCH(h, launch_adj_oneform_div(h->g, pin, b, a->fbar, h->stream), "adj one-form (div)");
     return ISF_OK;
@@ -241,11 +237,10 @@ int step_reverse(isf_handle* h, const float* parts_used, long long np, const Ste
     ISF_LAUNCH(h, launch_adj_oneform_vel(h->g, psi_out, b, a->ubar, h->g.hbar, 1, h->stream), "adj one-form (velocity)");
     ISF_CUDA(h, cudaMemsetAsync(a->ubar, 0, sizeof(float4) * h->g.NP, h->stream), "adj clear velocity cotangent");
     if (sj.jet) {
-        if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + 3 * N), tq + N, bar, true)) return rc;
-        ISF_LAUNCH(h, launch_adj_restrict(h->g, T + 2 * N, b, sj.j, a->acc, wscale, a->acc + a->qslot, h->stream),
-                   "adj restrict");
+        if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + 3 * N), tq + N, bar)) return rc;
+        ISF_LAUNCH(h, launch_adj_restrict(h->g, T + 2 * N, b, sj.j, a->acc, wscale, h->stream), "adj restrict");
     }
-    if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + N), tq, bar, false)) return rc;
+    if (int rc = adj_projection(h, reinterpret_cast<const float*>(T + N), tq, bar)) return rc;
     ISF_LAUNCH(h, launch_adj_normalize(h->g, T, b, h->stream), "adj normalize");
     return adj_schroedinger(h, bar);
 }
@@ -330,7 +325,7 @@ int isf_adj_pressure_project(isf_handle* h, const float* psi_in, float* psibar) 
     ISF_ALIGNED(h, psibar, 16, "psibar");
     if (int rc = adj_ensure(h)) return rc;
     if (int rc = projection_q(h, psi_in, h->adj->q)) return rc;
-    return adj_projection(h, psi_in, h->adj->q, psibar, false);
+    return adj_projection(h, psi_in, h->adj->q, psibar);
 }
 
 int isf_adj_restrict_velocity(isf_handle* h, const float* psi_in, float* psibar, const float kvec[3],
@@ -347,7 +342,7 @@ int isf_adj_restrict_velocity(isf_handle* h, const float* psi_in, float* psibar,
     if (int rc = clear_acc(h)) return rc;
     const JetArgs j = make_jet(kvec, jetmask, cen, len, rad, omgterm, phase_mode);
     ISF_LAUNCH(h, launch_adj_restrict(h->g, reinterpret_cast<const float4*>(psi_in), reinterpret_cast<float4*>(psibar), j,
-                                      h->adj->acc, 1.f, nullptr, h->stream),
+                                      h->adj->acc, 1.f, h->stream),
                "adj restrict");
     return read_acc(h, jetbar, 4);
 }
@@ -534,9 +529,8 @@ int isf_adj_gradient(isf_handle* h, const isf_adj_problem* p, const float* psi0,
         const float4* in = itape + (long long)it * N;
         ISF_LAUNCH(h, launch_restrict_to(h->g, in, work, j0, h->stream), "adj init restrict");
         if (int rc = projection_q(h, reinterpret_cast<const float*>(work), a->q)) return rc;
-        if (int rc = adj_projection(h, reinterpret_cast<const float*>(work), a->q, psibar0, true)) return rc;
-        ISF_LAUNCH(h, launch_adj_restrict(h->g, in, reinterpret_cast<float4*>(psibar0), j0, a->acc, 0.f,
-                                          a->acc + a->qslot, h->stream),
+        if (int rc = adj_projection(h, reinterpret_cast<const float*>(work), a->q, psibar0)) return rc;
+        ISF_LAUNCH(h, launch_adj_restrict(h->g, in, reinterpret_cast<float4*>(psibar0), j0, a->acc, 0.f, h->stream),
                    "adj init restrict");
     }
     double acc[5];

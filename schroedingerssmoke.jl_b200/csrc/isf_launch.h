@@ -224,19 +224,17 @@ cudaError_t launch_restrict_to(const Grid& g, const float4* in, float4* out, con
 cudaError_t launch_gauge_restrict(const Grid& g, const float4* in, const float* q, float4* mid, float4* out,
                                   const JetArgs& j, cudaStream_t s);
 cudaError_t launch_adj_normalize(const Grid& g, const float4* psi_in, float4* bar, cudaStream_t s);
-// with sum, adds the sum of qbar into *sum and sets *clear to 0
-cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar, double* sum,
-                             double* clear, cudaStream_t s);
+cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar,
+                             cudaStream_t s);
 cudaError_t launch_adj_oneform_div(const Grid& g, const float4* psi, float4* bar, const float* fbar, cudaStream_t s);
 // adds the one-form transpose of the padded velocity cotangent (scale hbar [/ d])
 cudaError_t launch_adj_oneform_vel(const Grid& g, const float4* psi, float4* bar, const float4* ubar, float hbar,
                                    int sharp, cudaStream_t s);
 cudaError_t launch_adj_from_aos(const Grid& g, const float* aos, float4* ubar, cudaStream_t s);
 cudaError_t launch_adj_to_aos(const Grid& g, const float4* ubar, float* aos, cudaStream_t s);
-// acc[0..2] += cotangent of kvec, acc[3] += cotangent of omega t times wscale;
-// qsum: null, or the sum of qbar of the projection the restricted psi went into
+// acc[0..2] += cotangent of kvec, acc[3] += cotangent of omega t times wscale
 cudaError_t launch_adj_restrict(const Grid& g, const float4* psi_in, float4* bar, const JetArgs& j, double* acc,
-                                float wscale, const double* qsum, cudaStream_t s);
+                                float wscale, cudaStream_t s);
 cudaError_t launch_adj_advect(const Grid& g, const float* parts, float* lam, long long np, const float* vel,
                               float4* ubar, cudaStream_t s);
 cudaError_t launch_loss(const float* x, const float* y, float* lam, long long np, double* loss, cudaStream_t s);

@@ -105,14 +105,10 @@ __global__ void k_adj_normalize(const float4* __restrict__ psi_in, float4* __res
 }
 
 // gauge: out = in exp(-i q).  qbar = sum_k Im(conj(bar_k) out_k);
-// bar_in = bar_out exp(+i q).  With sum, the sum of qbar over the grid is
-// added into *sum (k_adj_restrict) and *clear, the slot of the call before,
-// becomes 0.
+// bar_in = bar_out exp(+i q)
 __global__ void __launch_bounds__(256) k_adj_gauge(const float4* __restrict__ psi_in, const float* __restrict__ q,
-                                                   float4* __restrict__ bar, float* __restrict__ qbar, long long N,
-                                                   double* __restrict__ sum, double* __restrict__ clear) {
+                                                   float4* __restrict__ bar, float* __restrict__ qbar, long long N) {
     pdl_enter();
-    double total[1] = {0.0};
     for (long long c = blockIdx.x * (long long)blockDim.x + threadIdx.x; c < N; c += (long long)gridDim.x * blockDim.x) {
         const float qc = q[c];
         const float4 v = psi_in[c];
@@ -120,14 +116,8 @@ __global__ void __launch_bounds__(256) k_adj_gauge(const float4* __restrict__ ps
         float s, co;
         sincosf(qc, &s, &co);
         const float4 o = make_float4(v.x * co + v.y * s, v.y * co - v.x * s, v.z * co + v.w * s, v.w * co - v.z * s);
-        const float qb = (g.x * o.y - g.y * o.x) + (g.z * o.w - g.w * o.z);
-        qbar[c] = qb;
-        total[0] += qb;
+        qbar[c] = (g.x * o.y - g.y * o.x) + (g.z * o.w - g.w * o.z);
         bar[c] = make_float4(g.x * co - g.y * s, g.x * s + g.y * co, g.z * co - g.w * s, g.z * s + g.w * co);
-    }
-    if (sum) {
-        block_sum_add<1>(total, sum);
-        if (blockIdx.x == 0 && threadIdx.x == 0) *clear = 0.0;
     }
 }
 
@@ -241,24 +231,20 @@ __global__ void __launch_bounds__(256) k_adj_oneform(AdjOneFormArgs A) {
 // -phibar wscale (the adjoint of omega t times wscale: t for the adjoint of
 // omega itself).
 //
-// With qsum, the restricted psi went into a projection whose qbar
-// (k_adj_gauge) sums to *qsum.  The projection turns a phase alpha per cell
-// into the single phase mean(alpha) (the one-form of alpha is exact and the
-// Poisson solve inverts its divergence but for the mean), so phibar is
-// -*qsum / N in every nozzle cell.  Left to the sum over cells it is what
-// remains of a cancellation between the gauge's and the one-form's parts, with
-// a relative error of 1e-6 to 1e-5 that changed from run to run (2^18
-// particles on 128x64x64); from the sum of qbar it is below 1e-6.
-template <bool PROJECTED>
+// After a projection phibar could be had from the sum of its qbar alone: the
+// projection turns a phase per cell into the mean phase, wherever every edge
+// at the nozzle carries the phase difference.  An edge with z = 0 (psi exactly
+// zero on a side) carries none, so the sum over the cells is taken, which
+// holds in every case.  It is what remains of a cancellation between the
+// gauge's and the one-form's parts: 2e-7 to 2e-4 relative to 64 bits (30 states
+// on 56x40x40 to 128x80x80).
 __global__ void __launch_bounds__(256) k_adj_restrict(Grid g, const float4* __restrict__ psi_in,
                                                       float4* __restrict__ bar, JetArgs j, double* __restrict__ acc,
-                                                      float wscale, const double* __restrict__ qsum) {
+                                                      float wscale) {
     pdl_enter();
     double v4[4] = {0.0, 0.0, 0.0, 0.0};
     bool any = false;
     const int x = cell_x(), y = cell_y();
-    double phq = 0.0;
-    if constexpr (PROJECTED) phq = -*qsum * g.invN;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         if (x >= g.n[0] || y >= g.n[1]) break;
         const long long c = cell(g, x, y, z);
@@ -282,11 +268,8 @@ __global__ void __launch_bounds__(256) k_adj_restrict(Grid g, const float4* __re
         const float r1 = gb.x * co + gb.y * s, r2 = gb.z * co + gb.w * s;
         const float i1 = a1 > 0.f ? r1 / a1 : 0.f, i2 = a2 > 0.f ? r2 / a2 : 0.f;
         bar[c] = make_float4(i1 * v.x, i1 * v.y, i2 * v.z, i2 * v.w);
-        double phb = phq;
-        if constexpr (!PROJECTED) {
-            const float4 o = make_float4(a1 * co, a1 * s, a2 * co, a2 * s);
-            phb = -((gb.x * o.y - gb.y * o.x) + (gb.z * o.w - gb.w * o.z));
-        }
+        const float4 o = make_float4(a1 * co, a1 * s, a2 * co, a2 * s);
+        const double phb = -((gb.x * o.y - gb.y * o.x) + (gb.z * o.w - gb.w * o.z));
         if (j.phase_mode == 0) {
             v4[0] += phb;
             v4[1] += phb;
@@ -553,9 +536,9 @@ cudaError_t launch_gauge_restrict(const Grid& g, const float4* in, const float* 
 cudaError_t launch_adj_normalize(const Grid& g, const float4* psi_in, float4* bar, cudaStream_t s) {
     return launch_pdl(k_adj_normalize, dim3(grid_n(g.N, 256)), dim3(256), 0, s, psi_in, bar, g.N);
 }
-cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar, double* sum,
-                             double* clear, cudaStream_t s) {
-    return launch_pdl(k_adj_gauge, dim3(grid_n(g.N, 256)), dim3(256), 0, s, psi_in, q, bar, qbar, g.N, sum, clear);
+cudaError_t launch_adj_gauge(const Grid& g, const float4* psi_in, const float* q, float4* bar, float* qbar,
+                             cudaStream_t s) {
+    return launch_pdl(k_adj_gauge, dim3(grid_n(g.N, 256)), dim3(256), 0, s, psi_in, q, bar, qbar, g.N);
 }
 cudaError_t launch_adj_oneform_div(const Grid& g, const float4* psi, float4* bar, const float* fbar, cudaStream_t s) {
     AdjOneFormArgs a;
@@ -579,9 +562,8 @@ cudaError_t launch_adj_oneform_vel(const Grid& g, const float4* psi, float4* bar
     return launch_pdl(k_adj_oneform<false>, cell_grid(g), dim3(256), 0, s, a);
 }
 cudaError_t launch_adj_restrict(const Grid& g, const float4* psi_in, float4* bar, const JetArgs& j, double* acc,
-                                float wscale, const double* qsum, cudaStream_t s) {
-    return launch_pdl(qsum ? k_adj_restrict<true> : k_adj_restrict<false>, cell_grid(g), dim3(256), 0, s, g, psi_in, bar,
-                      j, acc, wscale, qsum);
+                                float wscale, cudaStream_t s) {
+    return launch_pdl(k_adj_restrict, cell_grid(g), dim3(256), 0, s, g, psi_in, bar, j, acc, wscale);
 }
 cudaError_t launch_adj_advect(const Grid& g, const float* parts, float* lam, long long np, const float* vel,
                               float4* ubar, cudaStream_t s) {
