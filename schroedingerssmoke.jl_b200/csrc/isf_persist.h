@@ -90,8 +90,9 @@ struct PPlan {
 };
 
 constexpr int kPersistThreads = 256;
-// slots (passes of all classes in one step) the kernel's shared slot table holds
-constexpr int kPersistMaxSlots = 271;
+// slots (passes of all classes in one step) the kernel's shared slot table holds:
+// 17 jet classes without particles (16 passes each), 15 with (18)
+constexpr int kPersistMaxSlots = 272;
 // slots an advection thread steps per work item
 constexpr int kAdvectSlots = 4;
 // x pencil lengths and (y, z) plane sizes the persistent kernel is built for
