@@ -535,9 +535,9 @@ int isf_schroedinger_flow(isf_handle* h, float* psi) {
     ISF_ENTER(h);
     if (!psi) return fail(h, ISF_ERR_INVALID, "isf_schroedinger_flow: null psi");
     ISF_ALIGNED(h, psi, 16, "psi");
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "schroedinger_flow");
     if (int rc = run_schroedinger(h, psi, false)) return rc;
-    return seq.submit(h->stream, "schroedinger_flow");
+    return seq.submit();
 }
 
 int isf_normalize_psi(isf_handle* h, float* psi) {
@@ -552,9 +552,9 @@ int isf_pressure_project(isf_handle* h, float* psi) {
     ISF_ENTER(h);
     if (!psi) return fail(h, ISF_ERR_INVALID, "isf_pressure_project: null psi");
     ISF_ALIGNED(h, psi, 16, "psi");
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "pressure_project");
     if (int rc = run_projection(h, psi, nullptr)) return rc;
-    return seq.submit(h->stream, "pressure_project");
+    return seq.submit();
 }
 
 int isf_velocity_one_form(isf_handle* h, const float* psi, float hbar) {
@@ -615,9 +615,9 @@ int isf_init_jet(isf_handle* h, float* psi, int32_t iters, const float kvec[3], 
     // restrict_velocity!(isf, psi, kvec, isjet, 0) + pressure_project!
     JetArgs j = make_jet(kvec, mask, cen ? cen : zero, len, rad, 0.f, phase_mode);
     for (int it = 0; it < iters; ++it) {
-        Sequence seq(h);
+        Sequence seq(h, h->stream, "init_jet");
         if (int rc = run_projection(h, psi, &j)) return rc;
-        if (int rc = seq.submit(h->stream, "init_jet")) return rc;
+        if (int rc = seq.submit()) return rc;
     }
     return ISF_OK;
 }
@@ -697,7 +697,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
         if (int rc = ensure_order(h, np)) return rc;
     // the psi passes and the one-form as one sequence; what the one-form waits
     // for (the advection two steps back, run_one_form) is waited for before it
-    Sequence fields(h);
+    Sequence fields(h, h->stream, "step");
     int rc = run_schroedinger(h, psi, true);  // schroedinger_flow! + normalize_psi
     if (rc) return rc;
     rc = run_projection(h, psi, nullptr);     // pressure_project!
@@ -711,7 +711,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
     // velocity_one_form!(isf, psi, isf.hbar) + staggered sharp
     rc = run_one_form(h, psi, h->g.hbar, 1, "step one_form");
     if (rc) return rc;
-    if ((rc = fields.submit(h->stream, "step"))) return rc;
+    if ((rc = fields.submit())) return rc;
     // add_particles! (before the projections in the reference; the particles
     // are independent of psi) and staggered_advect!.  With a particle stream
     // they run there, after this step's velocity, while the caller queues the
@@ -725,7 +725,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
     }
     // emission and advection as another; a sort between them launches on its own
     const bool sort_now = h->order_every > 0 && np > 0 && resort;
-    Sequence particles(h);
+    Sequence particles(h, ps, "step");
     if (emit) {
         EmitArgs e;
         for (int k = 0; k < 3; ++k) e.cen[k] = a->nozzle_cen[k];
@@ -739,7 +739,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
     const int* order = nullptr;
     if (h->order_every > 0 && np > 0) {
         if (sort_now) {
-            if ((rc = particles.submit(ps, "step"))) return rc;
+            if ((rc = particles.submit())) return rc;
             if (int rc_o = run_order(h, parts, np, ps, "step")) return rc_o;
         }
         ++h->order_age;
@@ -747,7 +747,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
     }
     if (np > 0)
         ISF_LAUNCH_ON(h, ps, launch_advect(h->g, parts, np, h->vel, h->counters, ps, 1, 0, order), "step advect");
-    if ((rc = particles.submit(ps, "step"))) return rc;
+    if ((rc = particles.submit())) return rc;
     if (h->side && (emit || np > 0)) {
         ISF_CUDA(h, cudaEventRecord(h->ev_read[h->vcur], h->side), "step particle event");
         ISF_CUDA(h, cudaEventRecord(h->ev_side, h->side), "step particle event");
@@ -780,11 +780,11 @@ int isf_poisson_solve(isf_handle* h, const float* f, float* q) {
     XArgs xa = xargs(h);
     xa.rin = f;
     xa.rout = q;
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "poisson_solve");
     ISF_LAUNCH(h, launch_xreal(XR_FWD, xa, h->stream), "poisson x fwd");
     if (int rc = run_poisson_spectral(h, "poisson")) return rc;
     ISF_LAUNCH(h, launch_xreal(XR_INV_REAL, xa, h->stream), "poisson x inv");
-    return seq.submit(h->stream, "poisson_solve");
+    return seq.submit();
 }
 
 int isf_fft3(isf_handle* h, float* data, int32_t sign) {

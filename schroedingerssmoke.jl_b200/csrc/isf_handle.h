@@ -128,17 +128,21 @@ void adj_free(isf_handle* h);
 // While a Sequence is alive the kernels launched through launch_pdl on this
 // thread are recorded; submit() issues them on st as one graph launch, or one
 // after another (isf_seq.cu).  The code in between queues nothing else on st that
-// has to come after one of them.  Not while profiling, which times every launch.
+// has to come after one of them.  A Sequence that ends without submit (its call
+// failed on the host) issues what it has, so the call has done what precedes
+// the failure.  Not while profiling, which times every launch.
 class Sequence {
   public:
-    explicit Sequence(isf_handle* h);
+    Sequence(isf_handle* h, cudaStream_t st, const char* where);
     ~Sequence();
-    int submit(cudaStream_t st, const char* where);
+    int submit();
 
   private:
-    int launch(cudaStream_t st, const char* where);
+    int launch();
 
     isf_handle* h_;
+    cudaStream_t st_;
+    const char* where_;
     LaunchList* outer_;
     bool on_;
 };

@@ -49,11 +49,13 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args... args) {
     if (LaunchList* l = t_record) {
+        const size_t n = l->recs.size();
         try {
             l->recs.push_back(
                 {reinterpret_cast<const void*>(kernel), grid, block, smem, l->offs.size(), sizeof...(KArgs)});
             (l->arg(static_cast<KArgs>(args)), ...);
         } catch (const std::bad_alloc&) {
+            l->recs.resize(n);  // not issued either (Sequence)
             return cudaErrorMemoryAllocation;
         }
         return cudaSuccess;

@@ -140,50 +140,56 @@ isf_seq* find(isf_handle* h) {
 
 }  // namespace
 
-Sequence::Sequence(isf_handle* h) : h_(h), outer_(t_record), on_(!h->prof_on && !t_record) {
+Sequence::Sequence(isf_handle* h, cudaStream_t st, const char* where)
+    : h_(h), st_(st), where_(where), outer_(t_record), on_(!h->prof_on && !t_record) {
     if (!on_) return;
     h->rec.clear();
     t_record = &h->rec;
 }
 
 Sequence::~Sequence() {
-    if (on_) t_record = outer_;
+    if (!on_) return;
+    t_record = outer_;
+    try {
+        issue(h_->rec, st_);  // the call's own error is the one reported
+    } catch (const std::bad_alloc&) {
+    }
 }
 
-int Sequence::submit(cudaStream_t st, const char* where) {
+int Sequence::submit() {
     if (!on_) return ISF_OK;  // issued already, or part of an outer sequence
     t_record = outer_;
     on_ = false;
     try {
-        return launch(st, where);
+        return launch();
     } catch (const std::bad_alloc&) {
-        return fail(h_, ISF_ERR_NOMEM, std::string(where) + ": host allocation failed");
+        return fail(h_, ISF_ERR_NOMEM, std::string(where_) + ": host allocation failed");
     }
 }
 
-int Sequence::launch(cudaStream_t st, const char* where) {
+int Sequence::launch() {
     LaunchList& l = h_->rec;
     if (l.recs.empty()) return ISF_OK;
     const size_t n = l.recs.size();
     if (n > 1 && n <= kMaxNodes && h_->g.N <= (n >= kLongSeq ? kLongCells : kShortCells)) {
         // a stream under capture takes the launches themselves
         cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        const bool free_stream = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+        const bool free_stream = cudaStreamIsCapturing(st_, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
         if (!free_stream) cudaGetLastError();
         isf_seq* s = free_stream ? find(h_) : nullptr;
         if (s && s->seen < kBuildAt) ++s->seen;
         if (s && (s->exec || (s->seen == kBuildAt && !s->failed && build(*s, l)))) {
-            const cudaError_t e = replay(*s, l, st);
+            const cudaError_t e = replay(*s, l, st_);
             if (e == cudaSuccess) return ISF_OK;
             // nothing of it was launched: the plain launches report what is wrong
             cudaGetLastError();
-            cudaStreamSynchronize(st);
+            cudaStreamSynchronize(st_);
             drop(*s);
             s->failed = true;
         }
     }
-    const cudaError_t e = issue(l, st);
-    return e == cudaSuccess ? ISF_OK : cuda_fail(h_, e, where);
+    const cudaError_t e = issue(l, st_);
+    return e == cudaSuccess ? ISF_OK : cuda_fail(h_, e, where_);
 }
 
 void seq_free(isf_handle* h) {

@@ -51,50 +51,50 @@ int isf_psi_to_f64(isf_handle* h, const float* psi, double* psi1, double* psi2) 
 int isf_f64_schroedinger_flow(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1,
                               double* out2) {
     ISF_ENTER(h);
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "f64 schroedinger_flow");
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_schroedinger_flow(h, psi)) return rc;
     if (int rc = isf_psi_to_f64(h, psi, out1, out2)) return rc;
-    return seq.submit(h->stream, "f64 schroedinger_flow");
+    return seq.submit();
 }
 
 int isf_f64_normalize(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1, double* out2) {
     ISF_ENTER(h);
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "f64 normalize");
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_normalize_psi(h, psi)) return rc;
     if (int rc = isf_psi_to_f64(h, psi, out1, out2)) return rc;
-    return seq.submit(h->stream, "f64 normalize");
+    return seq.submit();
 }
 
 int isf_f64_pressure_project(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1,
                              double* out2) {
     ISF_ENTER(h);
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "f64 pressure_project");
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_pressure_project(h, psi)) return rc;
     if (int rc = isf_psi_to_f64(h, psi, out1, out2)) return rc;
-    return seq.submit(h->stream, "f64 pressure_project");
+    return seq.submit();
 }
 
 int isf_f64_velocity_one_form(isf_handle* h, const double* psi1, const double* psi2, float* psi, float hbar, double* vx,
                               double* vy, double* vz) {
     ISF_ENTER(h);
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "f64 velocity_one_form");
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_velocity_one_form(h, psi, hbar)) return rc;
     if (int rc = isf_velocity_to_f64(h, vx, vy, vz)) return rc;
-    return seq.submit(h->stream, "f64 velocity_one_form");
+    return seq.submit();
 }
 
 int isf_f64_staggered_sharp(isf_handle* h, const double* vx, const double* vy, const double* vz, double* ox, double* oy,
                             double* oz) {
     ISF_ENTER(h);
-    Sequence seq(h);
+    Sequence seq(h, h->stream, "f64 staggered_sharp");
     if (int rc = isf_velocity_from_f64(h, vx, vy, vz)) return rc;
     if (int rc = isf_staggered_sharp(h)) return rc;
     if (int rc = isf_velocity_to_f64(h, ox, oy, oz)) return rc;
-    return seq.submit(h->stream, "f64 staggered_sharp");
+    return seq.submit();
 }
 
 int isf_velocity_from_f64(isf_handle* h, const double* vx, const double* vy, const double* vz) {
