@@ -161,6 +161,7 @@ void seq_free(isf_handle* h);
         const int ps_ = prof_begin(h, site);                     \
         cudaError_t e_ = (expr);                                 \
         ++(h)->launches;                                         \
+        if (t_record) t_record->name(site);                      \
         prof_end(h, ps_);                                        \
         if (e_ != cudaSuccess) return cuda_fail(h, e_, site);    \
     } while (0)
@@ -196,6 +197,7 @@ void seq_free(isf_handle* h);
         const int ps_ = prof_begin(h, site, st);                 \
         cudaError_t e_ = (expr);                                 \
         ++(h)->launches;                                         \
+        if (t_record) t_record->name(site);                      \
         prof_end(h, ps_, st);                                    \
         if (e_ != cudaSuccess) return cuda_fail(h, e_, site);    \
     } while (0)

@@ -14,7 +14,7 @@
 namespace isf {
 
 // The launches of one library call, recorded instead of issued (isf_seq.cu):
-// kernel, shape and a copy of the arguments each.
+// kernel, shape, launch site and a copy of the arguments each.
 struct LaunchList {
     struct Rec {
         const void* func;
@@ -22,14 +22,27 @@ struct LaunchList {
         size_t smem;
         size_t arg0;  // first entry of offs
         size_t nargs;
+        size_t site = 0;  // launch site (offset into names), 0: none given
     };
     std::vector<Rec> recs;
     std::vector<size_t> offs;      // argument offsets into bytes
     std::vector<unsigned char> bytes;
+    std::vector<char> names;       // launch sites, zero-terminated, after an empty one
     void clear() {
         recs.clear();
         offs.clear();
         bytes.clear();
+        names.clear();
+    }
+    // the launch site of the kernels recorded last
+    void name(const char* site) noexcept {
+        try {
+            if (names.empty()) names.push_back('\0');
+            const size_t at = names.size();
+            names.insert(names.end(), site, site + std::strlen(site) + 1);
+            for (size_t i = recs.size(); i > 0 && recs[i - 1].site == 0; --i) recs[i - 1].site = at;
+        } catch (const std::bad_alloc&) {
+        }
     }
     template <class T>
     void arg(const T& v) {

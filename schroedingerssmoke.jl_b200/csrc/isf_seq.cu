@@ -43,7 +43,8 @@ void args_of(LaunchList& l, const LaunchList::Rec& r, std::vector<void*>& out) {
     for (size_t i = 0; i < r.nargs; ++i) out[i] = l.bytes.data() + l.offs[r.arg0 + i];
 }
 
-cudaError_t issue(LaunchList& l, cudaStream_t st) {
+// the launches one after another; bad: the one that failed
+cudaError_t issue(LaunchList& l, cudaStream_t st, const LaunchList::Rec** bad = nullptr) {
     std::vector<void*> args;
     for (const LaunchList::Rec& r : l.recs) {
         args_of(l, r, args);
@@ -58,7 +59,10 @@ cudaError_t issue(LaunchList& l, cudaStream_t st) {
         cfg.attrs = attr;
         cfg.numAttrs = 1;
         const cudaError_t e = cudaLaunchKernelExC(&cfg, r.func, args.data());
-        if (e != cudaSuccess) return e;
+        if (e != cudaSuccess) {
+            if (bad) *bad = &r;
+            return e;
+        }
     }
     return cudaSuccess;
 }
@@ -188,8 +192,10 @@ int Sequence::launch() {
             s->failed = true;
         }
     }
-    const cudaError_t e = issue(l, st_);
-    return e == cudaSuccess ? ISF_OK : cuda_fail(h_, e, where_);
+    const LaunchList::Rec* bad = nullptr;
+    const cudaError_t e = issue(l, st_, &bad);
+    if (e == cudaSuccess) return ISF_OK;
+    return cuda_fail(h_, e, bad && bad->site ? l.names.data() + bad->site : where_);
 }
 
 void seq_free(isf_handle* h) {

@@ -59,6 +59,10 @@ int main(int argc, char** argv) {
     } else if (what == "stop") {  // the host fails after n kernels
         const int rc = call(&h, 1, n);
         std::printf("rc %d %s recording %d\n", rc, h.err.c_str(), t_record != nullptr);
+    } else if (what == "launch") {  // kernel n cannot be launched
+        g_fail_launch = n;
+        const int rc = call(&h, 1, 3);
+        std::printf("rc %d %s\n", rc, h.err.c_str());
     } else {
         return 2;
     }

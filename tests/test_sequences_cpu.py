@@ -40,3 +40,9 @@ def test_kernels_before_a_failure_run(run, done):
     """A call that fails on the host after some of its kernels has launched
     those, as it does without recording."""
     assert run("stop", done) == [f"launch {10 + k}" for k in range(done)] + ["rc 1 stopped recording 0"]
+
+
+@pytest.mark.parametrize("bad", [0, 1, 2])
+def test_a_launch_that_fails_is_reported_by_its_pass(run, bad):
+    done = [f"launch {10 + k}" for k in range(bad)]
+    assert run("launch", bad) == done + [f"rc 2 pass {'abc'[bad]}"]
