@@ -44,7 +44,7 @@ enum {
     ISF_OK = 0,
     ISF_ERR_INVALID = 1,     /* bad argument or unsupported size */
     ISF_ERR_CUDA = 2,        /* CUDA runtime error (message has the CUDA text) */
-    ISF_ERR_NOMEM = 3,       /* device allocation failed */
+    ISF_ERR_NOMEM = 3,       /* device or host allocation failed */
     ISF_ERR_NAN = 4,         /* isf_step with ISF_FLAG_CHECK_NAN found a non-finite psi */
     ISF_ERR_TIMEOUT = 5,     /* a bounded device-side wait of the persistent batch kernel ran out */
 };

@@ -437,10 +437,7 @@ int isf_create(const isf_params* p, isf_handle** out) {
     if (e == cudaSuccess) e = cudaMemset(h->F, 0, sizeof(float2) * nF);
     if (e != cudaSuccess) return cleanup(ISF_ERR_CUDA, std::string("isf_create: upload: ") + cudaGetErrorString(e));
     bind_tables(g, reinterpret_cast<const char*>(h->tables));
-    // room for a step's launches, so that the first call does not grow it
-    h->rec.recs.reserve(32);
-    h->rec.offs.reserve(64);
-    h->rec.bytes.reserve(32 * 1024);
+    if (!seq_reserve(h)) return cleanup(ISF_ERR_NOMEM, "isf_create: host allocation failed");
     *out = h;
     return ISF_OK;
 }

@@ -146,6 +146,9 @@ class Sequence {
     LaunchList* outer_;
     bool on_;
 };
+// room for a step's launches, so that the first call does not grow it; false
+// when the host has none
+bool seq_reserve(isf_handle* h);
 // releases the graphs of the handle's sequences
 void seq_free(isf_handle* h);
 

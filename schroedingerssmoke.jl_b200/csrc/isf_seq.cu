@@ -14,6 +14,7 @@
 // A graph is built (about 100 us) on the fourth call of its sequence, so
 // programs that make few calls never pay for it.
 #include <string>
+#include <utility>
 
 #include "isf_handle.h"
 
@@ -75,12 +76,16 @@ void drop(isf_seq& s) {
     s.nodes.clear();
 }
 
+// the thread's capture mode for the length of a scope
+struct CaptureMode {
+    cudaStreamCaptureMode mode;
+    explicit CaptureMode(cudaStreamCaptureMode m) : mode(m) { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~CaptureMode() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // the sequence's graph: a chain of kernel nodes, each allowed to start
 // while the one before it drains
-bool build(isf_seq& s, LaunchList& l) {
-    // a capture elsewhere in the process is none of this graph's business
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
+cudaError_t add_nodes(isf_seq& s, LaunchList& l) {
     std::vector<void*> args;
     cudaError_t e = cudaGraphCreate(&s.graph, 0);
     for (size_t i = 0; i < l.recs.size() && e == cudaSuccess; ++i) {
@@ -101,8 +106,19 @@ bool build(isf_seq& s, LaunchList& l) {
               : cudaGraphAddNode_v2(&node, s.graph, nullptr, nullptr, 0, &p);
         if (e == cudaSuccess) s.nodes.push_back(node);
     }
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&s.exec, s.graph, 0);
-    cudaThreadExchangeStreamCaptureMode(&mode);
+    return e == cudaSuccess ? cudaGraphInstantiate(&s.exec, s.graph, 0) : e;
+}
+
+// builds the graph, or leaves the sequence to plain launches for good
+bool build(isf_seq& s, LaunchList& l) {
+    // a capture elsewhere in the process is none of this graph's business
+    CaptureMode relaxed(cudaStreamCaptureModeRelaxed);
+    cudaError_t e;
+    try {
+        e = add_nodes(s, l);
+    } catch (const std::bad_alloc&) {
+        e = cudaErrorMemoryAllocation;
+    }
     if (e == cudaSuccess) return true;
     cudaGetLastError();
     drop(s);
@@ -137,8 +153,9 @@ isf_seq* find(isf_handle* h) {
         if (same) return &s;
     }
     if (h->seqs.size() >= kMaxSeqs) return nullptr;
-    h->seqs.emplace_back();
-    for (const LaunchList::Rec& r : l.recs) h->seqs.back().funcs.push_back(r.func);
+    isf_seq s;
+    for (const LaunchList::Rec& r : l.recs) s.funcs.push_back(r.func);
+    h->seqs.push_back(std::move(s));
     return &h->seqs.back();
 }
 
@@ -196,6 +213,18 @@ int Sequence::launch() {
     const cudaError_t e = issue(l, st_, &bad);
     if (e == cudaSuccess) return ISF_OK;
     return cuda_fail(h_, e, bad && bad->site ? l.names.data() + bad->site : where_);
+}
+
+bool seq_reserve(isf_handle* h) {
+    try {
+        h->rec.recs.reserve(32);
+        h->rec.offs.reserve(64);
+        h->rec.bytes.reserve(32 * 1024);
+        h->rec.names.reserve(1024);
+        return true;
+    } catch (const std::bad_alloc&) {
+        return false;
+    }
 }
 
 void seq_free(isf_handle* h) {

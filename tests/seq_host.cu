@@ -63,6 +63,21 @@ int main(int argc, char** argv) {
         g_fail_launch = n;
         const int rc = call(&h, 1, 3);
         std::printf("rc %d %s\n", rc, h.err.c_str());
+    } else if (what == "build") {  // host allocation n of the call that builds the graph fails
+        for (int i = 1; i <= 3; ++i)
+            if (call(&h, i, 3)) return 1;
+        g_fail_new = n;
+        const int rc = call(&h, 4, 3);
+        const bool failed = g_fail_new < 0;
+        g_fail_new = -1;
+        std::printf("rc %d mode %d\n", rc, g_mode);
+        if (call(&h, 5, 3)) return 1;
+        if (!failed) std::printf("all\n");
+    } else if (what == "reserve") {  // host allocation n of the handle's fails
+        g_fail_new = n;
+        const bool ok = seq_reserve(&h);
+        std::printf("%s\n", ok ? (g_fail_new < 0 ? "missed" : "all") : "no room");
+        g_fail_new = -1;
     } else {
         return 2;
     }

@@ -46,3 +46,27 @@ def test_kernels_before_a_failure_run(run, done):
 def test_a_launch_that_fails_is_reported_by_its_pass(run, bad):
     done = [f"launch {10 + k}" for k in range(bad)]
     assert run("launch", bad) == done + [f"rc 2 pass {'abc'[bad]}"]
+
+
+def test_no_host_memory_while_a_graph_is_built(run):
+    """Whichever host allocation of the building call fails, the call reports
+    it or launches its kernels, the thread's capture mode is as it was, and the
+    next call launches its own three kernels once."""
+    for n in range(100):
+        lines = run("build", n)[9:]
+        i = next(k for k, line in enumerate(lines) if line.startswith("rc "))
+        assert lines[i] in ("rc 0 mode 0", "rc 3 mode 0"), (n, lines)
+        kernels = lambda c: [[f"launch {10 * c + k}" for k in range(3)], [f"graph {c}0 {c}1 {c}2"]]  # noqa: E731
+        assert lines[:i] in ([[]] if lines[i].startswith("rc 3") else kernels(4)), (n, lines)
+        if lines[-1] == "all":
+            break
+        assert lines[i + 1:] in kernels(5), (n, lines)
+    assert lines[-1] == "all" and n >= 5
+
+
+def test_no_host_memory_for_the_recorded_launches(run):
+    seen = []
+    while not seen or seen[-1] != "all":
+        (line,) = run("reserve", len(seen))
+        seen.append(line)
+    assert seen == ["no room"] * (len(seen) - 1) + ["all"] and len(seen) >= 4
