@@ -87,12 +87,18 @@ __device__ __forceinline__ void pdl_enter() {
 // xsync() orders the exchanges between FFT stages (isf_fft.cuh); for
 // these two it is the same barrier as sync().
 struct CtaBar {
-    static constexpr bool kLaunch = true;
+    static constexpr bool kLaunch = true;  // a kernel launched on its own
+    static constexpr bool kJoin = true;    // psi passes take PlanJoined where it has the length
     __device__ __forceinline__ void sync() const { __syncthreads(); }
     __device__ __forceinline__ void xsync() const { __syncthreads(); }
 };
+// a launched kernel whose pass keeps Plan
+struct PlainBar : CtaBar {
+    static constexpr bool kJoin = false;
+};
 struct NamedBar {
     static constexpr bool kLaunch = false;
+    static constexpr bool kJoin = false;
     int id, n;
     __device__ __forceinline__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
     __device__ __forceinline__ void xsync() const { sync(); }
@@ -107,6 +113,7 @@ struct NamedBar {
 template <class B>
 struct WarpXBar {
     static constexpr bool kLaunch = B::kLaunch;
+    static constexpr bool kJoin = B::kJoin;
     B b;
     __device__ __forceinline__ void sync() const { b.sync(); }
     __device__ __forceinline__ void xsync() const { __syncwarp(); }

@@ -59,15 +59,15 @@ struct XTraits {
 };
 
 // the plan of an x or y / z pass: the psi passes of a kernel launched on its own
-// may join stages in registers; the persistent batch kernel, whose registers
-// are shared by every pass, keeps Plan<N>
-template <int N, class T, int ROLE, bool LAUNCH>
-using PlanOf = typename std::conditional<LAUNCH && sizeof(T) == 16 && joined(N, ROLE), PlanJoined<N>, Plan<N>>::type;
+// may join stages in registers (JOIN, chosen by the launcher); the persistent
+// batch kernel, whose registers are shared by every pass, keeps Plan<N>
+template <int N, class T, int ROLE, bool JOIN>
+using PlanOf = typename std::conditional<JOIN && sizeof(T) == 16 && joined(N, ROLE), PlanJoined<N>, Plan<N>>::type;
 
-template <int N, int OP, int G = 1, bool LAUNCH = true>
+template <int N, int OP, int G = 1, bool JOIN = true>
 struct XShape {
     static constexpr int C = XTraits<OP>::C;
-    static constexpr int NT = PlanOf<N, typename XTraits<OP>::T, ROLE_X, LAUNCH>::NT;
+    static constexpr int NT = PlanOf<N, typename XTraits<OP>::T, ROLE_X, JOIN>::NT;
     static constexpr int BLK = G * C * NT;
     static constexpr size_t SMEM = (size_t)G * N * C * sizeof(typename XTraits<OP>::T);
 };
@@ -79,7 +79,7 @@ __device__ __forceinline__ void xpass_body(const XArgs a, const Blk bk, unsigned
                                            const BarT& bar = BarT()) {
     using Tr = XTraits<OP>;
     using T = typename Tr::T;
-    using Pl = PlanOf<N, T, ROLE_X, BarT::kLaunch>;
+    using Pl = PlanOf<N, T, ROLE_X, BarT::kJoin>;
     constexpr int C = Tr::C;
     constexpr int NT = Pl::NT;
     const int grp = bk.tid / (C * NT), lt = bk.tid % (C * NT);
@@ -116,11 +116,14 @@ __device__ __forceinline__ void xpass_body(const XArgs a, const Blk bk, unsigned
     Pl::template run<Swz<C>, Tr::S, false>(x, t, q, sm, a.g.tw[0], src, dst, pencil_bar<NT, C>(bar));
 }
 
-template <int N, int OP, int G, bool FULL = false>
-__global__ void __launch_bounds__(XShape<N, OP, G>::BLK) k_xpass(XArgs a) {
+template <bool JOIN>
+using PassBar = typename std::conditional<JOIN, CtaBar, PlainBar>::type;
+
+template <int N, int OP, int G, bool FULL = false, bool JOIN = true>
+__global__ void __launch_bounds__(XShape<N, OP, G, JOIN>::BLK) k_xpass(XArgs a) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
-    xpass_body<N, OP, G, FULL>(a, launch_blk(), smraw);
+    xpass_body<N, OP, G, FULL>(a, launch_blk(), smraw, PassBar<JOIN>());
 }
 
 // ------------------------------------------- x pass of real data (Poisson)
@@ -494,12 +497,13 @@ struct YZArgs {
 #define ISF_YZ_PSI_SPECTRAL_MIN_THREADS 512
 #endif
 
-template <int N, class T, int OP, bool LAUNCH>
-using PlanYZ = PlanOf<N, T, (OP < YZ_MASK ? ROLE_YZ : ROLE_SPECTRAL), LAUNCH>;
+constexpr int yz_role(int op) { return op < YZ_MASK ? ROLE_YZ : ROLE_SPECTRAL; }
+template <int N, class T, int OP, bool JOIN>
+using PlanYZ = PlanOf<N, T, yz_role(OP), JOIN>;
 
-template <int N, class T, int OP = 0, int G = 1, bool LAUNCH = true>
+template <int N, class T, int OP = 0, int G = 1, bool JOIN = true>
 struct YZShape {
-    using Pl = PlanYZ<N, T, OP, LAUNCH>;
+    using Pl = PlanYZ<N, T, OP, JOIN>;
     static constexpr int C = 128 / (int)sizeof(T);
     static constexpr int NT = Pl::NT;
     static constexpr int BLK = G * C * NT;
@@ -525,7 +529,7 @@ __device__ __forceinline__ double2 zmul(double2 a, double2 b) {
 template <int N, class T, int OP, int G, bool FULL = false, class BarT = CtaBar>
 __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsigned char* smraw,
                                             const BarT& bar = BarT()) {
-    using Pl = PlanYZ<N, T, OP, BarT::kLaunch>;
+    using Pl = PlanYZ<N, T, OP, BarT::kJoin>;
     constexpr int C = YZShape<N, T>::C;
     constexpr int NT = Pl::NT;
     const int grp = bk.tid / (C * NT), lt = bk.tid % (C * NT);
@@ -595,11 +599,11 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
     }
 }
 
-template <int N, class T, int OP, int G, bool FULL = false>
-__global__ void __launch_bounds__(YZShape<N, T, OP, G>::BLK, YZShape<N, T, OP, G>::MINB) k_yzpass(YZArgs a) {
+template <int N, class T, int OP, int G, bool FULL = false, bool JOIN = true>
+__global__ void __launch_bounds__(YZShape<N, T, OP, G, JOIN>::BLK, YZShape<N, T, OP, G, JOIN>::MINB) k_yzpass(YZArgs a) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
-    yzpass_body<N, T, OP, G, FULL>(a, launch_blk(), smraw);
+    yzpass_body<N, T, OP, G, FULL>(a, launch_blk(), smraw, PassBar<JOIN>());
 }
 
 }  // namespace isf

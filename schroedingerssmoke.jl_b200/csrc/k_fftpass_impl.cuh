@@ -33,18 +33,21 @@ cudaError_t ensure_smem(K kernel, size_t smem, std::atomic<unsigned long long>& 
 
 inline unsigned batch_dim(int nsim) { return (unsigned)(nsim > 1 ? nsim : 1); }
 
-template <int N, int OP, int G, bool FULL = false>
+template <int N, int OP, int G, bool FULL = false, bool JOIN = true>
 cudaError_t launch_x_ng(const XArgs& a, cudaStream_t s) {
-    using Sh = XShape<N, OP, G>;
+    using Sh = XShape<N, OP, G, JOIN>;
     static std::atomic<unsigned long long> done{0};
     const long long rows = (long long)a.g.n[1] * a.g.n[2];
+    if constexpr (JOIN && G == 1 && sizeof(typename XTraits<OP>::T) == 16 && joined(N, ROLE_X))
+        if ((rows + Sh::C - 1) / Sh::C * batch_dim(a.nsim) < joined_from(N, ROLE_X))
+            return launch_x_ng<N, OP, G, FULL, false>(a, s);
     // grouped tiles (and the FULL variant) need whole tiles; single groups
     // guard a partial last one
     if ((G > 1 || FULL) && rows % (Sh::C * G) != 0) return cudaErrorInvalidValue;
-    cudaError_t e = ensure_smem(k_xpass<N, OP, G, FULL>, Sh::SMEM, done);
+    cudaError_t e = ensure_smem(k_xpass<N, OP, G, FULL, JOIN>, Sh::SMEM, done);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((rows + Sh::C * G - 1) / (Sh::C * G)), batch_dim(a.nsim));
-    return launch_pdl(k_xpass<N, OP, G, FULL>, grid, dim3(Sh::BLK), Sh::SMEM, s, a);
+    return launch_pdl(k_xpass<N, OP, G, FULL, JOIN>, grid, dim3(Sh::BLK), Sh::SMEM, s, a);
 }
 
 template <int N, int OP, int G, bool KM = false, int C = 16>
@@ -63,16 +66,19 @@ cudaError_t launch_xr_ng(const XArgs& a, cudaStream_t s) {
     return launch_pdl(kern, grid, dim3(Sh::BLK), Sh::SMEM, s, a);
 }
 
-template <int N, class T, int OP, int G, bool FULL = false>
+template <int N, class T, int OP, int G, bool FULL = false, bool JOIN = true>
 cudaError_t launch_yz_ng(const YZArgs& a, cudaStream_t s) {
-    using Sh = YZShape<N, T, OP, G>;
+    using Sh = YZShape<N, T, OP, G, JOIN>;
     static std::atomic<unsigned long long> done{0};
     const int other = (a.axis == 1) ? a.g.n[2] : a.g.n[1];
+    if constexpr (JOIN && G == 1 && sizeof(T) == 16 && joined(N, yz_role(OP)))
+        if ((long long)((a.row + Sh::C - 1) / Sh::C) * other * batch_dim(a.nsim) < joined_from(N, yz_role(OP)))
+            return launch_yz_ng<N, T, OP, G, FULL, false>(a, s);
     if (other % G != 0 || ((G > 1 || FULL) && a.row % Sh::C != 0)) return cudaErrorInvalidValue;
-    cudaError_t e = ensure_smem(k_yzpass<N, T, OP, G, FULL>, Sh::SMEM, done);
+    cudaError_t e = ensure_smem(k_yzpass<N, T, OP, G, FULL, JOIN>, Sh::SMEM, done);
     if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((a.row + Sh::C - 1) / Sh::C), (unsigned)(other / G), batch_dim(a.nsim));
-    return launch_pdl(k_yzpass<N, T, OP, G, FULL>, grid, dim3(Sh::BLK), Sh::SMEM, s, a);
+    return launch_pdl(k_yzpass<N, T, OP, G, FULL, JOIN>, grid, dim3(Sh::BLK), Sh::SMEM, s, a);
 }
 
 // every supported pencil length, each case expanding MACRO(n)
