@@ -288,21 +288,21 @@ int run_projection(isf_handle* h, float* psi, const JetArgs* jet) {
     xa.rin = h->f;
     ISF_LAUNCH(h, launch_stencil(ST_DIV, sa, h->stream), "projection div");
     ISF_LAUNCH(h, launch_xreal(XR_FWD, xa, h->stream), "projection x fwd");
-    if (int rc = run_poisson_spectral(h, "projection")) return rc;
+    if (int rc = run_poisson_spectral(h, ISF_POISSON_SITES("projection"))) return rc;
     ISF_LAUNCH(h, launch_xreal(XR_INV_GAUGE, xa, h->stream), "projection x inv + gauge");
     return ISF_OK;
 }
 
 // y / z transforms with fac/N between them, on the handle's half spectrum:
 // one plane kernel for a k-major spectrum, three y / z passes otherwise
-int run_poisson_spectral(isf_handle* h, const char* site) {
+int run_poisson_spectral(isf_handle* h, const PoissonSites& site) {
     if (h->kmajor) {
-        ISF_LAUNCH(h, launch_poisson_plane(h->g, h->F, 0, 1, h->stream), (std::string(site) + " yz planes").c_str());
+        ISF_LAUNCH(h, launch_poisson_plane(h->g, h->F, 0, 1, h->stream), site.planes);
         return ISF_OK;
     }
-    ISF_LAUNCH(h, launch_yzpass_c(YZ_FWD, yzhalf(h, 1), h->stream), (std::string(site) + " y fwd").c_str());
-    ISF_LAUNCH(h, launch_yzpass_c(YZ_FAC, yzhalf(h, 2), h->stream), (std::string(site) + " z fac").c_str());
-    ISF_LAUNCH(h, launch_yzpass_c(YZ_INV, yzhalf(h, 1), h->stream), (std::string(site) + " y inv").c_str());
+    ISF_LAUNCH(h, launch_yzpass_c(YZ_FWD, yzhalf(h, 1), h->stream), site.y_fwd);
+    ISF_LAUNCH(h, launch_yzpass_c(YZ_FAC, yzhalf(h, 2), h->stream), site.z_fac);
+    ISF_LAUNCH(h, launch_yzpass_c(YZ_INV, yzhalf(h, 1), h->stream), site.y_inv);
     return ISF_OK;
 }
 
@@ -532,7 +532,7 @@ int isf_schroedinger_flow(isf_handle* h, float* psi) {
     ISF_ENTER(h);
     if (!psi) return fail(h, ISF_ERR_INVALID, "isf_schroedinger_flow: null psi");
     ISF_ALIGNED(h, psi, 16, "psi");
-    Sequence seq(h, h->stream, "schroedinger_flow");
+    Sequence seq(h, h->stream, "schroedinger_flow", kShortCells);
     if (int rc = run_schroedinger(h, psi, false)) return rc;
     return seq.submit();
 }
@@ -549,7 +549,7 @@ int isf_pressure_project(isf_handle* h, float* psi) {
     ISF_ENTER(h);
     if (!psi) return fail(h, ISF_ERR_INVALID, "isf_pressure_project: null psi");
     ISF_ALIGNED(h, psi, 16, "psi");
-    Sequence seq(h, h->stream, "pressure_project");
+    Sequence seq(h, h->stream, "pressure_project", kShortCells);
     if (int rc = run_projection(h, psi, nullptr)) return rc;
     return seq.submit();
 }
@@ -612,7 +612,7 @@ int isf_init_jet(isf_handle* h, float* psi, int32_t iters, const float kvec[3], 
     // restrict_velocity!(isf, psi, kvec, isjet, 0) + pressure_project!
     JetArgs j = make_jet(kvec, mask, cen ? cen : zero, len, rad, 0.f, phase_mode);
     for (int it = 0; it < iters; ++it) {
-        Sequence seq(h, h->stream, "init_jet");
+        Sequence seq(h, h->stream, "init_jet", kShortCells);
         if (int rc = run_projection(h, psi, &j)) return rc;
         if (int rc = seq.submit()) return rc;
     }
@@ -694,7 +694,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
         if (int rc = ensure_order(h, np)) return rc;
     // the psi passes and the one-form as one sequence; what the one-form waits
     // for (the advection two steps back, run_one_form) is waited for before it
-    Sequence fields(h, h->stream, "step");
+    Sequence fields(h, h->stream, "step", kLongCells);
     int rc = run_schroedinger(h, psi, true);  // schroedinger_flow! + normalize_psi
     if (rc) return rc;
     rc = run_projection(h, psi, nullptr);     // pressure_project!
@@ -722,7 +722,7 @@ int isf_step(isf_handle* h, float* psi, float* parts, int64_t np, const isf_step
     }
     // emission and advection as another; a sort between them launches on its own
     const bool sort_now = h->order_every > 0 && np > 0 && resort;
-    Sequence particles(h, ps, "step");
+    Sequence particles(h, ps, "step particles", kShortCells);
     if (emit) {
         EmitArgs e;
         for (int k = 0; k < 3; ++k) e.cen[k] = a->nozzle_cen[k];
@@ -777,9 +777,9 @@ int isf_poisson_solve(isf_handle* h, const float* f, float* q) {
     XArgs xa = xargs(h);
     xa.rin = f;
     xa.rout = q;
-    Sequence seq(h, h->stream, "poisson_solve");
+    Sequence seq(h, h->stream, "poisson_solve", kShortCells);
     ISF_LAUNCH(h, launch_xreal(XR_FWD, xa, h->stream), "poisson x fwd");
-    if (int rc = run_poisson_spectral(h, "poisson")) return rc;
+    if (int rc = run_poisson_spectral(h, ISF_POISSON_SITES("poisson"))) return rc;
     ISF_LAUNCH(h, launch_xreal(XR_INV_REAL, xa, h->stream), "poisson x inv");
     return seq.submit();
 }

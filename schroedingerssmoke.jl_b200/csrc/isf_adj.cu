@@ -110,7 +110,7 @@ int projection_q(isf_handle* h, const float* psi, float* q) {
     xa.rin = h->f;
     xa.rout = q;
     ISF_LAUNCH(h, launch_xreal(XR_FWD, xa, h->stream), "adj poisson x fwd");
-    if (int rc = run_poisson_spectral(h, "adj poisson")) return rc;
+    if (int rc = run_poisson_spectral(h, ISF_POISSON_SITES("adj poisson"))) return rc;
     ISF_LAUNCH(h, launch_xreal(XR_INV_REAL, xa, h->stream), "adj poisson x inv");
     return ISF_OK;
 }
@@ -121,7 +121,7 @@ int poisson(isf_handle* h, const float* in, float* out) {
     xa.rin = in;
     xa.rout = out;
     ISF_LAUNCH(h, launch_xreal(XR_FWD, xa, h->stream), "adj poisson x fwd");
-    if (int rc = run_poisson_spectral(h, "adj poisson")) return rc;
+    if (int rc = run_poisson_spectral(h, ISF_POISSON_SITES("adj poisson"))) return rc;
     ISF_LAUNCH(h, launch_xreal(XR_INV_REAL, xa, h->stream), "adj poisson x inv");
     return ISF_OK;
 }

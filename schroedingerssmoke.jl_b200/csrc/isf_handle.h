@@ -17,7 +17,7 @@ struct isf_seq {
     cudaGraphExec_t exec = nullptr;
     std::vector<cudaGraphNode_t> nodes;
     cudaGraph_t graph = nullptr;
-    int seen = 0;             // calls so far (saturating)
+    int seen = 0;             // calls so far, up to the one that builds the graph
     bool failed = false;      // the graph could not be built: plain launches
 };
 
@@ -64,6 +64,12 @@ struct isf_handle {
     isf_adj_state* adj = nullptr;
     isf::LaunchList rec;               // the launches being recorded
     std::vector<isf_seq> seqs;         // sequences seen
+    // the last sequence of each kind of call (Sequence's where): its entry of seqs
+    struct SeqSite {
+        const char* where;
+        int last;
+    };
+    SeqSite seq_sites[16] = {};
     // cell order of the particle slots (isf_set_particle_order / isf_sort_particles)
     int order_every = 0;                 // isf_step re-sorts every order_every steps (0: storage order)
     int order_age = 0;                   // isf_step advections since the last sort
@@ -116,7 +122,12 @@ int run_schroedinger(isf_handle* h, float* psi, bool norm);
 int run_projection(isf_handle* h, float* psi, const JetArgs* jet);
 int run_one_form(isf_handle* h, const float* psi, float hbar, int sharp, const char* site);
 // the y / z transforms and the Laplacian multiply of the Poisson solve on h->F
-int run_poisson_spectral(isf_handle* h, const char* site);
+// (launch sites: literals, as a recorded launch keeps the pointer)
+struct PoissonSites {
+    const char *planes, *y_fwd, *z_fac, *y_inv;
+};
+#define ISF_POISSON_SITES(who) PoissonSites{who " yz planes", who " y fwd", who " z fac", who " y inv"}
+int run_poisson_spectral(isf_handle* h, const PoissonSites& site);
 
 // the cell order of np slots on stream st (launch sites "<site> order count / scan / scatter")
 int ensure_order(isf_handle* h, long long np);
@@ -125,15 +136,18 @@ int run_order(isf_handle* h, const float* parts, long long np, cudaStream_t st, 
 // releases the adjoint work buffers (isf_adj.cu)
 void adj_free(isf_handle* h);
 
-// While a Sequence is alive the kernels launched through launch_pdl on this
-// thread are recorded; submit() issues them on st as one graph launch, or one
-// after another (isf_seq.cu).  The code in between queues nothing else on st that
-// has to come after one of them.  A Sequence that ends without submit (its call
-// failed on the host) issues what it has, so the call has done what precedes
-// the failure.  Not while profiling, which times every launch.
+// The launches of a library call, on one stream.  Once the call's sequence of
+// kernels has come back often enough, the kernels launched through launch_pdl on
+// this thread while the Sequence is alive are recorded, and submit() issues
+// them as one graph launch (isf_seq.cu); until then they are launched as they
+// come and only noted.  The code in between queues nothing else on the stream
+// that has to come after one of them.  A Sequence that ends without submit (its
+// call failed on the host) issues what it has recorded, so the call has done
+// what precedes the failure.  Not while profiling, which times every launch, nor
+// on grids of more than max_cells.
 class Sequence {
   public:
-    Sequence(isf_handle* h, cudaStream_t st, const char* where);
+    Sequence(isf_handle* h, cudaStream_t st, const char* where, long long max_cells);
     ~Sequence();
     int submit();
 
@@ -143,9 +157,18 @@ class Sequence {
     isf_handle* h_;
     cudaStream_t st_;
     const char* where_;
+    isf_handle::SeqSite* site_ = nullptr;
     LaunchList* outer_;
     bool on_;
 };
+// Grids up to which a sequence becomes a graph: short sequences (up to seven
+// kernels) and longer ones.  Where the GPU is the bound a graph gains nothing,
+// and its start, which does not overlap the kernel before it, costs about 3 us:
+// the driver loop's short sequences (flow, projection) on 128x64x64 ran 108 us
+// one by one and 113 as graphs, on 100x50x50 103 and 107 but 76 and 54 with
+// three simulations side by side.  The fused step's one long sequence was no
+// slower up to 160x80x80 (155 and 149 us) and equal on 256x128x128.
+constexpr long long kShortCells = 300000, kLongCells = 1LL << 21;
 // room for a step's launches, so that the first call does not grow it; false
 // when the host has none
 bool seq_reserve(isf_handle* h);
@@ -164,7 +187,7 @@ void seq_free(isf_handle* h);
         const int ps_ = prof_begin(h, site);                     \
         cudaError_t e_ = (expr);                                 \
         ++(h)->launches;                                         \
-        if (t_record) t_record->name(site);                      \
+        if ((h)->rec.hold) (h)->rec.name(site);                  \
         prof_end(h, ps_);                                        \
         if (e_ != cudaSuccess) return cuda_fail(h, e_, site);    \
     } while (0)
@@ -200,7 +223,7 @@ void seq_free(isf_handle* h);
         const int ps_ = prof_begin(h, site, st);                 \
         cudaError_t e_ = (expr);                                 \
         ++(h)->launches;                                         \
-        if (t_record) t_record->name(site);                      \
+        if ((h)->rec.hold) (h)->rec.name(site);                  \
         prof_end(h, ps_, st);                                    \
         if (e_ != cudaSuccess) return cuda_fail(h, e_, site);    \
     } while (0)

@@ -13,36 +13,37 @@
 
 namespace isf {
 
-// The launches of one library call, recorded instead of issued (isf_seq.cu):
-// kernel, shape, launch site and a copy of the arguments each.
+// The launches of one library call (isf_seq.cu).  With hold they are recorded
+// instead of issued: kernel, shape, launch site and a copy of the arguments
+// each.  Without, only which kernels were launched.
 struct LaunchList {
+    bool hold = false;
+    bool over = false;  // more kernels were noted than recs has room for
     struct Rec {
         const void* func;
         dim3 grid, block;
         size_t smem;
         size_t arg0;  // first entry of offs
         size_t nargs;
-        size_t site = 0;  // launch site (offset into names), 0: none given
+        const char* site = nullptr;  // launch site
     };
     std::vector<Rec> recs;
     std::vector<size_t> offs;      // argument offsets into bytes
     std::vector<unsigned char> bytes;
-    std::vector<char> names;       // launch sites, zero-terminated, after an empty one
     void clear() {
+        over = false;
         recs.clear();
         offs.clear();
         bytes.clear();
-        names.clear();
     }
-    // the launch site of the kernels recorded last
-    void name(const char* site) noexcept {
-        try {
-            if (names.empty()) names.push_back('\0');
-            const size_t at = names.size();
-            names.insert(names.end(), site, site + std::strlen(site) + 1);
-            for (size_t i = recs.size(); i > 0 && recs[i - 1].site == 0; --i) recs[i - 1].site = at;
-        } catch (const std::bad_alloc&) {
-        }
+    // a kernel that is being launched
+    void note(const void* func) {
+        if (recs.size() < recs.capacity()) recs.push_back({func, dim3(), dim3(), 0, 0, 0});
+        else over = true;
+    }
+    // the launch site (a literal) of the kernels recorded last
+    void name(const char* site) {
+        for (size_t i = recs.size(); i > 0 && !recs[i - 1].site; --i) recs[i - 1].site = site;
     }
     template <class T>
     void arg(const T& v) {
@@ -52,7 +53,7 @@ struct LaunchList {
         offs.push_back(at);
     }
 };
-// the list this thread records into, or null: launches are issued
+// the list of the call this thread is in, or null
 extern thread_local LaunchList* t_record;
 
 // Launch with programmatic stream serialization: the kernel (which must call
@@ -62,16 +63,19 @@ template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                               Args... args) {
     if (LaunchList* l = t_record) {
-        const size_t n = l->recs.size();
-        try {
-            l->recs.push_back(
-                {reinterpret_cast<const void*>(kernel), grid, block, smem, l->offs.size(), sizeof...(KArgs)});
-            (l->arg(static_cast<KArgs>(args)), ...);
-        } catch (const std::bad_alloc&) {
-            l->recs.resize(n);  // not issued either (Sequence)
-            return cudaErrorMemoryAllocation;
+        if (l->hold) {
+            const size_t n = l->recs.size();
+            try {
+                l->recs.push_back(
+                    {reinterpret_cast<const void*>(kernel), grid, block, smem, l->offs.size(), sizeof...(KArgs)});
+                (l->arg(static_cast<KArgs>(args)), ...);
+            } catch (const std::bad_alloc&) {
+                l->recs.resize(n);  // not issued either (Sequence)
+                return cudaErrorMemoryAllocation;
+            }
+            return cudaSuccess;
         }
-        return cudaSuccess;
+        l->note(reinterpret_cast<const void*>(kernel));
     }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;

@@ -11,8 +11,11 @@
 // stream instead of 24.6 us.  Nothing is keyed by an address: another psi or
 // particle buffer costs the same as the last one.
 //
-// A graph is built (about 100 us) on the fourth call of its sequence, so
-// programs that make few calls never pay for it.
+// A graph costs 60 to 85 us of host time to build and 50 to give back, and saves
+// 5 to 15 us a call.  It is built on the 16th call of its sequence, when those
+// before would have paid for it; a handle that makes fewer never pays, and its
+// calls launch their kernels as they come, as if there were no sequences
+// (recording first makes a single call 1 to 2 us longer).
 #include <string>
 #include <utility>
 
@@ -27,17 +30,8 @@ namespace isf_int {
 namespace {
 
 constexpr size_t kMaxSeqs = 16;       // sequences kept per handle
-constexpr size_t kMaxNodes = 96;      // longer sequences are launched one by one
-constexpr int kBuildAt = 4;           // the call of a sequence that builds its graph
-// Grids up to which a sequence becomes a graph.  Where the GPU is the bound a
-// graph gains nothing, and its start, which does not overlap the kernel before
-// it, costs about 3 us: the driver loop's short sequences (flow, projection) on
-// 128x64x64 ran 108 us one by one and 113 as graphs, on 100x50x50 103 and 107
-// but 76 and 54 with three simulations side by side.  The fused step's one
-// long sequence was no slower up to 160x80x80 (155 and 149 us) and equal on
-// 256x128x128.
-constexpr size_t kLongSeq = 8;
-constexpr long long kShortCells = 300000, kLongCells = 1LL << 21;
+constexpr size_t kMaxNodes = 32;      // longer sequences are launched one by one (a step has up to 17)
+constexpr int kBuildAt = 16;          // the call of a sequence that builds its graph
 
 void args_of(LaunchList& l, const LaunchList::Rec& r, std::vector<void*>& out) {
     out.resize(r.nargs);
@@ -143,84 +137,108 @@ cudaError_t replay(isf_seq& s, LaunchList& l, cudaStream_t st) {
     return cudaGraphLaunch(s.exec, st);
 }
 
-// the handle's entry for the recorded kernels, or null when it has kMaxSeqs
+// the handle's entry for the kernels in h->rec, or -1 when it has kMaxSeqs
 // others (a handle's calls make fewer)
-isf_seq* find(isf_handle* h) {
+int find(isf_handle* h) {
     const LaunchList& l = h->rec;
-    for (isf_seq& s : h->seqs) {
+    for (size_t k = 0; k < h->seqs.size(); ++k) {
+        const isf_seq& s = h->seqs[k];
         bool same = s.funcs.size() == l.recs.size();
         for (size_t i = 0; same && i < s.funcs.size(); ++i) same = s.funcs[i] == l.recs[i].func;
-        if (same) return &s;
+        if (same) return (int)k;
     }
-    if (h->seqs.size() >= kMaxSeqs) return nullptr;
+    if (h->seqs.size() >= kMaxSeqs) return -1;
     isf_seq s;
     for (const LaunchList::Rec& r : l.recs) s.funcs.push_back(r.func);
     h->seqs.push_back(std::move(s));
-    return &h->seqs.back();
+    return (int)h->seqs.size() - 1;
 }
+
+// the handle's note of a kind of call, or null when it has no room
+isf_handle::SeqSite* site_of(isf_handle* h, const char* where) {
+    for (isf_handle::SeqSite& s : h->seq_sites) {
+        if (!s.where) s = {where, -1};
+        if (s.where == where) return &s;
+    }
+    return nullptr;
+}
+
+// does the next call of the sequence go through a graph?
+bool ready(const isf_seq& s) { return s.exec || (!s.failed && s.seen >= kBuildAt - 1); }
 
 }  // namespace
 
-Sequence::Sequence(isf_handle* h, cudaStream_t st, const char* where)
-    : h_(h), st_(st), where_(where), outer_(t_record), on_(!h->prof_on && !t_record) {
+Sequence::Sequence(isf_handle* h, cudaStream_t st, const char* where, long long max_cells)
+    : h_(h), st_(st), where_(where), outer_(t_record), on_(!h->prof_on && !t_record && h->g.N <= max_cells) {
     if (!on_) return;
     h->rec.clear();
+    h->rec.hold = false;
+    site_ = site_of(h, where);
+    if (site_ && site_->last >= 0 && ready(h->seqs[site_->last])) {
+        // a stream under capture takes the launches themselves
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+        else h->rec.hold = cap == cudaStreamCaptureStatusNone;
+    }
     t_record = &h->rec;
 }
 
 Sequence::~Sequence() {
     if (!on_) return;
     t_record = outer_;
+    if (!h_->rec.hold) return;
     try {
         issue(h_->rec, st_);  // the call's own error is the one reported
     } catch (const std::bad_alloc&) {
     }
+    h_->rec.hold = false;
 }
 
 int Sequence::submit() {
     if (!on_) return ISF_OK;  // issued already, or part of an outer sequence
     t_record = outer_;
     on_ = false;
+    const bool hold = h_->rec.hold;
+    int rc;
     try {
-        return launch();
+        rc = launch();
     } catch (const std::bad_alloc&) {
-        return fail(h_, ISF_ERR_NOMEM, std::string(where_) + ": host allocation failed");
+        rc = hold ? fail(h_, ISF_ERR_NOMEM, std::string(where_) + ": host allocation failed") : ISF_OK;
     }
+    h_->rec.hold = false;
+    return rc;
 }
 
 int Sequence::launch() {
     LaunchList& l = h_->rec;
-    if (l.recs.empty()) return ISF_OK;
     const size_t n = l.recs.size();
-    if (n > 1 && n <= kMaxNodes && h_->g.N <= (n >= kLongSeq ? kLongCells : kShortCells)) {
-        // a stream under capture takes the launches themselves
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-        const bool free_stream = cudaStreamIsCapturing(st_, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
-        if (!free_stream) cudaGetLastError();
-        isf_seq* s = free_stream ? find(h_) : nullptr;
-        if (s && s->seen < kBuildAt) ++s->seen;
-        if (s && (s->exec || (s->seen == kBuildAt && !s->failed && build(*s, l)))) {
-            const cudaError_t e = replay(*s, l, st_);
-            if (e == cudaSuccess) return ISF_OK;
+    if (n == 0) return ISF_OK;
+    const int k = n > 1 && n <= kMaxNodes && !l.over ? find(h_) : -1;
+    if (site_) site_->last = k;
+    if (k >= 0 && l.hold) {
+        isf_seq& s = h_->seqs[k];
+        if (s.exec || (ready(s) && build(s, l))) {
+            if (replay(s, l, st_) == cudaSuccess) return ISF_OK;
             // nothing of it was launched: the plain launches report what is wrong
             cudaGetLastError();
             cudaStreamSynchronize(st_);
-            drop(*s);
-            s->failed = true;
+            drop(s);
+            s.failed = true;
         }
     }
+    if (k >= 0 && h_->seqs[k].seen < kBuildAt - 1) ++h_->seqs[k].seen;
+    if (!l.hold) return ISF_OK;  // launched as they came
     const LaunchList::Rec* bad = nullptr;
     const cudaError_t e = issue(l, st_, &bad);
     if (e == cudaSuccess) return ISF_OK;
-    return cuda_fail(h_, e, bad && bad->site ? l.names.data() + bad->site : where_);
+    return cuda_fail(h_, e, bad && bad->site ? bad->site : where_);
 }
 
 bool seq_reserve(isf_handle* h) {
     try {
-        h->rec.recs.reserve(32);
+        h->rec.recs.reserve(kMaxNodes);
         h->rec.offs.reserve(64);
         h->rec.bytes.reserve(32 * 1024);
-        h->rec.names.reserve(1024);
         return true;
     } catch (const std::bad_alloc&) {
         return false;

@@ -51,7 +51,7 @@ int isf_psi_to_f64(isf_handle* h, const float* psi, double* psi1, double* psi2) 
 int isf_f64_schroedinger_flow(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1,
                               double* out2) {
     ISF_ENTER(h);
-    Sequence seq(h, h->stream, "f64 schroedinger_flow");
+    Sequence seq(h, h->stream, "f64 schroedinger_flow", kShortCells);
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_schroedinger_flow(h, psi)) return rc;
     if (int rc = isf_psi_to_f64(h, psi, out1, out2)) return rc;
@@ -60,7 +60,7 @@ int isf_f64_schroedinger_flow(isf_handle* h, const double* psi1, const double* p
 
 int isf_f64_normalize(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1, double* out2) {
     ISF_ENTER(h);
-    Sequence seq(h, h->stream, "f64 normalize");
+    Sequence seq(h, h->stream, "f64 normalize", kShortCells);
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_normalize_psi(h, psi)) return rc;
     if (int rc = isf_psi_to_f64(h, psi, out1, out2)) return rc;
@@ -70,7 +70,8 @@ int isf_f64_normalize(isf_handle* h, const double* psi1, const double* psi2, flo
 int isf_f64_pressure_project(isf_handle* h, const double* psi1, const double* psi2, float* psi, double* out1,
                              double* out2) {
     ISF_ENTER(h);
-    Sequence seq(h, h->stream, "f64 pressure_project");
+    // eight kernels without the plane solver
+    Sequence seq(h, h->stream, "f64 pressure_project", h->kmajor ? kShortCells : kLongCells);
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_pressure_project(h, psi)) return rc;
     if (int rc = isf_psi_to_f64(h, psi, out1, out2)) return rc;
@@ -80,7 +81,7 @@ int isf_f64_pressure_project(isf_handle* h, const double* psi1, const double* ps
 int isf_f64_velocity_one_form(isf_handle* h, const double* psi1, const double* psi2, float* psi, float hbar, double* vx,
                               double* vy, double* vz) {
     ISF_ENTER(h);
-    Sequence seq(h, h->stream, "f64 velocity_one_form");
+    Sequence seq(h, h->stream, "f64 velocity_one_form", kShortCells);
     if (int rc = isf_psi_from_f64(h, psi1, psi2, psi)) return rc;
     if (int rc = isf_velocity_one_form(h, psi, hbar)) return rc;
     if (int rc = isf_velocity_to_f64(h, vx, vy, vz)) return rc;
@@ -90,7 +91,7 @@ int isf_f64_velocity_one_form(isf_handle* h, const double* psi1, const double* p
 int isf_f64_staggered_sharp(isf_handle* h, const double* vx, const double* vy, const double* vz, double* ox, double* oy,
                             double* oz) {
     ISF_ENTER(h);
-    Sequence seq(h, h->stream, "f64 staggered_sharp");
+    Sequence seq(h, h->stream, "f64 staggered_sharp", kShortCells);
     if (int rc = isf_velocity_from_f64(h, vx, vy, vz)) return rc;
     if (int rc = isf_staggered_sharp(h)) return rc;
     if (int rc = isf_velocity_to_f64(h, ox, oy, oz)) return rc;

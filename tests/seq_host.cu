@@ -36,13 +36,15 @@ __global__ void ka(int) {}
 __global__ void kb(int) {}
 __global__ void kc(int) {}
 
-// a call of three kernels, the host failing before kernel `stop` (3: not at all)
-static int call(isf_handle* h, int tag, int stop) {
-    Sequence seq(h, nullptr, "call");
+// a call of three kernels without kernel `skip`, the host failing before kernel
+// `stop` (3: not at all)
+static int call(isf_handle* h, int tag, int stop = 3, int skip = -1) {
+    Sequence seq(h, nullptr, "call", 4096);
     void (*const k[3])(int) = {ka, kb, kc};
     const char* const site[3] = {"pass a", "pass b", "pass c"};
     for (int i = 0; i < 3; ++i) {
         if (i == stop) return fail(h, ISF_ERR_INVALID, "stopped");
+        if (i == skip) continue;
         ISF_LAUNCH(h, launch_pdl(k[i], dim3(1), dim3(32), 0, nullptr, 10 * tag + i), site[i]);
     }
     return seq.submit();
@@ -51,31 +53,40 @@ static int call(isf_handle* h, int tag, int stop) {
 int main(int argc, char** argv) {
     const std::string what = argc > 1 ? argv[1] : "";
     const int n = argc > 2 ? std::atoi(argv[2]) : 0;
+    const int before = argc > 3 ? std::atoi(argv[3]) : 0;  // calls before the one that matters
     isf_handle h;
-    h.g.N = 4096;
-    if (what == "repeat") {  // n calls
-        for (int i = 1; i <= n; ++i)
-            if (call(&h, i, 3)) return 1;
+    h.g.N = what == "large" ? 4097 : 4096;
+    if (!seq_reserve(&h)) return 1;
+    for (int i = 1; i <= before; ++i)
+        if (call(&h, i)) return 1;
+    const int tag = before + 1;
+    if (what == "repeat" || what == "large") {  // n calls
+        for (int i = 0; i < n; ++i)
+            if (call(&h, tag + i)) return 1;
+    } else if (what == "other") {  // n calls of other kernels
+        for (int i = 0; i < n; ++i)
+            if (call(&h, tag + i, 3, 1)) return 1;
     } else if (what == "stop") {  // the host fails after n kernels
-        const int rc = call(&h, 1, n);
+        const int rc = call(&h, tag, n);
         std::printf("rc %d %s recording %d\n", rc, h.err.c_str(), t_record != nullptr);
-    } else if (what == "launch") {  // kernel n cannot be launched
-        g_fail_launch = n;
-        const int rc = call(&h, 1, 3);
+    } else if (what == "launch") {  // kernel n cannot be launched, nor can the graph
+        g_fail_launch = 3 * before + n;
+        g_fail_graph = true;
+        if (before > 15) g_fail_launch = 3 * 15 + n;
+        const int rc = call(&h, tag);
         std::printf("rc %d %s\n", rc, h.err.c_str());
-    } else if (what == "build") {  // host allocation n of the call that builds the graph fails
-        for (int i = 1; i <= 3; ++i)
-            if (call(&h, i, 3)) return 1;
+    } else if (what == "build") {  // host allocation n of the call fails
         g_fail_new = n;
-        const int rc = call(&h, 4, 3);
+        const int rc = call(&h, tag);
         const bool failed = g_fail_new < 0;
         g_fail_new = -1;
         std::printf("rc %d mode %d\n", rc, g_mode);
-        if (call(&h, 5, 3)) return 1;
+        if (call(&h, tag + 1)) return 1;
         if (!failed) std::printf("all\n");
     } else if (what == "reserve") {  // host allocation n of the handle's fails
+        isf_handle other;
         g_fail_new = n;
-        const bool ok = seq_reserve(&h);
+        const bool ok = seq_reserve(&other);
         std::printf("%s\n", ok ? (g_fail_new < 0 ? "missed" : "all") : "no room");
         g_fail_new = -1;
     } else {
