@@ -417,6 +417,10 @@ ISF_API int isf_profile_get(const isf_handle* h, int32_t i, char* name, size_t c
                             int64_t* launches);
 /* kernels launched by h since isf_create */
 ISF_API int isf_launch_count(const isf_handle* h, uint64_t* out);
+/* Calls whose kernels went out as one graph launch, and sequences of kernels
+ * whose graph could not be built or launched (they are launched one by one from
+ * then on, with the same results). */
+ISF_API int isf_graph_count(const isf_handle* h, uint64_t* launched, uint64_t* failed);
 
 /* ---- FP64 structure-of-arrays front-end (src/MatlabPort.jl)
  *

@@ -169,6 +169,13 @@ class ISF:
         check(self.L.isf_launch_count(self.h, C.byref(out)), self.h)
         return int(out.value)
 
+    def graph_count(self) -> tuple[int, int]:
+        """Calls whose kernels went out as one graph launch, and sequences of
+        kernels whose graph failed (see isf_graph_count)."""
+        out, bad = C.c_uint64(), C.c_uint64()
+        check(self.L.isf_graph_count(self.h, C.byref(out), C.byref(bad)), self.h)
+        return int(out.value), int(bad.value)
+
     def set_particle_order(self, every: int):
         """isf_step advects through a cell-sorted permutation of the slots,
         rebuilt every `every` steps (0: storage order).  Positions are bitwise

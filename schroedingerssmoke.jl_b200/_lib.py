@@ -24,7 +24,8 @@ EXPORTS = (
     "isf_pressure_project", "isf_velocity_one_form", "isf_staggered_sharp", "isf_get_velocity",
     "isf_set_velocity", "isf_isjet", "isf_restrict_velocity", "isf_init_jet", "isf_add_particles", "isf_staggered_advect",
     "isf_step", "isf_div", "isf_poisson_solve", "isf_fft3", "isf_counters", "isf_counters_async", "isf_profile_start",
-    "isf_profile_stop", "isf_profile_sites", "isf_profile_get", "isf_launch_count", "isf_poisson_solve_static",
+    "isf_profile_stop", "isf_profile_sites", "isf_profile_get", "isf_launch_count", "isf_graph_count",
+    "isf_poisson_solve_static",
     "isf_static_last_error", "isf_batch_create", "isf_batch_destroy", "isf_batch_last_error",
     "isf_batch_set_psi", "isf_batch_get_psi", "isf_batch_set_particles", "isf_batch_get_particles",
     "isf_batch_state", "isf_batch_init_jet", "isf_batch_step", "isf_batch_set_step", "isf_batch_get_stream",
@@ -33,8 +34,8 @@ EXPORTS = (
     "isf_adj_velocity_one_form", "isf_adj_staggered_advect", "isf_adj_get_velocity_bar", "isf_adj_set_velocity_bar",
     "isf_adj_step", "isf_adj_loss", "isf_adj_gradient",
     "isf_f64_schroedinger_flow", "isf_f64_normalize", "isf_f64_pressure_project", "isf_f64_velocity_one_form",
-    "isf_f64_staggered_sharp", "isf_psi_from_f64", "isf_psi_to_f64", "isf_velocity_from_f64", "isf_velocity_to_f64", "isf_real_from_f64",
-    "isf_real_to_f64", "isf_complex_to_f64", "isf_gauge_transform", "isf_add_particles_soa",
+    "isf_f64_staggered_sharp", "isf_psi_from_f64", "isf_psi_to_f64", "isf_velocity_from_f64", "isf_velocity_to_f64",
+    "isf_real_from_f64", "isf_real_to_f64", "isf_complex_to_f64", "isf_gauge_transform", "isf_add_particles_soa",
     "isf_staggered_velocity", "isf_advect_active", "isf_keep_inside", "isf_gather_particles",
     "isf_set_particle_order", "isf_sort_particles", "isf_get_particle_order", "isf_batch_set_persistent",
 )
@@ -167,6 +168,7 @@ def load(path: str | None = None):
         "isf_profile_sites": [vp, C.POINTER(C.c_int32)],
         "isf_profile_get": [vp, i32, C.c_char_p, sz, C.POINTER(C.c_double), C.POINTER(C.c_int64)],
         "isf_launch_count": [vp, C.POINTER(C.c_uint64)],
+        "isf_graph_count": [vp, C.POINTER(C.c_uint64), C.POINTER(C.c_uint64)],
         "isf_poisson_solve_static": [C.POINTER(IsfParams), vp, vp],
         "isf_batch_create": [C.POINTER(IsfSimDesc), i32, i32, i32, C.POINTER(vp)],
         "isf_batch_destroy": [vp],

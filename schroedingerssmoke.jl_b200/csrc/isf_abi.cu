@@ -848,6 +848,13 @@ int isf_profile_get(const isf_handle* h, int32_t i, char* name, size_t cap, doub
     return ISF_OK;
 }
 
+int isf_graph_count(const isf_handle* h, uint64_t* launched, uint64_t* failed) {
+    if (!h || !launched || !failed) return fail(nullptr, ISF_ERR_INVALID, "isf_graph_count: null argument");
+    *launched = h->graph_launches;
+    *failed = h->graph_failures;
+    return ISF_OK;
+}
+
 int isf_launch_count(const isf_handle* h, uint64_t* out) {
     if (!h || !out) return fail(nullptr, ISF_ERR_INVALID, "isf_launch_count: null argument");
     *out = h->launches;

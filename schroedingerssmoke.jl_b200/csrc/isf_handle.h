@@ -70,6 +70,7 @@ struct isf_handle {
         int last;
     };
     SeqSite seq_sites[16] = {};
+    unsigned long long graph_launches = 0, graph_failures = 0;
     // cell order of the particle slots (isf_set_particle_order / isf_sort_particles)
     int order_every = 0;                 // isf_step re-sorts every order_every steps (0: storage order)
     int order_age = 0;                   // isf_step advections since the last sort

@@ -217,14 +217,19 @@ int Sequence::launch() {
     if (site_) site_->last = k;
     if (k >= 0 && l.hold) {
         isf_seq& s = h_->seqs[k];
+        const bool was_failed = s.failed;
         if (s.exec || (ready(s) && build(s, l))) {
-            if (replay(s, l, st_) == cudaSuccess) return ISF_OK;
+            if (replay(s, l, st_) == cudaSuccess) {
+                ++h_->graph_launches;
+                return ISF_OK;
+            }
             // nothing of it was launched: the plain launches report what is wrong
             cudaGetLastError();
             cudaStreamSynchronize(st_);
             drop(s);
             s.failed = true;
         }
+        if (s.failed && !was_failed) ++h_->graph_failures;
     }
     if (k >= 0 && h_->seqs[k].seen < kBuildAt - 1) ++h_->seqs[k].seen;
     if (!l.hold) return ISF_OK;  // launched as they came
