@@ -204,7 +204,12 @@ __device__ __forceinline__ float atan_poly(float s) {
 
 // atan2(y, x) for the one-form angles: t = min(|x|,|y|) / max(|x|,|y|) in
 // [0, 1], atan(t) = t P(t^2), then the octant / quadrant fix-ups.  |error| <=
-// 2.5e-7 rad for finite inputs; angle(0) = 0 as in Julia.
+// 2.5e-7 rad for finite inputs; angle(0) = 0 as in Julia.  One path for every
+// angle: with a branch in the stencils that leaves out the fix-ups below pi / 4
+// rings and smooth flows ran 0 to 2 % faster (256x128x128 step 250.4 instead of
+// 252.7 us), but where psi turns further over some edges, and a warp takes both
+// sides, the one-form took 35.6 us instead of 30.4 (2 % of the cells random) and
+// 34.1 instead of 30.6 (all random), on 100x100x100 14.9 instead of 12.5.
 __device__ __forceinline__ float isf_atan2(float y, float x) {
     const float ax = fabsf(x), ay = fabsf(y);
     const float mx = fmaxf(ax, ay), mn = fminf(ax, ay);
@@ -222,19 +227,11 @@ __device__ __forceinline__ float2 pair_z(float4 a, float4 b) {
     return make_float2(a.x * b.x + a.y * b.y + a.z * b.z + a.w * b.w, a.x * b.y - a.y * b.x + a.z * b.w - a.w * b.z);
 }
 
-// |angle| < pi / 4 (NaN and 0 are not): atan2 needs no min / max, no test of
-// a zero and no fix-ups there, and angle_small gives isf_atan2's bits.  The
-// stencils branch on it: most flows turn less than that over an edge nearly
-// everywhere (256x128x128 rings: div 38.1 -> 36.7 us, one-form 35.8 -> 34.6).
-__device__ __forceinline__ bool small_angle(float2 z) { return fabsf(z.y) < z.x; }
-__device__ __forceinline__ float angle_small(float2 z) {
-    const float t = __fdividef(z.y, z.x);
-    return t * atan_poly(t * t);
-}
-__device__ __forceinline__ float angle_of(float2 z) { return isf_atan2(z.y, z.x); }
-
 // Julia `angle(conj(a1)*b1 + conj(a2)*b2)` for psi pairs a, b (parallel.jl:108-111)
-__device__ __forceinline__ float pair_angle(float4 a, float4 b) { return angle_of(pair_z(a, b)); }
+__device__ __forceinline__ float pair_angle(float4 a, float4 b) {
+    const float2 z = pair_z(a, b);
+    return isf_atan2(z.y, z.x);
+}
 
 // particles.jl:6-10, evaluated in float with every operation rounded on its
 // own (no fused multiply-add), as the reference's broadcast over Float32

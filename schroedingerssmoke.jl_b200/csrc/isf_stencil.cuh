@@ -155,18 +155,8 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
                 const int r = ty + TY * m;
                 if (own[m]) {
                     const float4 c0 = tile[cur][r + 1][tx + 1];
-                    const float2 zx = pair_z(c0, tile[cur][r + 1][tx + 2]);
-                    const float2 zy = pair_z(c0, tile[cur][r + 2][tx + 1]);
-                    float ax, ay;
-                    if (small_angle(zx) && small_angle(zy)) {
-                        ax = angle_small(zx);
-                        ay = angle_small(zy);
-                    } else {
-                        ax = angle_of(zx);
-                        ay = angle_of(zy);
-                    }
-                    vxs[r][tx + 1] = ax;
-                    vys[r + 1][tx] = ay;
+                    vxs[r][tx + 1] = pair_angle(c0, tile[cur][r + 1][tx + 2]);
+                    vys[r + 1][tx] = pair_angle(c0, tile[cur][r + 2][tx + 1]);
                 }
             }
             // the tile's halo edges (x0-1 -> x0 per row, y0-1 -> y0 per column),
@@ -183,8 +173,7 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
             for (int m = 0; m < RPT; ++m) {
                 const int r = ty + TY * m;
                 if (own[m]) {
-                    const float2 zz = pair_z(tile[cur][r + 1][tx + 1], tile[nxt][r + 1][tx + 1]);
-                    const float vz = small_angle(zz) ? angle_small(zz) : angle_of(zz);
+                    const float vz = pair_angle(tile[cur][r + 1][tx + 1], tile[nxt][r + 1][tx + 1]);
                     const float t0 = (vxs[r][tx + 1] - vxs[r][tx]) * id0;
                     const float t1 = (vys[r + 1][tx] - vys[r][tx]) * id1;
                     const float t2 = (vz - vz_prev[m]) * id2;
@@ -199,19 +188,9 @@ __device__ __forceinline__ void stencil_body(const StencilArgs a, const Blk bk, 
                 const int r = ty + TY * m;
                 if (own[m]) {
                     const float4 c0 = tile[cur][r + 1][tx + 1];
-                    const float2 zx = pair_z(c0, tile[cur][r + 1][tx + 2]);
-                    const float2 zy = pair_z(c0, tile[cur][r + 2][tx + 1]);
-                    const float2 zz = pair_z(c0, tile[nxt][r + 1][tx + 1]);
-                    float ax, ay, az;
-                    if (small_angle(zx) && small_angle(zy) && small_angle(zz)) {
-                        ax = angle_small(zx) * hb;
-                        ay = angle_small(zy) * hb;
-                        az = angle_small(zz) * hb;
-                    } else {
-                        ax = angle_of(zx) * hb;
-                        ay = angle_of(zy) * hb;
-                        az = angle_of(zz) * hb;
-                    }
+                    float ax = pair_angle(c0, tile[cur][r + 1][tx + 2]) * hb;
+                    float ay = pair_angle(c0, tile[cur][r + 2][tx + 1]) * hb;
+                    float az = pair_angle(c0, tile[nxt][r + 1][tx + 1]) * hb;
                     if constexpr (SHARP) {
                         ax = __fmul_rn(ax, di0);
                         ay = __fmul_rn(ay, di1);
