@@ -62,20 +62,28 @@ cudaError_t launch_xpass(int op, const XArgs& a, cudaStream_t s) {
 }
 
 // Row pairs per CTA of the ungrouped real x passes: 4 below 4096 rows, 16 from
-// there on.  Short grids leave the GPU idle at 16 (64x32x32: 32 CTAs; the
-// checkpointed gradient there took 1318 us with 16 and 1295 with 4).  On
-// large ones 4 writes 64-byte instead of 256-byte segments of the k-major
+// there on.  Short grids leave the GPU idle at 16.  us per pass, 16 / 4 pairs:
+//   64 to 256 rows     forward 16: 2.6 / 2.4, 2.2 / 2.6, 100: 4.2 / 3.7, 512: 7.4 / 3.7;
+//                      gauge 8: 3.9 / 3.6, 12: 4.9 / 3.1, 56: 6.9 / 4.6, 512: 11.8 / 6.5
+//   2000 to 3584 rows  forward 8: 2.6 / 2.7, 100: 4.8 / 4.4, 512: 8.0 / 7.8; gauge 8: 4.8 / 4.0,
+//                      56: 10.0 / 5.3, 128: 5.9 / 5.6, 200: 10.2 / 8.0
+// On large ones 4 writes 64-byte instead of 256-byte segments of the k-major
 // spectrum (256x128x128 forward pass 15.4 -> 16.7 us), and although the staged
 // gauge alone is faster (34.8 -> 29.8 us), its shared memory holds up the
 // other kernels when several streams share the GPU: three ring simulations
 // side by side took 291 us per step with 16 and 329 with 4, one alone 300 and
-// 298.
+// 298.  At 512 a CTA of the staged gauge takes 82 KB and two are resident per SM:
+// with more than one wave of them, 16 is the faster one again.  The projection
+// alone / three side by side, 16 and 4: 48x48 rows 51.6 / 25.8, 46.2 / 24.0; 50x48
+// 55.6 / 28.8, 60.2 / 28.8; 64x56 62.3 / 37.5, 68.7 / 40.1.  (384: 50x64 rows 52.7 / 29.1,
+// 53.2 / 27.9; 64x56 52.8 / 33.0, 56.1 / 28.9.)
 constexpr long long kLongGridRows = 4096;
+constexpr long long long_grid_rows(int n) { return n < 512 ? kLongGridRows : 2 * 148 * 8 + 1; }
 
 template <int N, int OP, bool KM>
 static cudaError_t launch_xr_one(const XArgs& a, cudaStream_t s) {
     const long long rows = (long long)a.g.n[1] * a.g.n[2] * batch_dim(a.nsim);
-    return rows >= kLongGridRows ? launch_xr_ng<N, OP, 1, KM, 16>(a, s) : launch_xr_ng<N, OP, 1, KM, 4>(a, s);
+    return rows >= long_grid_rows(N) ? launch_xr_ng<N, OP, 1, KM, 16>(a, s) : launch_xr_ng<N, OP, 1, KM, 4>(a, s);
 }
 
 template <int N, int OP>
