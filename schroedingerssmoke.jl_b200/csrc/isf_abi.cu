@@ -51,6 +51,7 @@ void fill_grid(const int n[3], const int L[3], float hbar, float dt, Grid& g, st
     g.N = (long long)n[0] * n[1] * n[2];
     g.pnx = ((n[0] + 1 + ISF_VEL_ROW_ALIGN - 1) / ISF_VEL_ROW_ALIGN) * ISF_VEL_ROW_ALIGN;
     g.pnxy = g.pnx * (n[1] + 1);
+    g.ctw = cell_tile_width(n[0], n[1]);
     g.NP = (long long)g.pnxy * (n[2] + 1);
     g.hbar = hbar;
     g.dt = dt;

@@ -35,6 +35,7 @@ struct Grid {
     int pnx, pnxy;          // strides of the padded velocity grid: nx+1 (rounded up to the row alignment), pnx (ny+1)
     long long NP;           // cells of the padded velocity grid (float4 each)
     int norm_w;             // staggered interpolation weights divided by d (ISF_FLAG_NORMALIZED_WEIGHTS)
+    int ctw;                // log2 of the width of the cell kernels' (x, y) tiles (cell_tile_width)
 };
 
 // floats per padded velocity cell: vx, vy, vz and one unused
@@ -124,15 +125,33 @@ __device__ __forceinline__ auto pencil_bar(const B& b) {
     else return b;
 }
 
-// The cells of a grid as a launch of 256-thread blocks over 32 x 8 (x, y)
-// tiles, every block walking z from blockIdx.z in steps of gridDim.z: a
-// thread's coordinates cost no division (a flat index decoded with 64-bit
-// divisions made the nearest-neighbour kernels spend most of their
-// instructions on it).  At most about 16 blocks per SM.
-__device__ __forceinline__ int cell_x() { return (int)(blockIdx.x * 32 + (threadIdx.x & 31)); }
-__device__ __forceinline__ int cell_y() { return (int)(blockIdx.y * 8 + (threadIdx.x >> 5)); }
+// The cells of a grid as a launch of 256-thread blocks over (x, y) tiles, every
+// block walking z from blockIdx.z in steps of gridDim.z: a thread's coordinates
+// cost no division (a flat index decoded with 64-bit divisions made the
+// nearest-neighbour kernels spend most of their instructions on it).  At most
+// about 16 blocks per SM.  A tile is 32 x 8 cells; 16 x 16 or 8 x 32 (Grid::ctw)
+// where that leaves out a quarter of the lanes or more: on 16x512x512 half of 32 x 8
+// has no cells, and the one-form's transpose took 182 us there (103 in 16 x 16).
+__host__ __device__ constexpr int cell_tile_lanes(int nx, int ny, int w) {
+    return (nx + w - 1) / w * w * ((ny + 256 / w - 1) / (256 / w) * (256 / w));
+}
+constexpr int cell_tile_width(int nx, int ny) {  // log2
+    int s = 5;
+    for (int t = 4; t >= 3; --t)
+        if (4LL * cell_tile_lanes(nx, ny, 1 << t) <= 3LL * cell_tile_lanes(nx, ny, 1 << s)) s = t;
+    return s;
+}
+__host__ __device__ __forceinline__ int cell_x(const Grid& g, int block, int thread) {
+    return (block << g.ctw) + (thread & ((1 << g.ctw) - 1));
+}
+__host__ __device__ __forceinline__ int cell_y(const Grid& g, int block, int thread) {
+    return (block << (8 - g.ctw)) + (thread >> g.ctw);
+}
+__device__ __forceinline__ int cell_x(const Grid& g) { return cell_x(g, (int)blockIdx.x, (int)threadIdx.x); }
+__device__ __forceinline__ int cell_y(const Grid& g) { return cell_y(g, (int)blockIdx.y, (int)threadIdx.x); }
 inline dim3 cell_grid(const Grid& g) {
-    const unsigned bx = (unsigned)((g.n[0] + 31) / 32), by = (unsigned)((g.n[1] + 7) / 8);
+    const int w = 1 << g.ctw, h = 256 / w;
+    const unsigned bx = (unsigned)((g.n[0] + w - 1) / w), by = (unsigned)((g.n[1] + h - 1) / h);
     unsigned bz = 148u * 16u / (bx * by);
     bz = bz < 1 ? 1 : (bz > (unsigned)g.n[2] ? (unsigned)g.n[2] : bz);
     return dim3(bx, by, bz);

@@ -73,7 +73,7 @@ template <bool GAUGE>
 __global__ void __launch_bounds__(256) k_restrict_to(Grid g, const float4* __restrict__ in, const float* __restrict__ q,
                                                      float4* __restrict__ mid, float4* __restrict__ out, JetArgs j) {
     pdl_enter();
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const long long c = cell(g, x, y, z);
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(256) k_adj_gauge(const float4* __restrict__ ps
 // gathered here per cell from the edges i and i - e_a.  The velocity cotangent
 // lives on the padded grid; a cell on a low face collects the periodic copies
 // of its value on the +faces as it reads.  Bound by the seven psi cells and
-// the neighbours' cotangents, most of them L1 hits of the 32 x 8 tile.
+// the neighbours' cotangents, most of them L1 hits of the tile.
 struct AdjOneFormArgs {
     Grid g;
     const float4* psi;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(256) k_adj_oneform(AdjOneFormArgs A) {
     pdl_enter();
     const Grid& g = A.g;
     const int nx = g.n[0], ny = g.n[1], nz = g.n[2];
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= nx || y >= ny) return;
     const int xp = (x + 1 == nx) ? 0 : x + 1, xm = (x == 0) ? nx - 1 : x - 1;
     const int yp = (y + 1 == ny) ? 0 : y + 1, ym = (y == 0) ? ny - 1 : y - 1;
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(256) k_adj_restrict(Grid g, const float4* __re
     pdl_enter();
     double v4[4] = {0.0, 0.0, 0.0, 0.0};
     bool any = false;
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         if (x >= g.n[0] || y >= g.n[1]) break;
         const long long c = cell(g, x, y, z);
@@ -501,7 +501,7 @@ __global__ void k_loss(const float* __restrict__ x, const float* __restrict__ y,
 // periodic copies stay 0)
 __global__ void __launch_bounds__(256) k_adj_from_aos(Grid g, const float* __restrict__ aos, float4* __restrict__ ubar) {
     pdl_enter();
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const long long c = cell(g, x, y, z);
@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(256) k_adj_from_aos(Grid g, const float* __res
 // the velocity cotangent (padded, its copies collected) as AoS float3 per cell
 __global__ void __launch_bounds__(256) k_adj_to_aos(Grid g, const float4* __restrict__ ubar, float* __restrict__ aos) {
     pdl_enter();
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const long long c = cell(g, x, y, z);

@@ -31,7 +31,7 @@ __global__ void __launch_bounds__(256) k_restrict(Grid g, float4* __restrict__ p
     pdl_enter();
     const int sim = blockIdx.z % nsim, z0 = blockIdx.z / nsim, dz = gridDim.z / nsim;
     if (jets) j = jets[sim];
-    restrict_columns(g, psi + sim * bs_psi, j, cell_x(), cell_y(), z0, dz);
+    restrict_columns(g, psi + sim * bs_psi, j, cell_x(g), cell_y(g), z0, dz);
 }
 
 // isjet.(isf.positions, ...) (particles.jl:6-10, examples/benchmark.jl:26)
@@ -39,7 +39,7 @@ __global__ void __launch_bounds__(256) k_isjet(Grid g, uint8_t* __restrict__ out
                                                float rad) {
     pdl_enter();
     const float cen[3] = {c0, c1, c2};
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const float px = __fmul_rn((float)x, g.d[0]), py = __fmul_rn((float)y, g.d[1]), pz = __fmul_rn((float)z, g.d[2]);
@@ -62,7 +62,7 @@ __global__ void k_sharp(Grid g, float4* __restrict__ vel) {
 // div! (parallel.jl:131-152) from the padded velocity grid
 __global__ void __launch_bounds__(256) k_div(Grid g, const float4* __restrict__ vel, float* __restrict__ f) {
     pdl_enter();
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     const int xm = (x == 0) ? g.n[0] - 1 : x - 1, ym = (y == 0) ? g.n[1] - 1 : y - 1;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
@@ -75,32 +75,33 @@ __global__ void __launch_bounds__(256) k_div(Grid g, const float4* __restrict__ 
     }
 }
 
-// The velocity as AoS float3, one warp per 32 cells of a row: the cells' 384
-// bytes leave as three whole 128-byte stores per warp, each lane fetching the
-// components of its words from the lanes that loaded them (12-byte strided
-// stores touch every sector three times).
+// The velocity as AoS float3: the 384 bytes of a warp's 32 cells (of one row,
+// or of the rows of a narrower tile) leave as three stores of whole 128-byte
+// lines, each lane fetching the components of its words from the lanes that
+// loaded them (12-byte strided stores touch every sector three times).
 __global__ void __launch_bounds__(256) k_vel_to_aos(Grid g, const float4* __restrict__ vel, float* __restrict__ aos) {
     pdl_enter();
-    const int lane = threadIdx.x & 31, x0 = (int)blockIdx.x * 32, y = cell_y();
-    if (y >= g.n[1]) return;  // whole warps
-    const int nw = 3 * min(32, g.n[0] - x0);  // words of this warp's cells
+    const int lane = threadIdx.x & 31, first = threadIdx.x & ~31;
+    const int x = cell_x(g), y = cell_y(g);
+    if (cell_y(g, (int)blockIdx.y, first) >= g.n[1]) return;  // whole warps
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (x0 + lane < g.n[0]) v = vel[pcell(g, x0 + lane, y, z)];
-        float* o = aos + 3 * cell(g, x0, y, z);
+        if (x < g.n[0] && y < g.n[1]) v = vel[pcell(g, x, y, z)];
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
             const int w = lane + 32 * k, from = w / 3, comp = w - 3 * from;
             const float vx = __shfl_sync(0xffffffffu, v.x, from), vy = __shfl_sync(0xffffffffu, v.y, from),
                         vz = __shfl_sync(0xffffffffu, v.z, from);
-            if (w < nw) o[w] = comp == 0 ? vx : (comp == 1 ? vy : vz);
+            const int xf = cell_x(g, (int)blockIdx.x, first + from), yf = cell_y(g, (int)blockIdx.y, first + from);
+            if (xf < g.n[0] && yf < g.n[1])
+                aos[3 * cell(g, xf, yf, z) + comp] = comp == 0 ? vx : (comp == 1 ? vy : vz);
         }
     }
 }
 
 __global__ void __launch_bounds__(256) k_vel_from_aos(Grid g, const float* __restrict__ aos, float4* __restrict__ vel) {
     pdl_enter();
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const long long c = cell(g, x, y, z);

@@ -41,7 +41,7 @@ __global__ void k_psi_to_f64(const float4* __restrict__ psi, double2* __restrict
 __global__ void __launch_bounds__(kBlk) k_vel_from_f64(Grid g, const double* __restrict__ vx, const double* __restrict__ vy,
                                                        const double* __restrict__ vz, float4* __restrict__ vel) {
     pdl_enter();
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const long long c = cell(g, x, y, z);
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(kBlk) k_vel_from_f64(Grid g, const double* __r
 __global__ void __launch_bounds__(kBlk) k_vel_to_f64(Grid g, const float4* __restrict__ vel, double* __restrict__ vx,
                                                      double* __restrict__ vy, double* __restrict__ vz) {
     pdl_enter();
-    const int x = cell_x(), y = cell_y();
+    const int x = cell_x(g), y = cell_y(g);
     if (x >= g.n[0] || y >= g.n[1]) return;
     for (int z = blockIdx.z; z < g.n[2]; z += gridDim.z) {
         const long long c = cell(g, x, y, z);
