@@ -469,8 +469,9 @@ bool class_chain(const isf_batch* b, const BatchClass& c, int ci, std::vector<PP
         PPhase gi = new_phase(c, ci, PK_XR_INV_GAUGE, nx, rows / 32, ns, 1);
         gi.x = bx(c, 1);
         if (jets) {
-            // one virtual CTA per (32 x 8) column tile
-            PPhase r = new_phase(c, ci, PK_RESTRICT, 0, up(nx, 32), up(ny, 8), ns);
+            // virtual CTAs over the cell kernels' tiles, z in parts of kRestrictPlanes
+            PPhase r = new_phase(c, ci, PK_RESTRICT, 0, up(nx, 1 << c.g.ctw), up(ny, 256 >> c.g.ctw),
+                                 up(nz, kRestrictPlanes) * ns);
             r.psi = c.psi;
             out.push_back(r);
         }

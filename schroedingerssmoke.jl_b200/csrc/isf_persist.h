@@ -95,6 +95,11 @@ constexpr int kPersistThreads = 256;
 constexpr int kPersistMaxSlots = 272;
 // slots an advection thread steps per work item
 constexpr int kAdvectSlots = 4;
+// Planes a restriction item walks, one after another: with all of them in one
+// item five steps of 16 jets on 32^3 to 96x48x48 took 2019 us, with 8, 4 and 2
+// 1919, 1828 and 1868; six of 16x32x32 952, 808, 823 and 770; one of 64x32x32
+// 822, 765, 767 and 774.
+constexpr int kRestrictPlanes = 4;
 // x pencil lengths and (y, z) plane sizes the persistent kernel is built for
 bool persist_len_ok(int n);
 bool persist_plane_ok(int n);

@@ -128,10 +128,13 @@ __device__ __forceinline__ void run_tile(const PPlan& P, const PPhase& ph, int t
         case PK_XR_INV_GAUGE:
             with_xlen(ph.len, [&](auto n) { xreal_body<decltype(n)::value, XR_INV_GAUGE, 1, true>(ph.x, bk, sm, bar); });
             break;
-        case PK_RESTRICT:
-            restrict_columns(ph.g, ph.psi + (long long)bk.z * ph.g.N, P.jets[ph.first + bk.z], bk.x * 32 + (vt & 31),
-                             bk.y * 8 + (vt >> 5), 0, 1);
+        case PK_RESTRICT: {
+            // block z = simulation * (parts of z) + part
+            const int parts = ph.tps / (ph.gx * ph.gy), sim = bk.z / parts;
+            restrict_columns(ph.g, ph.psi + (long long)sim * ph.g.N, P.jets[ph.first + sim], cell_x(ph.g, bk.x, vt),
+                             cell_y(ph.g, bk.y, vt), bk.z - sim * parts, parts);
             break;
+        }
         case PK_PLANE:
             with_plane(ph.len, [&](auto n) {
                 constexpr int N = decltype(n)::value;
