@@ -20,7 +20,7 @@ CSRC = os.environ.get("ISF_CSRC") or os.path.join(HERE, "csrc")
 CHECK = os.environ.get("ISF_CHECK", "0") == "1"
 BUILD = os.environ.get("ISF_BUILD_DIR") or os.path.join(HERE, "_build_check" if CHECK else "_build")
 LIB = os.environ.get("ISF_LIB_OUT") or os.path.join(HERE, "libisf_check.so" if CHECK else "libisf.so")
-# extra nvcc flags, e.g. -DISF_ST_SZ=16 to build a tuning variant elsewhere
+# extra nvcc flags, e.g. -DISF_ADV_MINB=5 to build a tuning variant elsewhere
 EXTRA = os.environ.get("ISF_EXTRA_FLAGS", "").split()
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 

@@ -36,11 +36,11 @@ namespace isf {
 //              of C elements is 128 bytes, so every access is conflict free
 //              as it is, and a thread's accesses are constant offsets from one
 //              address (the swizzle costs about 4 integer instructions each)
-//   Pad<C, G>  pencil after pencil with one element of padding every 8, for
-//              lanes along j: strides of 1, 4 and 8 fall into distinct banks, and
-//              offsets are constant wherever a stage's strides are multiples
-//              of 8.  G elements make 128 bytes; the pitch sets the pencils that
-//              share a 128-byte access side by side (NT lanes each).
+//   Pad<C>     pencil after pencil of 8-byte elements with one element of padding
+//              every 8, for lanes along j: strides of 1, 4 and 8 fall into distinct
+//              banks, and offsets are constant wherever a stage's strides are
+//              multiples of 8.  The pitch sets the pencils that share a 128-byte
+//              access side by side (NT lanes each).
 // additive<D, B>: an offset D r from a base that is a multiple of B can be
 // added as step(D r).
 template <int C_>
@@ -68,14 +68,14 @@ struct Row {
     static constexpr bool additive() { return true; }
     static constexpr int step(int d) { return d * C; }
 };
-template <int C_, int G>
+template <int C_>
 struct Pad {
     static constexpr int C = C_;
     template <int N, int NT>
     static constexpr int pitch() {
-        const int rem = NT < G ? (G == 16 ? NT & ~1 : NT) : 4;  // wanted pitch mod G (even for 8-byte elements)
+        const int rem = NT < 16 ? NT & ~1 : 4;  // wanted pitch mod 16 (even: whole 16-byte vectors)
         int p = N + N / 8;
-        while (p % G != rem) ++p;
+        while (p % 16 != rem) ++p;
         return p;
     }
     template <int N, int NT>

@@ -154,7 +154,7 @@ struct XRShape {
     static constexpr int NT = Plan<N>::NT;
     static constexpr int BLK = G * C * NT;
     // the k-major inverse stages (A, B) of N/2 + 1 k per row pair in the tile
-    using L = typename std::conditional<C == 4, Pad<4, 16>, Swz<16>>::type;
+    using L = typename std::conditional<C == 4, Pad<4>, Swz<16>>::type;
     static constexpr size_t TILE = (size_t)L::template elems<N, NT>() * sizeof(float2);
     static constexpr size_t STAGE = (size_t)(N / 2 + 1) * C * sizeof(float4);
     static constexpr size_t GROUP = (KM && STAGE > TILE ? STAGE : TILE);  // bytes of one group (a multiple of 16)

@@ -117,10 +117,11 @@ class _Grid:
         self.chk(self.L.isf_velocity_from_f64(self.h, _vp(a), _vp(b), _vp(c)))
         return h1 or h2 or h3
 
-    def vel_out(self, host):
-        a, b, c = self.new(), self.new(), self.new()
-        self.chk(self.L.isf_velocity_to_f64(self.h, _vp(a), _vp(b), _vp(c)))
-        return _out(a, host), _out(b, host), _out(c, host)
+    def vel_call(self, fn, *args, host):
+        """fn on args: operator and conversions out in one library call"""
+        o = [self.new() for _ in range(3)]
+        self.chk(fn(self.h, *args, *(_vp(t) for t in o)))
+        return tuple(_out(t, host) for t in o)
 
     def real_in(self, f, dst, part=0, scale=1.0):
         """dst <- scale * (real part, part 0, or imaginary part, 1) of f"""
@@ -230,20 +231,14 @@ def StaggeredSharp(obj: ISF, vx, vy, vz):
     """MatlabPort.jl:99-104: the staggered vector field v^sharp = v / d."""
     g = obj._g
     (a, h1), (b, h2), (c, h3) = g.field(vx), g.field(vy), g.field(vz)
-    o = [g.new() for _ in range(3)]
-    g.chk(g.L.isf_f64_staggered_sharp(g.h, _vp(a), _vp(b), _vp(c), *(_vp(t) for t in o)))
-    host = h1 or h2 or h3
-    return tuple(_out(t, host) for t in o)
+    return g.vel_call(g.L.isf_f64_staggered_sharp, _vp(a), _vp(b), _vp(c), host=h1 or h2 or h3)
 
 
 def VelocityOneForm(obj: ISF, psi1, psi2, hbar=1.0):
     """MatlabPort.jl:106-126: v_a = hbar angle(conj psi1 psi1[+e_a] + conj psi2 psi2[+e_a])."""
     g = obj._g
     (a, h1), (b, h2) = g.field(psi1, torch.complex128), g.field(psi2, torch.complex128)
-    o = [g.new() for _ in range(3)]
-    g.chk(g.L.isf_f64_velocity_one_form(g.h, _vp(a), _vp(b), _vp(g.psi), float(hbar), *(_vp(t) for t in o)))
-    host = h1 or h2
-    return tuple(_out(t, host) for t in o)
+    return g.vel_call(g.L.isf_f64_velocity_one_form, _vp(a), _vp(b), _vp(g.psi), float(hbar), host=h1 or h2)
 
 
 def PoissonSolve(obj: ISF, f):
