@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(256) k_adj_oneform(AdjOneFormArgs A) {
 // at the nozzle carries the phase difference.  An edge with z = 0 (psi exactly
 // zero on a side) carries none, so the sum over the cells is taken, which
 // holds in every case.  It is what remains of a cancellation between the
-// gauge's and the one-form's parts: 2e-7 to 2e-4 relative to 64 bits (30 states
+// gauge's and the one-form's parts: 2e-7 to 7e-4 relative to 64 bits (70 states
 // on 56x40x40 to 128x80x80).
 __global__ void __launch_bounds__(256) k_adj_restrict(Grid g, const float4* __restrict__ psi_in,
                                                       float4* __restrict__ bar, JetArgs j, double* __restrict__ acc,

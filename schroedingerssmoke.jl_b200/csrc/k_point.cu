@@ -21,11 +21,13 @@ __global__ void k_normalize(float4* __restrict__ psi, long long N) {
 
 // restrict_velocity! (particles.jl:25-27) in place; a batch launch (jets !=
 // null) restricts simulation blockIdx.z mod nsim with its jets entry.  Only
-// the nozzle's cells are read and written, so the launch costs its latency
-// (about 3 us at any size).  It stands before the projection's passes: fused
-// into the divergence stencil and the gauge pass, both evaluated the
-// restriction for every load, and a nozzle projection took 112 us at 256x128x128
-// (98 now), 33 us on 128x64x64 (29 now), 22.6 us on 64x32x32 (18.5 now).
+// the nozzle's cells of psi are read and written.  A nozzle given by its geometry
+// takes 3.0 us on 64x32x32, 4.6 on 128x64x64 and 7.8 on 256x128x128 (a quarter of
+// the box wide); with a mask, whose bytes every column reads plane by plane, 3.3,
+// 5.1 and 12.  It stands before the projection's passes: fused into the
+// divergence stencil and the gauge pass, both evaluated the restriction for
+// every load, and a nozzle projection took 112 us at 256x128x128 instead of 98, 33
+// on 128x64x64 instead of 29 and 22.6 on 64x32x32 instead of 18.5.
 __global__ void __launch_bounds__(256) k_restrict(Grid g, float4* __restrict__ psi, JetArgs j,
                                                   const JetArgs* __restrict__ jets, int nsim, long long bs_psi) {
     pdl_enter();
