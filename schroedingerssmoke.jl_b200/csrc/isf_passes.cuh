@@ -501,6 +501,13 @@ constexpr int yz_role(int op) { return op < YZ_MASK ? ROLE_YZ : ROLE_SPECTRAL; }
 template <int N, class T, int OP, bool JOIN>
 using PlanYZ = PlanOf<N, T, yz_role(OP), JOIN>;
 
+// The tile layout: plain rows but for the psi y / z transforms at 192, which ran
+// up to 11 % longer in them at the same registers (us,
+// rows / swizzled: y on 80x192x64 9.0 / 8.1, 64x192x96 9.4 / 8.8, 128x192x96 13.8 / 13.5).
+template <int N, class T, int OP>
+using YZLayout = typename std::conditional<N == 192 && sizeof(T) == 16 && (OP < YZ_MASK), Swz<128 / (int)sizeof(T)>,
+                                           Row<128 / (int)sizeof(T)>>::type;
+
 template <int N, class T, int OP = 0, int G = 1, bool JOIN = true>
 struct YZShape {
     using Pl = PlanYZ<N, T, OP, JOIN>;
@@ -532,6 +539,7 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
     using Pl = PlanYZ<N, T, OP, BarT::kJoin>;
     constexpr int C = YZShape<N, T>::C;
     constexpr int NT = Pl::NT;
+    using L = YZLayout<N, T, OP>;
     const int grp = bk.tid / (C * NT), lt = bk.tid % (C * NT);
     T* sm = reinterpret_cast<T*>(smraw) + grp * (N * C);
     const int q = lt % C, t = lt / C;
@@ -559,9 +567,9 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
     };
 
     if constexpr (OP == YZ_FWD) {
-        Pl::template run<Row<C>, -1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
+        Pl::template run<L, -1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
     } else if constexpr (OP == YZ_INV) {
-        Pl::template run<Row<C>, +1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
+        Pl::template run<L, +1, false>(x, t, q, sm, tw, gsrc, gdst, bar);
     } else {
         // spectral multiply between the forward and the inverse transform of
         // this pencil; k along the pass axis is the pencil position j
@@ -580,7 +588,7 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
                 const double2 m = zmul(cxo, __ldg(&mt[j]));
                 return cmul(v, make_float2((float)m.x, msign * (float)m.y));
             };
-            Pl::template run_spectral<Row<C>>(x, t, q, sm, tw, gsrc, mmul, gdst, bar);
+            Pl::template run_spectral<L>(x, t, q, sm, tw, gsrc, mmul, gdst, bar);
         } else {
             static_assert(OP == YZ_FAC, "unhandled y/z op");
             // fac(k)/N, fac = -0.25 / sum_a (sin(pi k_a / n_a) / d_a)^2, fac(0) = 0
@@ -594,7 +602,7 @@ __device__ __forceinline__ void yzpass_body(const YZArgs a, const Blk bk, unsign
                 const float f = (pad || (zero_line && j == 0)) ? 0.f : (float)(sc * __drcp_rn(dxo + __ldg(&s2[j])));
                 return cscale(v, f);
             };
-            Pl::template run_spectral<Row<C>>(x, t, q, sm, tw, gsrc, fmul, gdst, bar);
+            Pl::template run_spectral<L>(x, t, q, sm, tw, gsrc, fmul, gdst, bar);
         }
     }
 }
