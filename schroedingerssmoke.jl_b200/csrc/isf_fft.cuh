@@ -553,7 +553,7 @@ constexpr bool joined(int n, int role) {
     if (n == 128 || n == 384) return role == ROLE_YZ;
     return (n == 96 || n == 100) && role == ROLE_SPECTRAL;
 }
-// The CTAs from which on a launch takes it.  A joined pencil has fewer threads
+// The numbers of CTAs with which a launch takes it.  A joined pencil has fewer threads
 // and more work in each, so where all CTAs are resident at once the plain plan
 // is done sooner.  us plain / joined by CTAs:
 //   z with the mask, 100  144: 5.8 / 8.1, 288: 6.4 / 8.3, 384: 9.0 / 8.7, 768: 13.6 / 10.8
@@ -561,10 +561,15 @@ constexpr bool joined(int n, int role) {
 //   y / z, 128            144: 4.7 / 5.2, 288: 5.5 / 5.9, 384: 6.3 / 6.2, 512: 6.8 / 6.5
 //   y / z, 112            192: 5.2 / 5.7, 384: 6.1 / 6.3, 512: 6.6 / 6.6, 768: 8.0 / 7.6
 //   x, 112                288: 5.0 / 5.7, 512: 6.6 / 6.6, 1152: 10.5 / 9.7
-// 96 and 384 were not slower at any count.
-constexpr long long joined_from(int n, int role) {
-    if (n == 96 || n == 384) return 0;
-    return n == 112 && role != ROLE_SPECTRAL ? 512 : 320;
+//   z with the mask, 96   480: 6.7 / 5.8, 560: 6.8 / 5.9, 640: 7.7 / 8.3, 768: 9.3 / 8.9,
+//                         1152: 11.2 / 9.6
+// At 96 the joined pass has 4 resident CTAs per SM and the plain one 5, so it is
+// slower only where the latter is done in one wave.  384 was not slower at any
+// count.
+constexpr bool joined_at(int n, int role, long long ctas) {
+    if (n == 96) return ctas <= 4 * 148 || ctas > 5 * 148;
+    if (n == 384) return true;
+    return ctas >= (n == 112 && role != ROLE_SPECTRAL ? 512 : 320);
 }
 #undef ISF_PLAN_NAMED
 

@@ -39,7 +39,7 @@ cudaError_t launch_x_ng(const XArgs& a, cudaStream_t s) {
     static std::atomic<unsigned long long> done{0};
     const long long rows = (long long)a.g.n[1] * a.g.n[2];
     if constexpr (JOIN && G == 1 && sizeof(typename XTraits<OP>::T) == 16 && joined(N, ROLE_X))
-        if ((rows + Sh::C - 1) / Sh::C * batch_dim(a.nsim) < joined_from(N, ROLE_X))
+        if (!joined_at(N, ROLE_X, (rows + Sh::C - 1) / Sh::C * batch_dim(a.nsim)))
             return launch_x_ng<N, OP, G, FULL, false>(a, s);
     // grouped tiles (and the FULL variant) need whole tiles; single groups
     // guard a partial last one
@@ -72,7 +72,7 @@ cudaError_t launch_yz_ng(const YZArgs& a, cudaStream_t s) {
     static std::atomic<unsigned long long> done{0};
     const int other = (a.axis == 1) ? a.g.n[2] : a.g.n[1];
     if constexpr (JOIN && G == 1 && sizeof(T) == 16 && joined(N, yz_role(OP)))
-        if ((long long)((a.row + Sh::C - 1) / Sh::C) * other * batch_dim(a.nsim) < joined_from(N, yz_role(OP)))
+        if (!joined_at(N, yz_role(OP), (long long)((a.row + Sh::C - 1) / Sh::C) * other * batch_dim(a.nsim)))
             return launch_yz_ng<N, T, OP, G, FULL, false>(a, s);
     if (other % G != 0 || ((G > 1 || FULL) && a.row % Sh::C != 0)) return cudaErrorInvalidValue;
     cudaError_t e = ensure_smem(k_yzpass<N, T, OP, G, FULL, JOIN>, Sh::SMEM, done);

@@ -26,3 +26,10 @@ def check(isfpkg, oracle_mod, dims):
 @pytest.mark.parametrize("dims", [(16, 192, 8), (20, 192, 12), (50, 192, 24), (8, 12, 192)])
 def test_flow_at_192(isfpkg, oracle_mod, dims):
     check(isfpkg, oracle_mod, dims)
+
+
+# z at 96 with the mask: 560 CTAs (joined), 600, 640, 672 (plain; the last with
+# a partial tile) and 768 (joined)
+@pytest.mark.parametrize("dims", [(40, 112, 96), (96, 50, 96), (80, 64, 96), (50, 96, 96), (24, 256, 96)])
+def test_flow_around_the_plain_plans_of_96(isfpkg, oracle_mod, dims):
+    check(isfpkg, oracle_mod, dims)
