@@ -556,10 +556,10 @@ constexpr bool joined(int n, int role) {
 // The numbers of CTAs with which a launch takes it.  A joined pencil has fewer threads
 // and more work in each, so where all CTAs are resident at once the plain plan
 // is done sooner.  us plain / joined by CTAs:
-//   z with the mask, 100  144: 5.8 / 8.1, 288: 6.4 / 8.3, 384: 9.0 / 8.7, 768: 13.6 / 10.8
+//   z with the mask, 100  144: 5.8 / 8.1, 288: 6.4 / 8.3, 320: 7.3 / 7.7, 384: 9.0 / 8.7, 768: 13.6 / 10.8
 //   z with the mask, 112  144: 6.3 / 7.8, 288: 6.3 / 7.6, 384: 9.2 / 7.9
 //   y / z, 128            144: 4.7 / 5.2, 288: 5.5 / 5.9, 384: 6.3 / 6.2, 512: 6.8 / 6.5
-//   y / z, 112            192: 5.2 / 5.7, 384: 6.1 / 6.3, 512: 6.6 / 6.6, 768: 8.0 / 7.6
+//   y / z, 112            192: 5.2 / 5.7, 384: 6.1 / 6.3, 560: 5.9 / 6.1, 768: 8.0 / 7.6
 //   x, 112                288: 5.0 / 5.7, 512: 6.6 / 6.6, 1152: 10.5 / 9.7
 //   z with the mask, 96   480: 6.7 / 5.8, 560: 6.8 / 5.9, 640: 7.7 / 8.3, 768: 9.3 / 8.9,
 //                         1152: 11.2 / 9.6
@@ -569,7 +569,9 @@ constexpr bool joined(int n, int role) {
 constexpr bool joined_at(int n, int role, long long ctas) {
     if (n == 96) return ctas <= 4 * 148 || ctas > 5 * 148;
     if (n == 384) return true;
-    return ctas >= (n == 112 && role != ROLE_SPECTRAL ? 512 : 320);
+    if (n == 100) return ctas >= 384;
+    if (n == 112 && role != ROLE_SPECTRAL) return ctas >= (role == ROLE_X ? 512 : 640);
+    return ctas >= 320;
 }
 #undef ISF_PLAN_NAMED
 

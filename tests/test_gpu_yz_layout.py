@@ -33,3 +33,9 @@ def test_flow_at_192(isfpkg, oracle_mod, dims):
 @pytest.mark.parametrize("dims", [(40, 112, 96), (96, 50, 96), (80, 64, 96), (50, 96, 96), (24, 256, 96)])
 def test_flow_around_the_plain_plans_of_96(isfpkg, oracle_mod, dims):
     check(isfpkg, oracle_mod, dims)
+
+
+# just below and from 384 CTAs (z at 100) and 640 (y at 112); the last partial
+@pytest.mark.parametrize("dims", [(32, 80, 100), (32, 96, 100), (56, 112, 80), (64, 112, 80), (50, 112, 100)])
+def test_flow_around_the_lines_of_100_and_112(isfpkg, oracle_mod, dims):
+    check(isfpkg, oracle_mod, dims)
